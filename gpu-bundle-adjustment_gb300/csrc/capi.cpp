@@ -61,6 +61,14 @@ void need(bool ok, const char* what) {
     if (!ok) throw std::invalid_argument(what);
 }
 
+// dense_potrs with its workspace allocated and freed on the caller's stream
+// (from the device's memory pool, as the solvers' buffers are).
+void potrs_with_workspace(const double* L, int n, int lda, int bt, double* b, const int* info, cudaStream_t stream) {
+    gba::StreamAllocScope scope(stream);
+    gba::DevBuf<unsigned char> ws(gba::dense_potrs_workspace(n));
+    gba::dense_potrs(L, n, lda, bt, b, info, ws.get(), stream);
+}
+
 gba::LMOptions to_options(const gba_lm_options* o) {
     gba::LMOptions r;
     if (!o) return r;
@@ -627,7 +635,7 @@ int gba_dense_potrs(const double* L, int n, int lda, double* b, const int* info,
     return guarded([&] {
         need(L && b && info, "null argument");
         need(n > 0 && n % 64 == 0 && lda >= n, "n must be a positive multiple of 64 and lda >= n");
-        gba::dense_potrs(L, n, lda, n / 64 - 1, b, info, static_cast<cudaStream_t>(stream));
+        potrs_with_workspace(L, n, lda, n / 64 - 1, b, info, static_cast<cudaStream_t>(stream));
     });
 }
 
@@ -645,7 +653,7 @@ int gba_band_potrs(const double* LB, int n, int ldb, int bt, double* b, const in
         need(LB && b && info, "null argument");
         need(n > 0 && n % 64 == 0, "n must be a positive multiple of 64");
         need(bt >= 0 && ldb >= (bt + 2) * 64, "ldb must be at least (bt + 2) * 64");
-        gba::dense_potrs(LB, n, ldb - 1, bt, b, info, static_cast<cudaStream_t>(stream));
+        potrs_with_workspace(LB, n, ldb - 1, bt, b, info, static_cast<cudaStream_t>(stream));
     });
 }
 

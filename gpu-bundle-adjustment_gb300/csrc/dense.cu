@@ -358,90 +358,155 @@ __global__ void __launch_bounds__(256) syrk_update_quad_kernel(double* __restric
 }
 
 // ---------------------------------------------------------------- triangular solves
+//
+// The 64 dependent steps of a substitution through a diagonal tile take two
+// FP64 instructions each, and GB300 issues one per warp every 64 cycles: 27 us a
+// tile. So the diagonal tiles are inverted first, all at once (tile_inverse),
+// and the substitution through the tiles is then one kernel per tile: x_j =
+// L_jj^-1 b_j (in every block, for itself) and the update of the block's own rows
+// (forward) or columns (backward). What bounds a step: the launch, the 64 x 64
+// product at 1.7 FMA per cycle, and the update; the operands (constant during the
+// solve) are loaded before the previous step has ended.
 
-// The diagonal block L_jj (lower triangle) and the reciprocals of its diagonal
-// into shared memory: the triangular solves below then take their 64 dependent
-// steps from shared memory, with multiplications (one division per column).
-__device__ __forceinline__ void load_diag_tile(const double* __restrict__ L, int j0, int lda, double (*t)[NB + 1],
-                                               double* rinv) {
-    for (int idx = threadIdx.x; idx < NB * NB; idx += NB) {
-        const int r = idx % NB, c = idx / NB;
-        t[c][r] = r >= c ? L[(j0 + r) + (long long)(j0 + c) * lda] : 0.0;
-    }
-    __syncthreads();
-    rinv[threadIdx.x] = 1.0 / t[threadIdx.x][threadIdx.x];
-    __syncthreads();
-}
-
-// y_j = L_jj^{-1} b_j (forward) for the diagonal block at j0; one CTA of NB threads.
-__global__ void trsv_lower_diag(const double* __restrict__ L, int j0, int lda, double* __restrict__ b,
-                                const int* __restrict__ info) {
-    __shared__ double x[NB];
-    __shared__ double t[NB][NB + 1];  // t[col][row]
+// L_jj^-1 of every tile, column-major (inv) and transposed (invt): rows of X
+// in order, X_k = (e_k - sum_m L_km X_m) / L_kk, as rank-1 updates of the rows below.
+constexpr int kInvT = 256;
+__global__ void __launch_bounds__(kInvT) tile_inverse(const double* __restrict__ L, int lda, double* __restrict__ inv,
+                                                     double* __restrict__ invt, const int* __restrict__ info) {
+    __shared__ double t[NB][NB + 1];  // t[col][row] of L
+    extern __shared__ double xs[];    // X, row-major, stride NB + 1
     __shared__ double rinv[NB];
+    pdl_wait();  // no early trigger: the first step reads the inverses before its own wait
     if (*info) return;
-    const int tr = threadIdx.x;  // NB threads
-    load_diag_tile(L, j0, lda, t, rinv);
-    x[tr] = b[j0 + tr];
+    const long long j0 = static_cast<long long>(blockIdx.x) * NB;
+    for (int i = threadIdx.x; i < NB * NB; i += kInvT) {
+        const int r = i & 63, c = i >> 6;
+        const double v = r >= c ? L[(j0 + r) + (j0 + c) * lda] : 0.0;
+        t[c][r] = v;
+        if (r == c) rinv[r] = 1.0 / v;
+        xs[r * (NB + 1) + c] = r == c ? 1.0 : 0.0;
+    }
     __syncthreads();
     for (int k = 0; k < NB; ++k) {
-        if (tr == k) x[k] *= rinv[k];
+        // row k is complete but for its pivot: columns 0 .. k
+        if (threadIdx.x <= k) xs[k * (NB + 1) + threadIdx.x] *= rinv[k];
         __syncthreads();
-        if (tr > k) x[tr] -= t[k][tr] * x[k];
-        __syncthreads();
-    }
-    b[j0 + tr] = x[tr];
-}
-
-// b[j0+NB : n) -= L[j0+NB:n, j0:j0+NB] b[j0 : j0+NB); thread per row.
-__global__ void gemv_lower_below(const double* __restrict__ L, int j0, int n, int lda, double* __restrict__ b,
-                                 const int* __restrict__ info) {
-    __shared__ double x[NB];
-    if (*info) return;
-    if (threadIdx.x < NB) x[threadIdx.x] = b[j0 + threadIdx.x];
-    __syncthreads();
-    const long long r = j0 + NB + blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    double s = 0.0;
-#pragma unroll 8
-    for (int k = 0; k < NB; ++k) s += L[r + (long long)(j0 + k) * lda] * x[k];
-    b[r] -= s;
-}
-
-// x_j = L_jj^{-T} y_j (backward) for the diagonal block at j0; one CTA of NB threads.
-__global__ void trsv_upper_diag(const double* __restrict__ L, int j0, int lda, double* __restrict__ b,
-                                const int* __restrict__ info) {
-    __shared__ double x[NB];
-    __shared__ double t[NB][NB + 1];  // t[col][row]
-    __shared__ double rinv[NB];
-    if (*info) return;
-    const int tr = threadIdx.x;
-    load_diag_tile(L, j0, lda, t, rinv);
-    x[tr] = b[j0 + tr];
-    __syncthreads();
-    for (int k = NB - 1; k >= 0; --k) {
-        if (tr == k) x[k] *= rinv[k];
-        __syncthreads();
-        // row tr of L^T is column tr of L: (L^T)(tr, k) = L(k, tr), k > tr
-        if (tr < k) x[tr] -= t[tr][k] * x[k];
+        // rows below, columns 0 .. k: a warp takes a row and 32 columns
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, halves = (k >> 5) + 1;
+        for (int w = warp; w < (NB - 1 - k) * halves; w += kInvT / 32) {
+            const int r = k + 1 + w / halves, c = 32 * (w % halves) + lane;
+            if (c <= k) xs[r * (NB + 1) + c] -= t[k][r] * xs[k * (NB + 1) + c];
+        }
         __syncthreads();
     }
-    b[j0 + tr] = x[tr];
+    double* o = inv + j0 * NB;
+    double* ot = invt + j0 * NB;
+    for (int i = threadIdx.x; i < NB * NB; i += kInvT) {
+        const int r = i & 63, c = i >> 6;
+        o[i] = xs[r * (NB + 1) + c];
+        ot[i] = xs[c * (NB + 1) + r];
+    }
 }
 
-// y[i0 : j0) -= L[j0:j0+NB, i0:j0]^T x_j; one warp per output row i (reads column i of L).
-__global__ void gemv_upper_above(const double* __restrict__ L, int i0, int j0, int lda, double* __restrict__ b,
-                                 const int* __restrict__ info) {
-    __shared__ double x[NB];
-    if (*info) return;
-    if (threadIdx.x < NB) x[threadIdx.x] = b[j0 + threadIdx.x];
+// x = M b for a 64 x 64 tile M (column-major, 0 outside the triangle): 256
+// threads, thread (row, g) sums columns g, g + 4, ... with non-zeros (m, loaded
+// by load_tile_cols); b and x in shared memory, part: 4 x 64 doubles.
+__device__ __forceinline__ bool tile_col_used(bool lower, int r, int c) {
+    return lower ? c <= (r | 31) : c >= (r & 32);  // uniform over a warp
+}
+template <bool kLower>
+__device__ __forceinline__ void load_tile_cols(const double* __restrict__ M, double (&m)[16]) {
+    const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) m[i] = tile_col_used(kLower, r, g + 4 * i) ? M[r + NB * (g + 4 * i)] : 0.0;
+}
+template <bool kLower>
+__device__ __forceinline__ void tile_product(const double (&m)[16], const double* b, double (*part)[NB], double* x) {
+    const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 16; i += 2) {
+        if (tile_col_used(kLower, r, g + 4 * i)) s0 = fma(m[i], b[g + 4 * i], s0);
+        if (tile_col_used(kLower, r, g + 4 * i + 4)) s1 = fma(m[i + 1], b[g + 4 * i + 4], s1);
+    }
+    part[g][r] = s0 + s1;
     __syncthreads();
-    const int warp = i0 + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (warp >= j0) return;
-    const double* col = L + (long long)warp * lda + j0;
-    double s = col[lane] * x[lane] + col[lane + 32] * x[lane + 32];
-    s = warp_sum(s);
-    if (lane == 0) b[warp] -= s;
+    if (threadIdx.x < NB) x[r] = (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+    __syncthreads();
+}
+
+constexpr int kSolT = 256;
+constexpr int kSolRows = 16;  // rows (columns) of L per pass of a block
+
+// Forward step j: y_j = L_jj^-1 b_j, b[j0 + 64 : r_end) -= L[.., j] y_j.
+__global__ void __launch_bounds__(kSolT) forward_step(const double* __restrict__ L, int j0, int r_end, int lda,
+                                                     const double* __restrict__ inv, double* __restrict__ b,
+                                                     double* __restrict__ y, const int* __restrict__ info) {
+    __shared__ double part[4][NB], bs[NB], x[NB], red[kSolRows][kSolT / kSolRows + 1];
+    const int lr = threadIdx.x & (kSolRows - 1), kg = threadIdx.x / kSolRows;  // row, group of four columns
+    double m[16], l[4] = {0.0, 0.0, 0.0, 0.0};
+    load_tile_cols<true>(inv + static_cast<long long>(j0) * NB, m);
+    int r = j0 + NB + blockIdx.x * kSolRows + lr;
+    if (r < r_end) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) l[i] = L[r + static_cast<long long>(j0 + 4 * kg + i) * lda];
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (*info) return;
+    if (threadIdx.x < NB) bs[threadIdx.x] = b[j0 + threadIdx.x];
+    __syncthreads();
+    tile_product<true>(m, bs, part, x);
+    if (blockIdx.x == 0 && threadIdx.x < NB) y[j0 + threadIdx.x] = x[threadIdx.x];
+    for (int base = j0 + NB + blockIdx.x * kSolRows; base < r_end; base += gridDim.x * kSolRows) {
+        const int nr = base + gridDim.x * kSolRows + lr;
+        const double s = fma(l[0], x[4 * kg], l[1] * x[4 * kg + 1]) + fma(l[2], x[4 * kg + 2], l[3] * x[4 * kg + 3]);
+        if (nr < r_end) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) l[i] = L[nr + static_cast<long long>(j0 + 4 * kg + i) * lda];
+        }
+        red[lr][kg] = s;
+        __syncthreads();
+        // sixteen partial sums per row, added by a half-warp tree
+        double v = red[kg][lr];
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, 16);
+        if (lr == 0 && base + kg < r_end) b[base + kg] -= v;
+        __syncthreads();
+    }
+}
+
+// Backward step j: x_j = L_jj^-T y_j (into b), y[i0 : j0) -= L[j, ..]^T x_j.
+__global__ void __launch_bounds__(kSolT) backward_step(const double* __restrict__ L, int i0, int j0, int lda,
+                                                      const double* __restrict__ invt, double* __restrict__ y,
+                                                      double* __restrict__ b, const int* __restrict__ info) {
+    __shared__ double part[4][NB], bs[NB], x[NB];
+    const int kg = threadIdx.x & 15, lc = threadIdx.x >> 4;  // group of four rows, column
+    double m[16], l[4] = {0.0, 0.0, 0.0, 0.0};
+    load_tile_cols<false>(invt + static_cast<long long>(j0) * NB, m);
+    int c = i0 + blockIdx.x * kSolRows + lc;
+    if (c < j0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) l[i] = L[j0 + 4 * kg + i + static_cast<long long>(c) * lda];
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (*info) return;
+    if (threadIdx.x < NB) bs[threadIdx.x] = y[j0 + threadIdx.x];
+    __syncthreads();
+    tile_product<false>(m, bs, part, x);
+    if (blockIdx.x == 0 && threadIdx.x < NB) b[j0 + threadIdx.x] = x[threadIdx.x];
+    for (; c - lc < j0; c += gridDim.x * kSolRows) {
+        double v = fma(l[0], x[4 * kg], l[1] * x[4 * kg + 1]) + fma(l[2], x[4 * kg + 2], l[3] * x[4 * kg + 3]);
+        const int nc = c + gridDim.x * kSolRows;
+        if (nc < j0) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) l[i] = L[j0 + 4 * kg + i + static_cast<long long>(nc) * lda];
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, 16);
+        if (kg == 0 && c < j0) y[c] -= v;
+    }
 }
 
 }  // namespace
@@ -485,29 +550,32 @@ void dense_potrf(double* A, int n, int lda, int bt, int* info, cudaStream_t s) {
     }
 }
 
-void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* info, cudaStream_t s) {
+size_t dense_potrs_workspace(int n) { return (2ull * NB + 1) * n * sizeof(double); }
+
+void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* info, void* workspace,
+                 cudaStream_t s) {
     if (n % NB != 0 || bt < 0 || (bt < n / NB - 1 ? lda + 1 < (bt + 2) * NB : lda < n))
         throw std::invalid_argument("dense_potrs: n must be a multiple of 64 and lda hold the band");
     const int nt = n / NB;
+    double* inv = static_cast<double*>(workspace);
+    double* invt = inv + static_cast<size_t>(NB) * n;
+    double* y = invt + static_cast<size_t>(NB) * n;
+    const int xsm = NB * (NB + 1) * sizeof(double);
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(tile_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, xsm));
+    launch_pdl(tile_inverse, nt, kInvT, xsm, s, L, lda, inv, invt, info);
+    // Two passes of a block at most where the rows allow it: a further pass costs
+    // a block less than a further block costs the launch.
+    const int most = 2 * device_sm_count();
     for (int jb = 0; jb < nt; ++jb) {
         const int j0 = jb * NB;
-        trsv_lower_diag<<<1, NB, 0, s>>>(L, j0, lda, b, info);
-        GBA_LAUNCH_CHECK();
         const int r_end = static_cast<int>(std::min<long long>(n, j0 + NB + (long long)bt * NB));
-        if (j0 + NB < r_end) {
-            gemv_lower_below<<<ceil_div(r_end - j0 - NB, 256), 256, 0, s>>>(L, j0, r_end, lda, b, info);
-            GBA_LAUNCH_CHECK();
-        }
+        const int grid = std::max(1, std::min(most, ceil_div(r_end - j0 - NB, kSolRows)));
+        launch_pdl(forward_step, grid, kSolT, 0, s, L, j0, r_end, lda, inv, b, y, info);
     }
     for (int jb = nt - 1; jb >= 0; --jb) {
-        const int j0 = jb * NB;
-        trsv_upper_diag<<<1, NB, 0, s>>>(L, j0, lda, b, info);
-        GBA_LAUNCH_CHECK();
-        const int i0 = std::max(0, j0 - bt * NB);
-        if (j0 > i0) {
-            gemv_upper_above<<<ceil_div(32ll * (j0 - i0), 256), 256, 0, s>>>(L, i0, j0, lda, b, info);
-            GBA_LAUNCH_CHECK();
-        }
+        const int j0 = jb * NB, i0 = std::max(0, j0 - bt * NB);
+        const int grid = std::max(1, std::min(most, ceil_div(j0 - i0, kSolRows)));
+        launch_pdl(backward_step, grid, kSolT, 0, s, L, i0, j0, lda, invt, y, b, info);
     }
 }
 
@@ -525,6 +593,7 @@ void Solver::ensure_schur_storage() {
     band_mode_ = band;
     S_.release();
     S_.alloc(static_cast<size_t>(n_pad_) * (band ? band_ldb_ : n_pad_));
+    if (!chol_ws_.get()) chol_ws_.alloc(dense_potrs_workspace(n_pad_));
     schur_layout_planned_ = want;
 }
 
@@ -573,7 +642,7 @@ int Solver::schur_dense(double lambda) {
         GBA_CUDA_CHECK(cudaMemcpyAsync(pcg_x_.get(), rhs_.get(), n_pad_ * sizeof(double), cudaMemcpyDeviceToDevice,
                                        stream_));
     }
-    dense_potrs(S_.get(), n_pad_, lda, bt, pcg_x_.get(), info_.get(), stream_);
+    dense_potrs(S_.get(), n_pad_, lda, bt, pcg_x_.get(), info_.get(), chol_ws_.get(), stream_);
     if (band_mode_) {
         permute_cameras<<<ceil_div(9 * C_, 256), 256, 0, stream_>>>(perm, C_, false, pcg_x_.get(), dc_.get());
         GBA_LAUNCH_CHECK();

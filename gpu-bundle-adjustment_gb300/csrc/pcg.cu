@@ -2031,25 +2031,6 @@ __global__ void __launch_bounds__(kSL) sdiag_finalize_lane(const int* __restrict
 
 }  // namespace
 
-// Launch of a kernel of the PCG iteration chain with programmatic stream
-// serialization: it may be scheduled while the kernel before it finishes, and
-// waits for it in pdl_wait().
-template <typename... KArgs, typename... Args>
-static void launch_chained(void (*kernel)(KArgs...), int grid, int block, cudaStream_t stream, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(static_cast<unsigned>(grid));
-    cfg.blockDim = dim3(static_cast<unsigned>(block));
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    GBA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...));
-    count_launch();
-}
-
 // Implicit product partials for a given x (FP32 or float-float arithmetic). x
 // is in the arithmetic type (FP32: the PCG direction copy; float-float: dc) or
 // null (then a = 1: the right-hand side). Partials in cam_part_ (9 per chunk).
@@ -2100,13 +2081,13 @@ static void camera_parts_ff(Solver& s) {
 static void implicit_parts_acc(Solver& s, const float* x, const double* done) {
     cudaEvent_t ev = s.prof_start();
     if (s.n_wchunk_ > 0) {
-        launch_chained(schur_matvec_warp, ceil_div(s.n_wchunk_, kMWarps), 32 * kMWarps, s.stream_,
+        launch_pdl(schur_matvec_warp, ceil_div(s.n_wchunk_, kMWarps), 32 * kMWarps, 0, s.stream_,
                        reinterpret_cast<const int2*>(s.wchunk_.get()), s.n_wchunk_, s.s_cam_.get(), s.s_pt_.get(),
                        s.acc_id_.get(), s.Jc32_.get(), s.Jp32_.get(), s.js_, s.Vinv32_.get(), x, s.y_acc_.get(),
                        done);
     }
     if (s.n_lchunk_ > 0) {  // points with 33 to 256 observations, packed per CTA
-        launch_chained(schur_matvec_long, s.n_lchunk_, kPT, s.stream_,
+        launch_pdl(schur_matvec_long, s.n_lchunk_, kPT, 0, s.stream_,
                        reinterpret_cast<const int2*>(s.lchunk_.get()), s.lpts_.get(), s.pt_off_.get(),
                        s.s_cam_.get(), s.acc_id_.get(), s.Jc32_.get(), s.Jp32_.get(), s.js_, s.Vinv32_.get(), x,
                        s.y_acc_.get(), done);
@@ -2262,7 +2243,7 @@ PcgStats Solver::schur_pcg(double lambda, const LMOptions& opts, bool learned, u
                 if (one_pass_) {
                     implicit_parts_acc(*this, pcg_p32_.get(), done);
                     cudaEvent_t fev = prof_start();
-                    launch_chained(pcg_q_finalize_acc, npq, kVT, stream_, y_acc_.get(), acc_off_.get(),
+                    launch_pdl(pcg_q_finalize_acc, npq, kVT, 0, stream_, y_acc_.get(), acc_off_.get(),
                                    ul32_.get(), pcg_p32_.get(), C_, pcg_q_.get(), red_pq, sc);
                     prof_stop("pcg_q_finalize", fev);
                 } else {
@@ -2273,17 +2254,17 @@ PcgStats Solver::schur_pcg(double lambda, const LMOptions& opts, bool learned, u
                     GBA_LAUNCH_CHECK();
                     prof_stop("pcg_q_finalize", fev);
                 }
-                launch_chained(pcg_update, nub, kUT, stream_, pcg_e_.get(), pcg_r_.get(), pcg_z_.get(),
+                launch_pdl(pcg_update, nub, kUT, 0, stream_, pcg_e_.get(), pcg_r_.get(), pcg_z_.get(),
                                pcg_p32_.get(), pcg_q_.get(), Pinv_.get(), C_, red_pq, npq, red, red2, sc, Zc, red_zr);
                 if (coarse) {
                     cudaEvent_t cev = prof_start();
-                    launch_chained(coarse_w, nub, kUT, stream_, pcg_r_.get(), csz32_.get(), Pinv_.get(),
+                    launch_pdl(coarse_w, nub, kUT, 0, stream_, pcg_r_.get(), csz32_.get(), Pinv_.get(),
                                    ceinv_.get(), C_, red_zr, nub, c1, pcg_z_.get(), red_szw, sc, 0);
-                    launch_chained(coarse_z, nub, kUT, stream_, pcg_r_.get(), Zc, ceinv_.get(), C_, red_szw, nub,
+                    launch_pdl(coarse_z, nub, kUT, 0, stream_, pcg_r_.get(), Zc, ceinv_.get(), C_, red_szw, nub,
                                    c1, pcg_z_.get(), static_cast<float*>(nullptr), red2, sc, 0);
                     prof_stop("coarse_apply", cev);
                 }
-                launch_chained(pcg_direction, nvb, kVT, stream_, pcg_p32_.get(), pcg_z_.get(), n, red, red2, nub,
+                launch_pdl(pcg_direction, nvb, kVT, 0, stream_, pcg_p32_.get(), pcg_z_.get(), n, red, red2, nub,
                                max_iters, sc);
             }
             read_back({{h, sc, sizeof h}});

@@ -270,6 +270,7 @@ public:
     DevBuf<int> pair_e_, pair_f_, block_off_, block_ce_, block_cf_;
     DevBuf<double> T_, S_, rhs_, dc_, dp_, red_part_;
     DevBuf<int> info_;
+    DevBuf<unsigned char> chol_ws_;  // workspace of dense_potrs, allocated with S_
     // mixed Schur
     DevBuf<double> Sdiag_, Pfac_;  // S diagonal blocks (81C), preconditioner factors (packed, 45 per camera)
     DevBuf<float> Pinv_;           // explicit preconditioner blocks M_c = (L L^T)^-1 (81C, FP32)
@@ -368,8 +369,12 @@ void launch_batch_inverse3_spd(const double* A, double* Ainv, int* ok, int n, cu
 // else the 1-based failed column.
 void dense_potrf(double* A, int n, int lda, int bt, int* info, cudaStream_t s);
 
-// Solves L L^T x = b in place (b on the device, length n), L from dense_potrf.
-void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* info, cudaStream_t s);
+// Solves L L^T x = b in place (b on the device, length n), L from dense_potrf
+// (nothing is done where *info != 0). workspace: dense_potrs_workspace(n) bytes of
+// device memory, the call's own until the stream has passed it.
+size_t dense_potrs_workspace(int n);
+void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* info, void* workspace,
+                 cudaStream_t s);
 // Residual + Jacobian for E independent observations (device pointers, original
 // layout). Jc, Jp may be null. FP64 or FP32 arithmetic.
 void launch_eval_edges_f64(const double* cams, const double* pts, const int* oc, const int* op,
