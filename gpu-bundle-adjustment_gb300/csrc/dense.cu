@@ -34,24 +34,54 @@ namespace {
 constexpr int NB = 64;       // panel width / tile size
 constexpr int kSP = NB + 8;  // shared-memory stride (doubles) of K-major tiles: conflict-free DMMA fragments
 
-__global__ void compute_T_kernel(const double* __restrict__ W, const double* __restrict__ Vinv,
-                                 const int* __restrict__ s_pt, int E, double* __restrict__ T) {
-    for (long long s = blockIdx.x * (long long)blockDim.x + threadIdx.x; s < E; s += (long long)gridDim.x * blockDim.x) {
-        const double* Vi = Vinv + 6ll * s_pt[s];
-        const double v00 = Vi[0], v10 = Vi[1], v11 = Vi[2], v20 = Vi[3], v21 = Vi[4], v22 = Vi[5];
-        const double* We = W + 27 * s;
-        double* Te = T + 27 * s;
-#pragma unroll
-        for (int i = 0; i < 9; ++i) {
-            const double w0 = We[3 * i], w1 = We[3 * i + 1], w2 = We[3 * i + 2];
-            Te[3 * i] = w0 * v00 + w1 * v10 + w2 * v20;
-            Te[3 * i + 1] = w0 * v10 + w1 * v11 + w2 * v21;
-            Te[3 * i + 2] = w0 * v20 + w1 * v21 + w2 * v22;
-        }
-    }
+// T_e = W_e V'^-1 (9 x 3, row by row) and T_e bp_p at the observation's
+// camera-major position (tb, 9 values), for the right-hand side. One thread per
+// row: 24 contiguous bytes in and out.
+constexpr int kTT = 288;
+__global__ void __launch_bounds__(kTT) compute_T_kernel(const double* __restrict__ W, const double* __restrict__ Vinv,
+                                                       const double* __restrict__ bp, const int* __restrict__ s_pt,
+                                                       const int* __restrict__ cam_pos, int E, double* __restrict__ T,
+                                                       double* __restrict__ tb) {
+    const long long t = blockIdx.x * static_cast<long long>(kTT) + threadIdx.x;
+    if (t >= 9ll * E) return;
+    const long long s = t / 9;
+    const int i = static_cast<int>(t - 9 * s);
+    const long long p = s_pt[s];
+    const double* Vi = Vinv + 6 * p;
+    const double* b = bp + 3 * p;
+    const double w0 = W[3 * t], w1 = W[3 * t + 1], w2 = W[3 * t + 2];
+    const double t0 = w0 * Vi[0] + w1 * Vi[1] + w2 * Vi[3];
+    const double t1 = w0 * Vi[1] + w1 * Vi[2] + w2 * Vi[4];
+    const double t2 = w0 * Vi[3] + w1 * Vi[4] + w2 * Vi[5];
+    T[3 * t] = t0;
+    T[3 * t + 1] = t1;
+    T[3 * t + 2] = t2;
+    tb[9ll * cam_pos[s] + i] = t0 * b[0] + t1 * b[1] + t2 * b[2];
 }
 
-// One thread per (block, row i): S(9ce+i, 9cf+j) = -sum_{(e,f) in block} T_e(i,:) . W_f(j,:)
+// acc_j += T_e(i,:) . W_f(j,:) for row i of the pair (e, f).
+__device__ __forceinline__ void add_pair(const double* __restrict__ T, const double* __restrict__ W, int e, int f, int i,
+                                         double (&acc)[9]) {
+    const double* Te = T + 27ll * e + 3 * i;
+    const double t0 = Te[0], t1 = Te[1], t2 = Te[2];
+    const double* Wf = W + 27ll * f;
+#pragma unroll
+    for (int j = 0; j < 9; ++j) acc[j] += t0 * Wf[3 * j] + t1 * Wf[3 * j + 1] + t2 * Wf[3 * j + 2];
+}
+
+// S(9ce + i, 9cf + j) = -v, or its transpose where the renumbering put the block above the diagonal.
+__device__ __forceinline__ void store_block(double* __restrict__ S, int lda, const int* __restrict__ perm, int ce, int cf,
+                                            int i, int j, double v) {
+    const long long pe = perm ? perm[ce] : ce, pf = perm ? perm[cf] : cf;
+    if (pe >= pf)
+        S[9 * pe + i + (9 * pf + j) * lda] = -v;
+    else
+        S[9 * pf + j + (9 * pe + i) * lda] = -v;
+}
+
+// Assembly of the blocks of at most kShortPairs pairs: one thread per (block, row i),
+// S(9ce+i, 9cf+j) = -sum_{(e,f) in block} T_e(i,:) . W_f(j,:). What bounds it: the
+// FP64 pipe (243 FMA per pair).
 __global__ void __launch_bounds__(288) assemble_kernel(const int* __restrict__ block_off,
                                                       const int* __restrict__ block_ce,
                                                       const int* __restrict__ block_cf, const int* __restrict__ pe,
@@ -62,29 +92,63 @@ __global__ void __launch_bounds__(288) assemble_kernel(const int* __restrict__ b
     const long long b = t / 9;
     const int i = static_cast<int>(t % 9);
     if (b >= nblocks) return;
+    const int q0 = block_off[b], q1 = block_off[b + 1];
+    if (q1 - q0 > Solver::kShortPairs) return;
     double acc[9];
 #pragma unroll
     for (int j = 0; j < 9; ++j) acc[j] = 0.0;
-    for (int q = block_off[b]; q < block_off[b + 1]; ++q) {
-        const double* Te = T + 27ll * pe[q] + 3 * i;
-        const double t0 = Te[0], t1 = Te[1], t2 = Te[2];
-        const double* Wf = W + 27ll * pf[q];
+    for (int q = q0; q < q1; ++q) add_pair(T, W, pe[q], pf[q], i, acc);
 #pragma unroll
-        for (int j = 0; j < 9; ++j) acc[j] += t0 * Wf[3 * j] + t1 * Wf[3 * j + 1] + t2 * Wf[3 * j + 2];
+    for (int j = 0; j < 9; ++j) store_block(S, lda, perm, block_ce[b], block_cf[b], i, j, acc[j]);
+}
+
+// The longer blocks (a camera's own block holds all its observations; with few
+// cameras, every block holds thousands of pairs), in chunks of kChunkPairs: one CTA
+// per chunk, thread (slice, row i) takes every kSlices-th pair, the slices added in
+// order; a thread per block and row ran one pair after the other (13.7 ms for 136
+// blocks of 84,000 observations; 0.15 ms by chunks).
+constexpr int kSlices = 32;
+__global__ void __launch_bounds__(9 * kSlices) assemble_chunks_kernel(const int4* __restrict__ chunks,
+                                                                     const int* __restrict__ pe,
+                                                                     const int* __restrict__ pf,
+                                                                     const double* __restrict__ T,
+                                                                     const double* __restrict__ W,
+                                                                     double* __restrict__ part) {
+    __shared__ double sh[kSlices][81];
+    const int4 c = chunks[blockIdx.x];  // block, first pair, end pair
+    const int slice = threadIdx.x / 9, i = threadIdx.x - 9 * slice;
+    double acc[9];
+#pragma unroll
+    for (int j = 0; j < 9; ++j) acc[j] = 0.0;
+    for (int q = c.y + slice; q < c.z; q += kSlices) add_pair(T, W, pe[q], pf[q], i, acc);
+#pragma unroll
+    for (int j = 0; j < 9; ++j) sh[slice][9 * i + j] = acc[j];
+    __syncthreads();
+    // 81 sums of kSlices values, three threads each (a third of the slices in order)
+    __shared__ double third[3][81];
+    if (threadIdx.x < 243) {
+        const int k = threadIdx.x % 81, g = threadIdx.x / 81;
+        double v = 0.0;
+        for (int sl = 11 * g; sl < min(kSlices, 11 * g + 11); ++sl) v += sh[sl][k];
+        third[g][k] = v;
     }
-    const int pe_ = perm ? perm[block_ce[b]] : block_ce[b];
-    const int pf_ = perm ? perm[block_cf[b]] : block_cf[b];
-    if (pe_ >= pf_) {
-        const long long row = 9ll * pe_ + i;
-        const long long col0 = 9ll * pf_;
-#pragma unroll
-        for (int j = 0; j < 9; ++j) S[row + (col0 + j) * lda] = -acc[j];
-    } else {  // the renumbering put the block above the diagonal: store its transpose
-        const long long col = 9ll * pe_ + i;
-        const long long row0 = 9ll * pf_;
-#pragma unroll
-        for (int j = 0; j < 9; ++j) S[(row0 + j) + col * lda] = -acc[j];
-    }
+    __syncthreads();
+    if (threadIdx.x < 81)
+        part[81ll * blockIdx.x + threadIdx.x] = (third[0][threadIdx.x] + third[1][threadIdx.x]) + third[2][threadIdx.x];
+}
+
+// S blocks from their chunks' sums, in order: long block l has chunks [off[l], off[l + 1]).
+__global__ void __launch_bounds__(96) assemble_finalize_kernel(const int* __restrict__ off,
+                                                              const int4* __restrict__ chunks,
+                                                              const int* __restrict__ block_ce,
+                                                              const int* __restrict__ block_cf,
+                                                              const double* __restrict__ part, int lda,
+                                                              const int* __restrict__ perm, double* __restrict__ S) {
+    if (threadIdx.x >= 81) return;
+    const int c0 = off[blockIdx.x], c1 = off[blockIdx.x + 1], b = chunks[c0].x;
+    double v = 0.0;
+    for (int c = c0; c < c1; ++c) v += part[81ll * c + threadIdx.x];
+    store_block(S, lda, perm, block_ce[b], block_cf[b], threadIdx.x / 9, threadIdx.x % 9, v);
 }
 
 // Diagonal blocks += U_c + lambda * max(diag U_c, 1e-12); identity on padding.
@@ -127,35 +191,42 @@ __global__ void permute_cameras(const int* __restrict__ perm, int C, bool to_ban
         out[t] = in[pos];
 }
 
-// rhs_c = bc_c - sum_{e in c} T_e bp_{p(e)}; one CTA per camera, ordered sums.
-__global__ void __launch_bounds__(128) rhs_kernel(const int* __restrict__ cam_off, const int* __restrict__ cam_slots,
-                                                 const int* __restrict__ s_pt, const double* __restrict__ T,
-                                                 const double* __restrict__ bp, const double* __restrict__ bc,
-                                                 double* __restrict__ rhs) {
-    __shared__ double wpart[4][9];
-    const int c = blockIdx.x;
-    double acc[9];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) acc[k] = 0.0;
-    for (int i = cam_off[c] + threadIdx.x; i < cam_off[c + 1]; i += 128) {
-        const int s = cam_slots[i];
-        const double* Te = T + 27ll * s;
-        const double* b = bp + 3ll * s_pt[s];
-        const double b0 = b[0], b1 = b[1], b2 = b[2];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) acc[k] += Te[3 * k] * b0 + Te[3 * k + 1] * b1 + Te[3 * k + 2] * b2;
+// Right-hand side: per camera chunk the sum of its T_e bp (tb, camera-major:
+// contiguous), thread (position, component), positions added in order; then
+// rhs_c = bc_c - the chunk sums in order.
+constexpr int kRhsPos = 28;
+__global__ void __launch_bounds__(9 * kRhsPos) rhs_chunks_kernel(const int* __restrict__ cchunk_begin,
+                                                                const int* __restrict__ cchunk_cam,
+                                                                const int* __restrict__ cam_off, int chunk_slots,
+                                                                const double* __restrict__ tb,
+                                                                double* __restrict__ part) {
+    __shared__ double sh[9 * kRhsPos];
+    const int k = blockIdx.x, b = cchunk_begin[k], e = min(b + chunk_slots, cam_off[cchunk_cam[k] + 1]);
+    double v0 = 0.0, v1 = 0.0;
+    const double* p = tb + 9ll * b;
+    const int n = 9 * (e - b);
+    int i = threadIdx.x;
+    for (; i + 9 * kRhsPos < n; i += 18 * kRhsPos) {
+        v0 += p[i];
+        v1 += p[i + 9 * kRhsPos];
     }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < 9; ++k) {
-        const double v = warp_sum(acc[k]);
-        if (lane == 0) wpart[warp][k] = v;
-    }
+    if (i < n) v0 += p[i];
+    sh[threadIdx.x] = v0 + v1;
     __syncthreads();
     if (threadIdx.x < 9) {
-        const double v = wpart[0][threadIdx.x] + wpart[1][threadIdx.x] + wpart[2][threadIdx.x] + wpart[3][threadIdx.x];
-        rhs[9ll * c + threadIdx.x] = bc[9ll * c + threadIdx.x] - v;
+        double v = 0.0;
+        for (int q = 0; q < kRhsPos; ++q) v += sh[9 * q + threadIdx.x];
+        part[9ll * k + threadIdx.x] = v;
     }
+}
+__global__ void rhs_finalize_kernel(const int* __restrict__ cam_chunk_off, const double* __restrict__ part,
+                                    const double* __restrict__ bc, int C, double* __restrict__ rhs) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= 9 * C) return;
+    const int c = t / 9, k = t - 9 * c;
+    double v = 0.0;
+    for (int q = cam_chunk_off[c]; q < cam_chunk_off[c + 1]; ++q) v += part[9ll * q + k];
+    rhs[t] = bc[t] - v;
 }
 
 // ---------------------------------------------------------------- Cholesky
@@ -602,8 +673,11 @@ int Solver::schur_dense(double lambda) {
     const int lda = band_mode_ ? band_ldb_ - 1 : n_pad_;
     const int bt = band_mode_ ? band_bt_ : n_pad_ / NB - 1;
     const int* perm = band_mode_ ? cam_perm_.get() : nullptr;
-    compute_T_kernel<<<std::min(ceil_div(E_, 256), 32 * device_sm_count()), 256, 0, stream_>>>(
-        W_.get(), Vinv_.get(), s_pt_.get(), E_, T_.get());
+    // T_e bp (9 per observation) in the place of the camera pass's Jacobian records
+    // (20 per observation), which are not read after it
+    double* tb = JcR_.get();
+    compute_T_kernel<<<ceil_div(9ll * E_, kTT), kTT, 0, stream_>>>(W_.get(), Vinv_.get(), bp_.get(), s_pt_.get(),
+                                                                 cam_pos_.get(), E_, T_.get(), tb);
     GBA_LAUNCH_CHECK();
     GBA_CUDA_CHECK(cudaMemsetAsync(S_.get(), 0, S_.size() * sizeof(double), stream_));
     if (n_blocks_ > 0) {
@@ -612,14 +686,30 @@ int Solver::schur_dense(double lambda) {
             block_off_.get(), block_ce_.get(), block_cf_.get(), pair_e_.get(), pair_f_.get(), T_.get(), W_.get(),
             n_blocks_, lda, perm, S_.get());
         GBA_LAUNCH_CHECK();
+        if (n_long_ > 0) {
+            const int4* chunks = reinterpret_cast<const int4*>(long_chunks_.get());
+            assemble_chunks_kernel<<<n_long_chunks_, 9 * kSlices, 0, stream_>>>(chunks, pair_e_.get(), pair_f_.get(),
+                                                                               T_.get(), W_.get(), long_part_.get());
+            GBA_LAUNCH_CHECK();
+            assemble_finalize_kernel<<<n_long_, 96, 0, stream_>>>(long_off_.get(), chunks, block_ce_.get(),
+                                                                  block_cf_.get(), long_part_.get(), lda, perm,
+                                                                  S_.get());
+            GBA_LAUNCH_CHECK();
+        }
         prof_stop("schur_assemble", ev);
     }
     add_damped_u_kernel<<<ceil_div(81ll * C_ + (n_pad_ - 9 * C_), 256), 256, 0, stream_>>>(U_.get(), lambda, C_,
                                                                                         n_pad_, lda, perm, S_.get());
     GBA_LAUNCH_CHECK();
     GBA_CUDA_CHECK(cudaMemsetAsync(rhs_.get(), 0, rhs_.size() * sizeof(double), stream_));
-    rhs_kernel<<<C_, 128, 0, stream_>>>(cam_off_.get(), cam_slots_.get(), s_pt_.get(), T_.get(), bp_.get(),
-                                        bc_.get(), rhs_.get());
+    if (n_cchunk_ > 0) {
+        rhs_chunks_kernel<<<n_cchunk_, 9 * kRhsPos, 0, stream_>>>(cchunk_begin_.get(), cchunk_cam_.get(),
+                                                                 cam_off_.get(), kCamChunkSlots, tb,
+                                                                 cam_part_.get());
+        GBA_LAUNCH_CHECK();
+    }
+    rhs_finalize_kernel<<<ceil_div(9ll * C_, 128), 128, 0, stream_>>>(cam_chunk_off_.get(), cam_part_.get(),
+                                                                     bc_.get(), C_, rhs_.get());
     GBA_LAUNCH_CHECK();
     if (harvest_) {
         if (!Sdiag_.get()) Sdiag_.alloc(81ull * C_);

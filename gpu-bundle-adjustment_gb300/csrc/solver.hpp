@@ -241,6 +241,7 @@ public:
     // 1e-8 on workload 3 ran out of steps): camera c's at [acc_off_[c],
     // acc_off_[c + 1]), the slot's in acc_id_.
     static constexpr int kAccSlots = 32;
+    static constexpr int kCamChunkSlots = 1024;  // most positions of a camera chunk
     bool one_pass_ = false;
     int n_acc_ = 0;
     // the warp-level point passes' work: warp chunks (whole points, at most
@@ -268,6 +269,13 @@ public:
     long long n_pairs_ = 0;
     int n_blocks_ = 0;
     DevBuf<int> pair_e_, pair_f_, block_off_, block_ce_, block_cf_;
+    // blocks of more than kShortPairs pairs, assembled in chunks of at most
+    // kChunkPairs: long_chunks_ int4 {block, first pair, end pair, 0}; long block
+    // l's chunks [long_off_[l], long_off_[l + 1]); long_part_ 81 sums per chunk
+    static constexpr int kShortPairs = 48, kChunkPairs = 256;
+    int n_long_ = 0, n_long_chunks_ = 0;
+    DevBuf<int> long_chunks_, long_off_;
+    DevBuf<double> long_part_;
     DevBuf<double> T_, S_, rhs_, dc_, dp_, red_part_;
     DevBuf<int> info_;
     DevBuf<unsigned char> chol_ws_;  // workspace of dense_potrs, allocated with S_

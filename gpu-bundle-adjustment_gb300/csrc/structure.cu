@@ -106,7 +106,7 @@ int device_sm_count() {
 namespace {
 
 constexpr int kPointChunk = 256;   // max slots (and max points) per point-pass CTA
-constexpr int kCamChunk = 1024;    // max slots per camera-pass CTA
+constexpr int kCamChunk = Solver::kCamChunkSlots;  // max slots per camera-pass CTA
 
 __global__ void iota_kernel(int* v, int n) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] = i;
@@ -290,6 +290,32 @@ __global__ void block_split_kernel(const unsigned long long* __restrict__ ukey, 
         const unsigned long long k = ukey[i];
         ce[i] = static_cast<int>(k / static_cast<unsigned long long>(C));
         cf[i] = static_cast<int>(k % static_cast<unsigned long long>(C));
+    }
+}
+
+// Per block of the pair list: 1 if long, and its chunks (packed: long << 32 | chunks).
+__global__ void long_count_kernel(const int* __restrict__ block_off, int nb, unsigned long long* __restrict__ cnt) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x) {
+        const int n = b < nb ? block_off[b + 1] - block_off[b] : 0;
+        cnt[b] = n > Solver::kShortPairs
+                     ? (1ull << 32) + static_cast<unsigned>((n + Solver::kChunkPairs - 1) / Solver::kChunkPairs)
+                     : 0ull;
+    }
+}
+// Their chunk table, from the exclusive sums of those counts (blocks and chunks below 2^32).
+__global__ void long_fill_kernel(const int* __restrict__ block_off, const unsigned long long* __restrict__ base, int nb,
+                                 int4* __restrict__ chunks, int* __restrict__ off) {
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b <= nb; b += gridDim.x * blockDim.x) {
+        const int l = static_cast<int>(base[b] >> 32), c0 = static_cast<int>(base[b] & 0xffffffffu);
+        if (b == nb) {
+            off[l] = c0;
+            continue;
+        }
+        if (base[b + 1] == base[b]) continue;
+        off[l] = c0;
+        const int q1 = block_off[b + 1];
+        for (int q = block_off[b], c = c0; q < q1; q += Solver::kChunkPairs, ++c)
+            chunks[c] = make_int4(b, q, min(q1, q + Solver::kChunkPairs), 0);
     }
 }
 
@@ -703,6 +729,29 @@ void Solver::build_pairs() {
     }
     block_split_kernel<<<grid_for(nb), 256, 0, stream_>>>(ukey.get(), nb, C, block_ce_.get(), block_cf_.get());
     GBA_LAUNCH_CHECK();
+    // the long blocks' chunks (in block order)
+    DevBuf<unsigned long long> lcnt(nb + 1ull), lbase(nb + 1ull);
+    long_count_kernel<<<grid_for(nb + 1ll), 256, 0, stream_>>>(block_off_.get(), nb, lcnt.get());
+    GBA_LAUNCH_CHECK();
+    tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, lcnt.get(), lbase.get(), nb + 1, stream_);
+    {
+        DevBuf<unsigned char> tmp(tb);
+        GBA_CUDA_CHECK(cub::DeviceScan::ExclusiveSum(tmp.get(), tb, lcnt.get(), lbase.get(), nb + 1, stream_));
+    }
+    unsigned long long nlong = 0;
+    read_back({{&nlong, lbase.get() + nb, sizeof nlong}});
+    n_long_ = static_cast<int>(nlong >> 32);
+    n_long_chunks_ = static_cast<int>(nlong & 0xffffffffu);
+    if (n_long_ > 0) {
+        long_chunks_.alloc(4ull * n_long_chunks_);
+        long_off_.alloc(n_long_ + 1ull);
+        long_part_.alloc(81ull * n_long_chunks_);
+        long_fill_kernel<<<grid_for(nb + 1ll), 256, 0, stream_>>>(block_off_.get(), lbase.get(), nb,
+                                                                  reinterpret_cast<int4*>(long_chunks_.get()),
+                                                                  long_off_.get());
+        GBA_LAUNCH_CHECK();
+    }
     sync();
 }
 
