@@ -28,6 +28,7 @@ LIB_SOURCES = [
     "structure.cu",
     "edge.cu",
     "blocks.cu",
+    "chol.cu",
     "dense.cu",
     "pcg.cu",
     "mlp.cu",

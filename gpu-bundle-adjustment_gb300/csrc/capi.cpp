@@ -61,8 +61,13 @@ void need(bool ok, const char* what) {
     if (!ok) throw std::invalid_argument(what);
 }
 
-// dense_potrs with its workspace allocated and freed on the caller's stream
-// (from the device's memory pool, as the solvers' buffers are).
+// dense_potrf and dense_potrs with their workspaces allocated and freed on the
+// caller's stream (from the device's memory pool, as the solvers' buffers are).
+void potrf_with_workspace(double* A, int n, int lda, int bt, int* info, cudaStream_t stream) {
+    gba::StreamAllocScope scope(stream);
+    gba::DevBuf<unsigned char> ws(gba::dense_potrf_workspace(n));
+    gba::dense_potrf(A, n, lda, bt, info, ws.get(), stream);
+}
 void potrs_with_workspace(const double* L, int n, int lda, int bt, double* b, const int* info, cudaStream_t stream) {
     gba::StreamAllocScope scope(stream);
     gba::DevBuf<unsigned char> ws(gba::dense_potrs_workspace(n));
@@ -627,7 +632,7 @@ int gba_dense_potrf(double* A, int n, int lda, int* info, void* stream) {
     return guarded([&] {
         need(A && info, "null argument");
         need(n > 0 && n % 64 == 0 && lda >= n, "n must be a positive multiple of 64 and lda >= n");
-        gba::dense_potrf(A, n, lda, n / 64 - 1, info, static_cast<cudaStream_t>(stream));
+        potrf_with_workspace(A, n, lda, n / 64 - 1, info, static_cast<cudaStream_t>(stream));
     });
 }
 
@@ -644,7 +649,7 @@ int gba_band_potrf(double* AB, int n, int ldb, int bt, int* info, void* stream) 
         need(AB && info, "null argument");
         need(n > 0 && n % 64 == 0, "n must be a positive multiple of 64");
         need(bt >= 0 && ldb >= (bt + 2) * 64, "ldb must be at least (bt + 2) * 64");
-        gba::dense_potrf(AB, n, ldb - 1, bt, info, static_cast<cudaStream_t>(stream));
+        potrf_with_workspace(AB, n, ldb - 1, bt, info, static_cast<cudaStream_t>(stream));
     });
 }
 

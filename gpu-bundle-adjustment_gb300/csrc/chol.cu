@@ -1,0 +1,842 @@
+// Blocked Cholesky factorisation of dense and band SPD matrices in scaled
+// 64-bit fixed point (fix64.cuh), with the trailing update on the 5th-generation
+// tensor cores.
+//
+// Reference: the host Eigen LLT of the reduced camera system (src/lm.cu:598-604).
+//
+// GB300's FP64 pipe is the bound of an FP64 factorisation: 1.05 TFLOP/s for the
+// chip, 64 cycles per warp FMA, whether by DFMA or DMMA. Here no FP64
+// arithmetic is left on the path:
+//   scale     row exponents e_i from the diagonal (A_ii 2^(-2 e_i) in [1/8, 1/2))
+//   convert   the lower triangle, in place, to 64-bit integers (2^-60 units)
+//   per 64-column panel
+//     panel   the 64 x 64 diagonal tile and the rows below it (chol_panel): the
+//             factor's columns as FP64 in place, and the rows' base-512 digits
+//             as FP16 tiles for the update
+//     update  C -= L L^T over the remaining lower tiles (chol_update): the
+//             digit products by tcgen05.mma (FP16 in, FP32 accumulators in
+//             TMEM, exact: small integers), recombined into the 64-bit entries
+// Every entry is an exact sum of products rounded at 2^-60 of
+// sqrt(A_ii A_jj), so the factor is closer to the exact one than FP64's.
+//
+// A row that cannot belong to an SPD matrix (a diagonal entry that is not
+// positive, an entry that is not finite or larger than the diagonal allows, a
+// row of the factor that outgrows its diagonal entry) is marked in bad[]: its
+// entries count as zero, and the factorisation stops at its pivot, as FP64
+// arithmetic does at the negative or NaN pivot it meets there. An infinite
+// diagonal entry is a pivot of weight infinity: its row and column of the
+// factor are zero.
+//
+// Tile addressing: element (i, j) at A[i + j lda] in both layouts (dense.cu).
+
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <climits>
+
+#include "common.cuh"
+#include "fix64.cuh"
+#include "solver.hpp"
+
+namespace gba {
+namespace {
+
+using fx::Acc;
+using fx::Limbs;
+
+constexpr int NB = 64;                        // panel width / tile size
+constexpr int kTileB = NB * NB * 2;           // bytes of one FP16 digit tile
+constexpr int kNS = fx::kSlices;
+
+// Workspace: digit tiles (kNS per 64-row tile), row exponents, row flags.
+struct Work {
+    unsigned char* tiles;
+    int* e;
+    int* bad;  // 1: fails at this row's pivot; 2: infinite diagonal entry
+};
+Work carve(void* ws, int n) {
+    Work w;
+    w.tiles = static_cast<unsigned char*>(ws);
+    w.e = reinterpret_cast<int*>(w.tiles + static_cast<size_t>(n / NB) * kNS * kTileB);
+    w.bad = w.e + n;
+    return w;
+}
+
+__global__ void chol_scale(const double* __restrict__ A, int n, int lda, int* __restrict__ e, int* __restrict__ bad,
+                           int* __restrict__ info) {
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) *info = 0;
+    if (i >= n) return;
+    const double d = A[i + static_cast<long long>(i) * lda];
+    const bool ok = fx::finite_positive(d);
+    e[i] = ok ? fx::row_exponent(d) : 0;
+    bad[i] = ok ? 0 : d > 0.0 ? 2 : 1;
+}
+
+// One CTA per lower tile (ti, tj), ti - tj <= bt: FP64 -> fixed point in place.
+// The strict upper triangle of a diagonal tile is not touched.
+__global__ void __launch_bounds__(256) chol_convert(double* __restrict__ A, int nt, int lda, int bt,
+                                                   const int* __restrict__ e, int* __restrict__ bad) {
+    const int tj = blockIdx.x, ti = tj + blockIdx.y;
+    if (ti >= nt) return;
+    pdl_wait();
+    pdl_trigger();
+    const int r = threadIdx.x & 63, i = ti * NB + r;
+    const int ei = e[i];
+    const bool inf_row = bad[i] == 2;
+    long long* F = reinterpret_cast<long long*>(A);
+    bool mine = false;
+    double v[16];
+    int ec[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const int j = tj * NB + (threadIdx.x >> 6) + 4 * k;
+        v[k] = j <= i && bad[j] != 2 ? A[i + static_cast<long long>(j) * lda] : 0.0;
+        ec[k] = e[j];
+    }
+#pragma unroll
+    for (int k = 0; k < 16; ++k) {
+        const int j = tj * NB + (threadIdx.x >> 6) + 4 * k;
+        if (j > i) continue;
+        bool b = false;
+        long long f = fx::to_fixed(v[k], ei + ec[k], &b);
+        if (inf_row) {
+            f = 0;
+            b = false;
+        }
+        F[i + static_cast<long long>(j) * lda] = f;
+        mine = mine || b;
+    }
+    if (mine) bad[i] = 1;
+}
+
+// ---------------------------------------------------------------- panel
+//
+// One CTA factors the panel's diagonal tile (every CTA of the grid does, each
+// for itself: the tile is the critical path, and the SMs would idle otherwise)
+// together with 16 rows below it, then solves the further rows it was given.
+//
+// What bounds it is the chain of 64 pivots, each a reciprocal square root and
+// three dependent 64-bit products (some 400 cycles), so one warp does nothing
+// else, alone on its SM sub-partition: the pivot warp holds a window of 32 rows,
+// one per lane (rows 0 to 31 of the tile for its first 32 columns, then rows 32 to
+// 63), and advances four columns a round without waiting for anybody: it
+// applies the previous round's rank-4 update to the next four columns itself.
+// On the other three sub-partitions ten warps hold all rows (a thread owns one
+// row and the columns j = 4 m + q of it, as 64-bit accumulators that shift
+// down by one slot a round) and apply the rounds' updates, the window's
+// columns two rounds ahead first; two warps solve the rows outside the window, a
+// row per lane, a round behind the pivot warp. The solving warps, whose chain
+// the others wait for, share theirs with the two lightest updating warps.
+constexpr int kWin = 32;                  // rows of the pivot warp's window
+constexpr int kExtra = 16;                // rows below the tile in the first group
+constexpr int kRows = NB + kExtra;
+constexpr int kOut = kRows - kWin;        // rows outside the first window
+constexpr int kUpdateWarps = kRows / 8;
+constexpr int kWorkers = 32 * (kUpdateWarps + 2);  // threads of the updating and solving warps
+constexpr int kPanelThreads = 512;        // warps 4, 8, 12 share the pivot warp's sub-partition and rest
+constexpr int kRows2 = kPanelThreads / 4; // rows per pass of the further rows
+constexpr int kLvS = NB + 1;              // stride of the row-major factor values
+constexpr int kLS = NB + 2;               // stride of the limbs of a row (16-byte aligned)
+
+struct PanelSmem {
+    Limbs L[NB * kLS];           // [row][column] limbs of the diagonal tile's factor
+    Limbs lx[kExtra * 4];        // [row][4] limbs of the current columns, rows below the tile
+    long long xw[2][4][kWin];    // the window's columns of a round (by the round's parity)
+    long long xn[4][kOut];       // the current four columns of the other rows
+    long long lv[kRows2 * kLvS]; // factor values by row, for the output
+    fx::Rsqrt y[NB];             // reciprocal pivots (y0 = 0: a pivot of weight infinity)
+    float rest[kWin];            // rows 32 to 63: what their squares leave of the diagonal entry
+    int diag_bad[NB];
+    int fail;                    // 1 + failed column of the tile
+    int fail_round;              // 1 + the round it is in (the pivot warp runs ahead of the others' checks)
+};
+
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory");
+}
+// Named barriers: the window's columns of round b are there; round b's pivots
+// are, for the updating and for the solving warps (apart: the solving warps
+// must not wait for the updating ones' last round); the solving warps are done;
+// the next columns are published; rows 32 to 63 are solved for columns 28 to
+// 31. The pivot warp is at most two rounds ahead of the updating warps (it waits for
+// the window's columns) and three of the solving ones, hence the two and four
+// barriers in turn.
+__device__ __forceinline__ int bar_window(int b) { return 1 + (b & 1); }
+__device__ __forceinline__ int bar_pivots(int b) { return 3 + (b & 1); }
+__device__ __forceinline__ int bar_pivots_solving(int b) { return 8 + (b & 3); }
+constexpr int kBarSolved = 5, kBarNext = 6, kBarHandover = 7;
+constexpr int kWindowCount = 32 + 32 * kUpdateWarps, kPivotsCount = 32 + 32 * kUpdateWarps, kPivotsSolving = 32 + 64;
+
+// Limbs of four consecutive columns.
+__device__ __forceinline__ void load_limbs4(const Limbs* p, Limbs (&l)[4]) {
+    const int4 a = reinterpret_cast<const int4*>(p)[0], b = reinterpret_cast<const int4*>(p)[1];
+    l[0] = {a.x, a.y};
+    l[1] = {a.z, a.w};
+    l[2] = {b.x, b.y};
+    l[3] = {b.z, b.w};
+}
+__device__ __forceinline__ void store_limbs4(Limbs* p, const Limbs (&l)[4]) {
+    reinterpret_cast<int4*>(p)[0] = make_int4(l[0].hi, l[0].lo, l[1].hi, l[1].lo);
+    reinterpret_cast<int4*>(p)[1] = make_int4(l[2].hi, l[2].lo, l[3].hi, l[3].lo);
+}
+
+// Squares of a row of the factor against its diagonal entry: a row that outgrows
+// it is not of an SPD matrix.
+__device__ __forceinline__ float square_of(long long x) {
+    const float f = static_cast<float>(static_cast<int>(x >> 32)) * 0x1p-28f;
+    return f * f;
+}
+
+// The pivot warp (rows 32 (b / 8) + lane in round b).
+__device__ __forceinline__ void pivot_warp(PanelSmem& sm, float diag) {
+    const int lane = threadIdx.x;
+    float rest = diag;
+    int state = sm.diag_bad[lane];  // 1: the row has failed, 2: a pivot of weight infinity
+    Limbs prev[4];
+#pragma unroll 1
+    for (int b = 0; b < 16; ++b) {
+        const int k0 = 4 * b, row = (b >> 3) * kWin + lane, p0 = k0 & (kWin - 1);
+        bar_sync(bar_window(b), kWindowCount);
+        if (b == 8) {  // the second window's rows come from the solving warp
+            bar_sync(kBarHandover, 64);
+            load_limbs4(sm.L + row * kLS + k0 - 4, prev);
+            rest = sm.rest[lane];
+            state = sm.diag_bad[row];
+        }
+        Acc t[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) t[c] = {sm.xw[b & 1][c][lane], 0};
+        if (b > 0) {  // the previous round's update of these columns
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                Limbs l[4];
+                load_limbs4(sm.L + (k0 + c) * kLS + k0 - 4, l);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) fx::fms(t[c], prev[k], l[k]);
+            }
+        }
+        long long x[4], dv = fx::value(t[0]);  // dv: the pivot, on its row's lane
+        int fail = 0;
+        float sq = 0.f;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const long long v = fx::value(t[c]);
+            const long long d = __shfl_sync(0xffffffffu, dv, p0 + c);
+            const int st = __shfl_sync(0xffffffffu, state, p0 + c);
+            if (!fail && (st == 1 || (st == 0 && d <= 0))) fail = k0 + c + 1;
+            fx::Rsqrt y = fx::rsqrt_fixed(d);  // (of a failed pivot: not used)
+            bool ob = false;
+            const long long ax = fx::scale_abs(v, y, &ob);
+            const Limbs al = fx::split(ax);
+            if (c < 3) {  // the next pivot, from its lane's own entry
+                Acc dn = t[c + 1];
+                if (st != 2) fx::fms(dn, al, al);
+                dv = fx::value(dn);
+            }
+            const bool zero = st == 2 || row < k0 + c;  // (or above the diagonal of the tile)
+            if (ob && !zero && state == 0) state = 1;
+            x[c] = zero ? 0 : v < 0 ? -ax : ax;
+            prev[c] = zero ? Limbs{0, 0} : v < 0 ? Limbs{-al.hi, -al.lo} : al;
+            if (lane == p0 + c) {
+                if (st == 2) y.y0 = 0;
+                sm.y[k0 + c] = y;
+            }
+            if (!zero) sq += square_of(ax);
+#pragma unroll
+            for (int r = c + 1; r < 4; ++r) {
+                Limbs l;
+                l.hi = __shfl_sync(0xffffffffu, prev[c].hi, p0 + r);
+                l.lo = __shfl_sync(0xffffffffu, prev[c].lo, p0 + r);
+                fx::fms(t[r], prev[c], l);
+            }
+        }
+        if (row >= k0 + 4) {  // below the pivot block: the squares stay within the diagonal entry
+            rest -= sq;
+            if (state == 0 && rest < -0.01f) state = 1;
+            if (state == 1) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) x[c] = 0, prev[c] = {0, 0};
+            }
+        }
+        store_limbs4(sm.L + row * kLS + k0, prev);
+        if (fail && lane == 0) {
+            sm.fail = fail;
+            sm.fail_round = b + 1;
+        }
+        __syncwarp();
+        bar_arrive(bar_pivots_solving(b), kPivotsSolving);
+        bar_arrive(bar_pivots(b), kPivotsCount);
+        if (fail) return;
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sm.lv[row * kLvS + k0 + c] = x[c];
+    }
+}
+
+// A solving warp: row g of the tile's rows (row >= 64: below it), a round behind the pivots.
+__device__ __forceinline__ void solving_warp(PanelSmem& sm, int g, bool live, float rest, bool* rbad) {
+    bar_sync(kBarNext, kWorkers);
+    Limbs* const mine = g < NB ? sm.L + g * kLS : sm.lx + 4 * (min(g, kRows - 1) - NB);
+    const int gn = min(g, kRows - 1) - kWin;
+#pragma unroll 1
+    for (int b = 0; b < 16; ++b) {
+        const int k0 = 4 * b;
+        bar_sync(bar_pivots_solving(b), kPivotsSolving);
+        if (sm.fail_round == b + 1) return;
+        if (g >= NB || b < 8) {  // rows 32 to 63 are the pivot warp's from round 8 on
+            Acc t[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) t[c] = {sm.xn[c][gn], 0};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int k = k0 + c;
+                const fx::Rsqrt y = sm.y[k];
+                bool ob = false;
+                long long x = y.y0 ? fx::scale(fx::value(t[0]), y, &ob) : 0;
+                rest -= square_of(x);
+                if (ob || rest < -0.01f) *rbad = true;
+                if (*rbad) x = 0;
+                const Limbs xl = fx::split(x);
+                if (live) {
+                    (g < NB ? mine + k : mine + c)[0] = xl;
+                    sm.lv[g * kLvS + k] = x;
+                }
+#pragma unroll
+                for (int r = 1; r < 4; ++r) {  // (past the round's columns: not used)
+                    fx::fms(t[r], xl, sm.L[min(k + r, NB - 1) * kLS + k]);
+                    t[r - 1] = t[r];
+                }
+            }
+            if (live && g < NB) {
+                sm.rest[g - kWin] = rest;
+                if (*rbad) sm.diag_bad[g] = 1;
+            }
+            if (b == 7 && g < NB) {
+                __syncwarp();
+                bar_arrive(kBarHandover, 64);
+            }
+        }
+        bar_arrive(kBarSolved, kWorkers);
+        if (b < 15) bar_sync(kBarNext, kWorkers);
+    }
+}
+
+// An updating warp: the thread's row g and columns 4 m + q.
+__device__ __forceinline__ void updating_warp(PanelSmem& sm, Acc (&a)[16], int g, int q) {
+    if (g < kWin) {
+        sm.xw[0][q][g] = a[0].c;
+        sm.xw[1][q][g] = a[1].c;
+    } else {
+        sm.xn[q][g - kWin] = a[0].c;
+    }
+    bar_arrive(bar_window(0), kWindowCount);
+    bar_arrive(bar_window(1), kWindowCount);
+    bar_arrive(kBarNext, kWorkers);
+    const int gw = g & ~7;  // the warp's first row (its rows share a window)
+#pragma unroll 1
+    for (int b = 0; b < 16; ++b) {
+        const int k0 = 4 * b, w0 = (b >> 3) * kWin, w1 = w0 + kWin;  // the window's rows
+        const bool window = gw >= w0 && gw < w1, outside = gw >= w1;
+        const Limbs* const col = sm.L + (k0 + q) * kLS + k0;  // limbs of row k0 + q, columns k0 ..
+        bar_sync(bar_pivots(b), kPivotsCount);
+        if (sm.fail_round == b + 1) return;
+        Limbs xr[4], l[4];
+        // the window's columns two rounds ahead (those of the next round are the pivot warp's)
+        if (window) {
+            load_limbs4(sm.L + g * kLS + k0, xr);
+            if (k0 + 8 < w1) {
+                load_limbs4(col + 8 * kLS, l);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) fx::fms(a[2], xr[c], l[c]);
+                sm.xw[b & 1][q][g - w0] = fx::value(a[2]);
+            }
+        }
+        if (b <= 13 && b != 6 && b != 7) bar_arrive(bar_window(b + 2), kWindowCount);
+        bar_sync(kBarSolved, kWorkers);
+        if (b == 15) break;
+        // the rows outside the window: the next round's columns first, for the solving warps
+        if (outside) {
+            load_limbs4(g < NB ? sm.L + g * kLS + k0 : sm.lx + 4 * (g - NB), xr);
+#pragma unroll
+            for (int m = 1; m < 3; ++m) {
+                if (m > 15 - b) break;
+                load_limbs4(col + 4 * m * kLS, l);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) fx::fms(a[m], xr[c], l[c]);
+            }
+            sm.xn[q][g - kWin] = fx::value(a[1]);
+            if (g < NB && (b == 6 || b == 7)) sm.xw[b & 1][q][g - kWin] = fx::value(a[2]);
+        }
+        if (b == 6 || b == 7) bar_arrive(bar_window(b + 2), kWindowCount);
+        bar_arrive(kBarNext, kWorkers);
+        // the columns further right, up to the window's, the row's or the panel's last
+        const int end = window ? min(w1, gw + 8) : outside ? min(NB, g < NB ? gw + 8 : NB) : 0;
+#pragma unroll
+        for (int m = 3; m < 16; ++m) {
+            if (k0 + 4 * m >= end) break;
+            load_limbs4(col + 4 * m * kLS, l);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) fx::fms(a[m], xr[c], l[c]);
+        }
+#pragma unroll
+        for (int m = 0; m < 15; ++m) a[m] = a[m + 1];
+    }
+}
+
+// FP64 columns and FP16 digit tiles of the rows in sm.lv[first, first + count):
+// row i of them is matrix row r0 + i.
+__device__ void panel_output(const PanelSmem& sm, int first, int count, int r0, double* __restrict__ A, int j0,
+                             int lda, const int* __restrict__ e, unsigned char* __restrict__ tiles) {
+    // digits: one thread per row and run of eight columns, a 16-byte store per digit,
+    // in the 128-byte-swizzled K-major layout that the update's MMA reads
+    for (int t = threadIdx.x; t < count * 8; t += kPanelThreads) {
+        const int i = t % count, kc = t / count;
+        const int r = r0 + i, rt = r & 63;
+        int q[8][kNS];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) fx::digits(sm.lv[(first + i) * kLvS + 8 * kc + k], q[k]);
+        unsigned char* dst =
+            tiles + static_cast<size_t>(r >> 6) * kNS * kTileB + (rt >> 3) * 1024 + (rt & 7) * 128 + ((kc ^ (rt & 7)) << 4);
+#pragma unroll
+        for (int s = 0; s < kNS; ++s) {
+            __half2 h[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                h[k] = __halves2half2(__int2half_rn(q[2 * k][s]), __int2half_rn(q[2 * k + 1][s]));
+            *reinterpret_cast<uint4*>(dst + s * kTileB) = *reinterpret_cast<uint4*>(h);
+        }
+    }
+    for (int t = threadIdx.x; t < count * NB; t += kPanelThreads) {
+        const int i = t % count, k = t / count;
+        const int r = r0 + i;
+        A[r + static_cast<long long>(j0 + k) * lda] = fx::to_double(sm.lv[(first + i) * kLvS + k], e[r]);
+    }
+}
+
+__global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restrict__ A, int j0, int lda, int nbelow,
+                                                              int rpc, const int* __restrict__ e,
+                                                              int* __restrict__ bad,
+                                                              unsigned char* __restrict__ tiles,
+                                                              int* __restrict__ info) {
+    extern __shared__ __align__(16) unsigned char panel_smem[];
+    PanelSmem& sm = *reinterpret_cast<PanelSmem*>(panel_smem);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    pdl_wait();
+    pdl_trigger();
+    // one read per block: block 0 of this grid may set the flag meanwhile
+    if (tid == 0) {
+        sm.fail = *info;
+        sm.fail_round = 0;
+    }
+    __syncthreads();
+    if (sm.fail) return;
+    const long long* F = reinterpret_cast<const long long*>(A);
+    const int b0 = blockIdx.x * rpc, b1 = min(nbelow, b0 + rpc);  // this CTA's rows below the tile
+    const int nx = max(0, min(kExtra, b1 - b0));                  // of them in the first group
+    if (tid < NB) sm.diag_bad[tid] = bad[j0 + tid];
+    // what the squares of a row of the factor may add up to, and whether it has failed
+    auto matrix_row = [&](int g) { return g < NB ? j0 + g : j0 + NB + b0 + (g - NB); };
+    auto diagonal = [&](int g) {
+        const int r = matrix_row(g);
+        return bad[r] == 2 ? 1.f : static_cast<float>(F[r + static_cast<long long>(r) * lda]) * 0x1p-60f;
+    };
+    __syncthreads();
+    // workers by sub-partition 1, 2, 3 (warp & 3) and slot (warp >> 2): updating
+    // warps 0 to 9 hold rows 8 w .., of which 4 to 9 have the most work; 10 and 11 solve
+    const int worker = (warp & 3) == 1 ? (warp >> 2 ? 2 + 2 * (warp >> 2) : 0)
+                       : (warp & 3) == 2 ? (warp >> 2 ? 3 + 2 * (warp >> 2) : 1)
+                                         : (warp >> 2 < 2 ? 2 + (warp >> 2) : 8 + (warp >> 2));
+    bool rbad = false;
+    int srow = -1;
+    if (warp == 0) {
+        pivot_warp(sm, diagonal(lane));
+    } else if ((warp & 3) == 0) {
+        // rests
+    } else if (worker < kUpdateWarps) {
+        const int g = 8 * worker + (lane >> 2), q = lane & 3;
+        const bool live = g < NB || g - NB < nx;
+        Acc a[16];
+#pragma unroll
+        for (int m = 0; m < 16; ++m) {
+            const int j = 4 * m + q;
+            a[m].c = live && (g >= NB || j <= g) ? F[matrix_row(g) + static_cast<long long>(j0 + j) * lda] : 0;
+            a[m].m = 0;
+        }
+        updating_warp(sm, a, g, q);
+    } else {
+        const int g = worker == kUpdateWarps ? kWin + lane : NB + lane;
+        const bool live = g < NB || g - NB < nx;
+        if (live) {
+            srow = g;
+            rbad = bad[matrix_row(g)] == 1;
+        }
+        solving_warp(sm, g, live, live ? diagonal(g) : 0.f, &rbad);
+    }
+    __syncthreads();
+    if (sm.fail) {
+        if (blockIdx.x == 0 && tid == 0) *info = j0 + sm.fail;
+        return;
+    }
+    if (srow >= NB && rbad) bad[matrix_row(srow)] = 1;
+    if (nx > 0) panel_output(sm, NB, nx, j0 + NB + b0, A, j0, lda, e, tiles);
+    if (blockIdx.x == 0) {  // the diagonal tile's factor
+        for (int t = tid; t < NB * NB; t += kPanelThreads) {
+            const int i = t & 63, k = t >> 6;
+            if (i < k) continue;
+            double v = fx::to_double(sm.lv[i * kLvS + k], e[j0 + i]);
+            if (i == k && sm.diag_bad[i] == 2) v = __longlong_as_double(0x7ff0000000000000ll);
+            A[(j0 + i) + static_cast<long long>(j0 + k) * lda] = v;
+        }
+    }
+    // further rows, kRows2 at a time: the factor is known, four threads of a
+    // warp solve a row with shuffles
+    for (int c0 = b0 + kExtra; c0 < b1; c0 += kRows2) {
+        const int g = tid >> 2, q = tid & 3;
+        const int n = min(kRows2, b1 - c0);
+        const int r = j0 + NB + c0 + g;
+        const bool lv = g < n;
+        bool rb = lv ? bad[r] == 1 : true;
+        float rs = lv ? static_cast<float>(F[r + static_cast<long long>(r) * lda]) * 0x1p-60f : 0.f;
+        if (lv && bad[r] == 2) rs = 1.f;
+        Acc a[16];
+#pragma unroll
+        for (int m = 0; m < 16; ++m) {
+            a[m].c = lv ? F[r + static_cast<long long>(j0 + 4 * m + q) * lda] : 0;
+            a[m].m = 0;
+        }
+        __syncthreads();  // sm.lv of the previous rows has been written out
+        if (8 * warp < n) {
+            for (int b = 0; b < 16; ++b) {
+                const int k0 = 4 * b;
+                Limbs xl[4], l[4];
+                load_limbs4(sm.L + (k0 + q) * kLS + k0, l);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    bool ob = false;
+                    long long x = 0;
+                    const fx::Rsqrt y = sm.y[k0 + c];
+                    if (q == c) {
+                        x = fx::scale(fx::value(a[0]), y, &ob);
+                        if (ob || rb || y.y0 == 0) x = 0;
+                    }
+                    const Limbs mine = fx::split(x);
+                    xl[c].hi = __shfl_sync(0xffffffffu, mine.hi, c, 4);
+                    xl[c].lo = __shfl_sync(0xffffffffu, mine.lo, c, 4);
+                    rb = __shfl_sync(0xffffffffu, ob ? 1 : 0, c, 4) || rb;
+                    const float xf = static_cast<float>(xl[c].hi) * 0x1p-30f;
+                    rs = fmaf(-xf, xf, rs);
+                    if (rs < -0.01f) rb = true;
+                    if (q == c) sm.lv[g * kLvS + k0 + c] = x;
+                    if (c < 3) fx::fms(a[0], xl[c], l[c]);  // columns left of q: not used again
+                }
+#pragma unroll
+                for (int m = 1; m < 16; ++m) {
+                    if (m > 15 - b) break;
+                    load_limbs4(sm.L + (4 * (b + m) + q) * kLS + k0, l);
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) fx::fms(a[m], xl[c], l[c]);
+                }
+#pragma unroll
+                for (int m = 0; m < 15; ++m) a[m] = a[m + 1];
+            }
+            if (lv && rb && q == 0) bad[r] = 1;
+        }
+        __syncthreads();
+        panel_output(sm, 0, n, j0 + NB + c0, A, j0, lda, e, tiles);
+    }
+}
+
+// ---------------------------------------------------------------- trailing update
+//
+// C(I, J) -= L(I) L(J)^T for the lower tiles: 128 rows (two 64-row tiles) by 64
+// columns, K = 64 (the panel). With L = sum_s q_s 2^(52 - 9 s), the products of
+// digits s and t weigh 2^(44 - 9 (s + t)) units: group d = s + t is summed in one
+// FP32 accumulator of 64 TMEM columns (7 groups: 448 of 512 columns); 28 digit
+// products of 4 MMAs (K = 16). The sums of groups 0 to 4 stay below 2^24 and
+// are exact; a rounding in groups 5 and 6, whose bound is 2^24.4, would weigh
+// at most one of the entries' 2^-60 units. The products left out
+// (d > 6) weigh a third of a unit (root mean square).
+//
+// One CTA per SM walks a contiguous run of tiles (row block by row block, so the
+// row block's digits are loaded once): warp 0 loads digit tiles (bulk copies,
+// columns double-buffered), warp 1 issues the MMAs, sixteen warps recombine. The
+// low groups (4, 5, 6) come first: the recombination of one part overlaps
+// the MMAs of the other. What bounds it: 28 x 4 MMAs of 128 x 64 x 16 a tile, which
+// read their operands from shared memory at 6 KB per MMA, and the 16 bytes of
+// each entry per panel from and to HBM.
+constexpr int kUpdWarps = 16;  // recombining warps: 32 rows x 16 columns each
+constexpr int kUpdThreads = 64 + 32 * kUpdWarps;
+constexpr int kABytes = kNS * 2 * kTileB, kBBytes = kNS * kTileB;
+constexpr int kUpdSmem = kABytes + 2 * kBBytes + 1024;
+constexpr int kWaitLimit = 1 << 18;  // polls of a barrier before a role gives up (then info = INT_MIN)
+
+enum { B_FULLA = 0, B_EMPTYA, B_FULLB, B_EMPTYB = 4, B_LOFULL = 6, B_LOEMPTY, B_HIFULL, B_HIEMPTY, B_COUNT };
+
+__device__ __forceinline__ uint32_t smem_u32(const void* p) {
+    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, int count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect(uint32_t bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait for the phase of the given parity; false when it gave up (or another role has).
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* gave_up) {
+    for (int i = 0; i < kWaitLimit; ++i) {
+        uint32_t done;
+        asm volatile(
+            "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+            : "=r"(done)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (done) return true;
+        if ((i & 1023) == 1023 && *gave_up) return false;
+    }
+    *gave_up = 1;
+    return false;
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+// K-major operand, rows of 128 bytes in 8-row groups of 1024 bytes, 128-byte swizzle.
+__device__ __forceinline__ uint64_t operand_desc(uint32_t addr) {
+    return static_cast<uint64_t>((addr & 0x3ffff) >> 4) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void mma_f16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n.reg .pred p;\nsetp.ne.b32 p, %4, 0;\n"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(accumulate ? 1u : 0u)
+        : "memory");
+}
+__device__ __forceinline__ void mma_commit(uint32_t bar) {
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ void tmem_load8(uint32_t addr, float (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7])
+                 : "r"(addr));
+}
+__device__ __forceinline__ void tmem_wait_load() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+
+// An integer-valued FP32 accumulator as an integer: by the add of 1.5 2^23 for
+// |v| < 2^22 (groups 0 and 1), else by conversion.
+__device__ __forceinline__ int small_int(float v) { return __float_as_int(v + 12582912.f) - 0x4b400000; }
+
+// Tile t of the trailing matrix of nt 64-row tiles: row block I (tiles 2 I, 2 I + 1), column tile J.
+__device__ __forceinline__ void tile_of(long long t, int* I, int* J) {
+    int i = static_cast<int>((sqrtf(4.f * static_cast<float>(t) + 1.f) - 1.f) * 0.5f);
+    while (static_cast<long long>(i) * (i + 1) > t) --i;
+    while (static_cast<long long>(i + 1) * (i + 2) <= t) ++i;
+    *I = i;
+    *J = static_cast<int>(t - static_cast<long long>(i) * (i + 1));
+}
+
+__global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict__ A, int j1, int nt, long long ntiles,
+                                                             int lda, const unsigned char* __restrict__ tiles,
+                                                             int* __restrict__ info) {
+    extern __shared__ unsigned char upd_raw[];
+    __shared__ __align__(8) unsigned long long bars[B_COUNT];
+    __shared__ uint32_t tmem_base;
+    __shared__ volatile int gave_up;
+    __shared__ int info_s;
+    const uint32_t base = (smem_u32(upd_raw) + 1023u) & ~1023u;
+    const uint32_t sA = base, sB = base + kABytes;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t bar0 = smem_u32(bars);
+    auto bar = [&](int i) { return bar0 + 8u * i; };
+    if (tid == 0) {
+        for (int i = 0; i < B_COUNT; ++i) mbar_init(bar(i), i == B_LOEMPTY || i == B_HIEMPTY ? kUpdWarps : 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        gave_up = 0;
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], 512;" ::"r"(smem_u32(&tmem_base))
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    pdl_wait();
+    pdl_trigger();
+    if (tid == 0) info_s = *info;  // one read per block
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = tmem_base;
+    const int failed = info_s;
+    const long long t0 = ntiles * blockIdx.x / gridDim.x, t1 = failed ? t0 : ntiles * (blockIdx.x + 1) / gridDim.x;
+    const int tile0 = j1 / NB;  // first tile of the trailing matrix
+
+    if (warp == 0 && lane == 0) {
+        int lastI = -1, na = 0;
+        for (long long t = t0; t < t1; ++t) {
+            int I, J;
+            tile_of(t, &I, &J);
+            if (I != lastI) {
+                if (na > 0 && !mbar_wait(bar(B_EMPTYA), (na - 1) & 1, &gave_up)) break;
+                const bool two = 2 * I + 1 < nt;
+                mbar_expect(bar(B_FULLA), two ? kABytes : kABytes / 2);
+                const unsigned char* src = tiles + static_cast<size_t>(tile0 + 2 * I) * kNS * kTileB;
+                for (int s = 0; s < kNS; ++s) {
+                    bulk_load(sA + s * 2 * kTileB, src + s * kTileB, kTileB, bar(B_FULLA));
+                    if (two)
+                        bulk_load(sA + s * 2 * kTileB + kTileB, src + (kNS + s) * kTileB, kTileB, bar(B_FULLA));
+                }
+                lastI = I;
+                ++na;
+            }
+            const int i = static_cast<int>(t - t0), st = i & 1;
+            if (i >= 2 && !mbar_wait(bar(B_EMPTYB + st), ((i >> 1) - 1) & 1, &gave_up)) break;
+            mbar_expect(bar(B_FULLB + st), kBBytes);
+            bulk_load(sB + st * kBBytes, tiles + static_cast<size_t>(tile0 + J) * kNS * kTileB, kBBytes,
+                      bar(B_FULLB + st));
+        }
+    } else if (warp == 1 && lane == 0) {
+        const uint32_t idesc = (1u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24);  // FP16 x FP16 -> FP32, M 128, N 64
+        int lastI = -1, na = 0;
+        for (long long t = t0; t < t1; ++t) {
+            int I, J;
+            tile_of(t, &I, &J);
+            const int i = static_cast<int>(t - t0), st = i & 1;
+            if (I != lastI) {
+                if (!mbar_wait(bar(B_FULLA), na & 1, &gave_up)) break;
+                lastI = I;
+                ++na;
+            }
+            if (!mbar_wait(bar(B_FULLB + st), (i >> 1) & 1, &gave_up)) break;
+            const uint32_t b = sB + st * kBBytes;
+            auto group = [&](int d) {
+                bool acc = false;
+                for (int s = 0; s <= d; ++s) {
+                    const uint64_t da = operand_desc(sA + s * 2 * kTileB), db = operand_desc(b + (d - s) * kTileB);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {  // K = 16: 32 bytes along the swizzled row
+                        mma_f16(tmem + 64 * d, da + 2 * k, db + 2 * k, idesc, acc);
+                        acc = true;
+                    }
+                }
+            };
+            if (i > 0 && !mbar_wait(bar(B_LOEMPTY), (i - 1) & 1, &gave_up)) break;
+            tc_fence_after();
+            for (int d = 4; d < kNS; ++d) group(d);
+            mma_commit(bar(B_LOFULL));
+            if (i > 0 && !mbar_wait(bar(B_HIEMPTY), (i - 1) & 1, &gave_up)) break;
+            tc_fence_after();
+            for (int d = 0; d < 4; ++d) group(d);
+            mma_commit(bar(B_HIFULL));
+            mma_commit(bar(B_EMPTYB + st));
+            int I2 = -1, J2;
+            if (t + 1 < t1) tile_of(t + 1, &I2, &J2);
+            if (I2 != I) mma_commit(bar(B_EMPTYA));
+        }
+    } else if (warp >= 2) {
+        const int quarter = warp & 3, part = (warp - 2) >> 2;  // TMEM lanes 32 quarter .., columns 16 part ..
+        const uint32_t tm = tmem + (static_cast<uint32_t>(32 * quarter) << 16) + 16 * part;
+        long long* F = reinterpret_cast<long long*>(A);
+        for (long long t = t0; t < t1; ++t) {
+            int I, J;
+            tile_of(t, &I, &J);
+            const int i = static_cast<int>(t - t0);
+            const int rloc = 128 * I + 32 * quarter + lane, cloc = 64 * J + 16 * part;  // within the trailing matrix
+            const bool in = rloc < 64 * nt;
+            long long* p = F + (j1 + rloc) + static_cast<long long>(j1 + cloc) * lda;
+            long long c[16];
+#pragma unroll
+            for (int k = 0; k < 16; ++k) c[k] = in && rloc >= cloc + k ? p[static_cast<long long>(k) * lda] : 0;
+            if (!mbar_wait(bar(B_LOFULL), i & 1, &gave_up)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int k0 = 0; k0 < 16; k0 += 8) {
+                float g4[8], g5[8], g6[8];
+                tmem_load8(tm + 4 * 64 + k0, g4);
+                tmem_load8(tm + 5 * 64 + k0, g5);
+                tmem_load8(tm + 6 * 64 + k0, g6);
+                tmem_wait_load();
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    c[k0 + k] -= static_cast<long long>(__float2int_rn(g4[k])) * 256 +
+                                 __float2int_rn(0.5f * fmaf(g6[k], 0x1p-9f, g5[k]));
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(B_LOEMPTY));
+            if (!mbar_wait(bar(B_HIFULL), i & 1, &gave_up)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int k0 = 0; k0 < 16; k0 += 8) {
+                float g0[8], g1[8], g2[8], g3[8];
+                tmem_load8(tm + k0, g0);
+                tmem_load8(tm + 64 + k0, g1);
+                tmem_load8(tm + 128 + k0, g2);
+                tmem_load8(tm + 192 + k0, g3);
+                tmem_wait_load();
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    const int top = small_int(g0[k]) * 512 + small_int(g1[k]);  // 2^35
+                    c[k0 + k] -= (static_cast<long long>(top) << 35) +
+                                 static_cast<long long>(__float2int_rn(g2[k])) * (1 << 26) +
+                                 static_cast<long long>(__float2int_rn(g3[k])) * (1 << 17);
+                }
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(B_HIEMPTY));
+            asm volatile("" : "+l"(p));  // the sixteen addresses are formed again, not held across the recombination
+#pragma unroll
+            for (int k = 0; k < 16; ++k)
+                if (in && rloc >= cloc + k) p[static_cast<long long>(k) * lda] = c[k];
+        }
+    }
+    __syncwarp();
+    if (gave_up)
+        for (int i = 0; i < 200; ++i) __nanosleep(1000);  // copies and MMAs in flight land before the block ends
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
+    if (tid == 0 && gave_up) *info = INT_MIN;
+}
+
+}  // namespace
+
+size_t dense_potrf_workspace(int n) {
+    return static_cast<size_t>(n / NB) * kNS * kTileB + 2 * sizeof(int) * static_cast<size_t>(n);
+}
+
+// bt: tiles below the diagonal tile that hold nonzeros (n / 64 - 1 for a
+// dense matrix; lda = ldb - 1 with ldb >= (bt + 2) 64 for a band).
+void dense_potrf(double* A, int n, int lda, int bt, int* info, void* workspace, cudaStream_t s) {
+    if (n % NB != 0 || bt < 0 || (bt < n / NB - 1 ? lda + 1 < (bt + 2) * NB : lda < n))
+        throw std::invalid_argument("dense_potrf: n must be a multiple of 64 and lda hold the band");
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(chol_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(PanelSmem)));
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(chol_update, cudaFuncAttributeMaxDynamicSharedMemorySize, kUpdSmem));
+    const Work w = carve(workspace, n);
+    const int nt = n / NB, sms = device_sm_count();
+    launch_pdl(chol_scale, ceil_div(n, 256), 256, 0, s, A, n, lda, w.e, w.bad, info);
+    launch_pdl(chol_convert, dim3(nt, std::min(bt, nt - 1) + 1), 256, 0, s, A, nt, lda, bt, w.e, w.bad);
+    for (int jb = 0; jb < nt; ++jb) {
+        const int j0 = jb * NB, below = std::min(nt - jb - 1, bt), rows = below * NB;
+        // rows per CTA: kExtra are solved along with the diagonal tile; more only
+        // where the panel has more than that for every SM
+        const int rpc = kExtra * std::max(1, ceil_div(rows, kExtra * sms));
+        launch_pdl(chol_panel, std::max(1, ceil_div(rows, rpc)), kPanelThreads, sizeof(PanelSmem), s, A, j0, lda, rows, rpc,
+               w.e, w.bad, w.tiles, info);
+        if (below == 0) continue;
+        const long long pairs = below / 2;
+        const long long tiles = pairs * (pairs + 1) + (below % 2 ? below : 0);
+        launch_pdl(chol_update, static_cast<unsigned>(std::min<long long>(tiles, sms)), kUpdThreads, kUpdSmem, s, A, j0 + NB,
+               below, tiles, lda, w.tiles, info);
+    }
+}
+
+}  // namespace gba

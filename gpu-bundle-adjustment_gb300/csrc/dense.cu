@@ -1,5 +1,6 @@
-// Plain form: on-device assembly of the dense reduced camera system and its
-// blocked FP64 Cholesky on the DMMA tensor cores.
+// Plain form: on-device assembly of the reduced camera system, the triangular
+// solves with its Cholesky factor (chol.cu) and the FP64 factorisation of
+// the explicitly dense layout.
 //
 // Reference: the host assembly src/lm.cu:488-594 (T_e = W_e V'^-1, privatised
 // S -= T_e W_f^T over edge pairs of each point, merge, rhs, damped U blocks) and
@@ -9,7 +10,7 @@
 //     with cam(e) >= cam(f) are sorted once by camera-pair block, and each
 //     9x9 block is written once as the ordered sum of its pairs (no atomics,
 //     deterministic), then the damped U blocks are added;
-//   * the factorisation is right-looking blocked Cholesky (panel width 64):
+//   * the FP64 factorisation is right-looking blocked Cholesky (panel width 64):
 //     diagonal-block potrf in shared memory, panel triangular solve, and the
 //     trailing update C -= A B^T with mma.sync.m8n8k4 FP64 (DMMA).
 // S is column-major, n_pad x n_pad (n_pad = 9C rounded up to 64, identity on
@@ -229,7 +230,11 @@ __global__ void rhs_finalize_kernel(const int* __restrict__ cam_chunk_off, const
     rhs[t] = bc[t] - v;
 }
 
-// ---------------------------------------------------------------- Cholesky
+// ---------------------------------------------------------------- FP64 Cholesky
+//
+// The explicitly dense layout keeps the reference's arithmetic: an FP64
+// factorisation (the trailing update by mma.sync m8n8k4, the FP64 pipe's rate), to
+// check the fixed-point one (chol.cu), which serves every other call, against.
 
 // Factor the NB x NB diagonal block at (j0, j0) in shared memory.
 // The pivot's square root and its reciprocal are taken once per column (by
@@ -384,8 +389,8 @@ __global__ void __launch_bounds__(256) syrk_update_kernel(double* __restrict__ A
 }
 
 // The trailing update by 32 x 32 quadrants (four CTAs per 64 x 64 tile, the
-// upper quadrant of a diagonal tile skipped): for steps with few tiles (a
-// band's bt(bt+1)/2), so that the update spreads over four times as many SMs.
+// upper quadrant of a diagonal tile skipped): for steps with few tiles, so
+// that the update spreads over four times as many SMs.
 // 8 warps per quadrant, each warp 8 x 16 = 1 x 2 DMMA tiles.
 constexpr int kSPq = 32 + 8;  // shared-memory stride (doubles) of the quadrant's K-major operands
 __global__ void __launch_bounds__(256) syrk_update_quad_kernel(double* __restrict__ A, int j0, int ntiles, int lda,
@@ -582,11 +587,7 @@ __global__ void __launch_bounds__(kSolT) backward_step(const double* __restrict_
 
 }  // namespace
 
-// bt: tiles below the diagonal tile that hold nonzeros (n / 64 - 1 for a
-// dense matrix; lda = ldb - 1 with ldb >= (bt + 2) 64 for a band).
-void dense_potrf(double* A, int n, int lda, int bt, int* info, cudaStream_t s) {
-    if (n % NB != 0 || bt < 0 || (bt < n / NB - 1 ? lda + 1 < (bt + 2) * NB : lda < n))
-        throw std::invalid_argument("dense_potrf: n must be a multiple of 64 and lda hold the band");
+static void dense_potrf_fp64(double* A, int n, int lda, int* info, cudaStream_t s) {
     GBA_CUDA_CHECK(cudaMemsetAsync(info, 0, sizeof(int), s));
     static bool attr = false;
     const int smem = 2 * NB * kSP * sizeof(double);
@@ -601,13 +602,9 @@ void dense_potrf(double* A, int n, int lda, int bt, int* info, cudaStream_t s) {
         const int j0 = jb * NB;
         potrf_diag_kernel<<<1, 256, 0, s>>>(A, j0, lda, info);
         GBA_LAUNCH_CHECK();
-        const int below = std::min(nt - jb - 1, bt);
-        if (below == 0) {
-            if (jb == nt - 1) break;
-            continue;
-        }
-        // few panel tiles (a band, or the last steps of a dense matrix): split
-        // them over more CTAs
+        const int below = nt - jb - 1;
+        if (below == 0) break;
+        // few panel tiles (the last steps): split them over more CTAs
         const int sms = device_sm_count();
         const int rows = below * 4 <= sms ? 16 : NB;
         trsm_panel_kernel<<<below * (NB / rows), 256, tsmem, s>>>(A, j0, lda, rows, info);
@@ -664,7 +661,7 @@ void Solver::ensure_schur_storage() {
     band_mode_ = band;
     S_.release();
     S_.alloc(static_cast<size_t>(n_pad_) * (band ? band_ldb_ : n_pad_));
-    if (!chol_ws_.get()) chol_ws_.alloc(dense_potrs_workspace(n_pad_));
+    if (!chol_ws_.get()) chol_ws_.alloc(std::max(dense_potrf_workspace(n_pad_), dense_potrs_workspace(n_pad_)));
     schur_layout_planned_ = want;
 }
 
@@ -717,10 +714,14 @@ int Solver::schur_dense(double lambda) {
         GBA_LAUNCH_CHECK();
     }
     cudaEvent_t ev = prof_start();
-    dense_potrf(S_.get(), n_pad_, lda, bt, info_.get(), stream_);
+    if (schur_layout_ == 1)
+        dense_potrf_fp64(S_.get(), n_pad_, lda, info_.get(), stream_);
+    else
+        dense_potrf(S_.get(), n_pad_, lda, bt, info_.get(), chol_ws_.get(), stream_);
     prof_stop("dense_potrf", ev);
     int info = 0;
     read_back({{&info, info_.get(), sizeof info}});
+    if (info < 0) throw std::runtime_error("dense_potrf: a wait of the trailing update ran out");
     if (info != 0) return info;
     // solve in a copy so rhs stays the assembled right-hand side (in the band
     // layout the copy is in the renumbered camera order; the padding stays 0)

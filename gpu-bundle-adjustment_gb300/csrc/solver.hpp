@@ -278,7 +278,7 @@ public:
     DevBuf<double> long_part_;
     DevBuf<double> T_, S_, rhs_, dc_, dp_, red_part_;
     DevBuf<int> info_;
-    DevBuf<unsigned char> chol_ws_;  // workspace of dense_potrs, allocated with S_
+    DevBuf<unsigned char> chol_ws_;  // workspace of dense_potrf and dense_potrs, allocated with S_
     // mixed Schur
     DevBuf<double> Sdiag_, Pfac_;  // S diagonal blocks (81C), preconditioner factors (packed, 45 per camera)
     DevBuf<float> Pinv_;           // explicit preconditioner blocks M_c = (L L^T)^-1 (81C, FP32)
@@ -374,8 +374,11 @@ void launch_batch_inverse3_spd(const double* A, double* Ainv, int* ok, int n, cu
 // must be a multiple of 64. Dense: bt = n / 64 - 1, lda >= n. Band of bt
 // 64-row tiles below the diagonal tile: lda = ldb - 1, ldb >= (bt + 2) 64 rows
 // kept per column from the diagonal down. info (device int) = 0 on success,
-// else the 1-based failed column.
-void dense_potrf(double* A, int n, int lda, int bt, int* info, cudaStream_t s);
+// else the 1-based failed column (negative: a bounded wait in a kernel ran
+// out). workspace: dense_potrf_workspace(n) bytes of device memory, 16-byte
+// aligned, the call's own until the stream has passed it (chol.cu).
+size_t dense_potrf_workspace(int n);
+void dense_potrf(double* A, int n, int lda, int bt, int* info, void* workspace, cudaStream_t s);
 
 // Solves L L^T x = b in place (b on the device, length n), L from dense_potrf
 // (nothing is done where *info != 0). workspace: dense_potrs_workspace(n) bytes of

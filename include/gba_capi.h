@@ -65,7 +65,10 @@ typedef struct gba_lm_options {
  * of the cameras reordered by reverse Cuthill-McKee on the camera graph (block
  * rows of S within the band, the factor keeps the band). AUTO takes the band
  * when it holds at most a third of the dense matrix (sparse covisibility, e.g.
- * sequential captures); random covisibility stays dense. */
+ * sequential captures); random covisibility stays dense. AUTO and BAND factor S
+ * in scaled 64-bit fixed point (chol.cu: exact products, rounding 2^-60 of the
+ * diagonal); DENSE, asked for explicitly, in FP64 as the reference does, to
+ * check the others against (many times slower on large problems). */
 enum { GBA_SCHUR_AUTO = 0, GBA_SCHUR_DENSE = 1, GBA_SCHUR_BAND = 2 };
 
 enum { GBA_LOSS_NONE = 0, GBA_LOSS_HUBER = 1 };
@@ -332,9 +335,12 @@ int gba_batch_chol9_factor_solve(const double* A, const double* b, double* x, in
  * include/gba/schur.cuh:112-116). [device] A (n x 9 row-major, lower read), Ainv (n x 9). */
 int gba_batch_inverse3_spd(const double* A, double* Ainv, int* ok, int n, void* stream);
 
-/* Blocked FP64 Cholesky (lower, column-major, DMMA trailing update), in place.
- * Replaces Eigen::LLT<MatrixXd, Lower> (reference src/lm.cu:598-603).
- * n multiple of 64, lda >= n. [device] A, info (int: 0 or failed column). */
+/* Blocked Cholesky (lower, column-major), in place: FP64 in and out, scaled 64-bit
+ * fixed point inside (products exact, entries rounded at 2^-60 of
+ * sqrt(A_ii A_jj); closer to the exact factor than FP64 arithmetic). Replaces Eigen::LLT<MatrixXd, Lower> (reference src/lm.cu:598-603).
+ * n multiple of 64, lda >= n. [device] A, info (int: 0, the failed column, or
+ * negative when a bounded wait inside a kernel ran out). Workspace (0.9 n KB)
+ * is taken from and returned to the device's memory pool on the stream. */
 int gba_dense_potrf(double* A, int n, int lda, int* info, void* stream);
 /* Solves L L^T x = b in place after gba_dense_potrf (reference src/lm.cu:604). [device] */
 int gba_dense_potrs(const double* L, int n, int lda, double* b, const int* info, void* stream);
