@@ -1,10 +1,12 @@
 // Learned coarse-space correction: MLP training and inference kernels.
 //
-//   GEMMs      mma.sync.m16n8k16 BF16 x BF16 -> FP32 (BF16 weights and
-//              activations in shared memory, FP32 accumulation and storage);
-//              one kernel with strided operand loads serves the forward
-//              (X W^T), input-gradient (dY W) and weight-gradient (dY^T X) shapes.
-//   backward   from the loss gradient w.r.t. the outputs (the loss, the
+//   forward    one kernel: 32 rows of the batch per CTA through all three layers
+//              (mma.sync.m16n8k16 BF16 x BF16 -> FP32, weights and activations in
+//              shared memory). A batch is a few thousand rows of 37,000 products each:
+//              the launch and the weights' trip from L2 bound it, not the tensor cores.
+//   backward   one kernel for both input gradients and each CTA's share of the
+//              parameter gradients (its rows), one that adds the shares in order;
+//              from the loss gradient w.r.t. the outputs (the loss, the
 //              eigenvector share outside the coarse space, is a global function
 //              of all cameras' outputs; the training script forms its gradient).
 //   Adam       FP32 masters, BF16 copies refreshed after each step.
@@ -13,6 +15,7 @@
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -29,13 +32,11 @@
 namespace gba {
 namespace {
 
-constexpr int kGT = 128;  // GEMM threads (4 warps, 2 x 2 warp grid of 32 x 32)
 constexpr long long kW1 = 0, kB1 = kW1 + 1ll * kMlpH * kMlpIn, kW2 = kB1 + kMlpH, kB2 = kW2 + 1ll * kMlpH * kMlpH,
                     kW3 = kB2 + kMlpH, kB3 = kW3 + 1ll * kMlpOut * kMlpH;
 constexpr long long kBf16Count = 1ll * kMlpH * kMlpIn + 1ll * kMlpH * kMlpH + 1ll * kMlpOut * kMlpH;
 
 __device__ __forceinline__ __nv_bfloat16 to_bf16(float v) { return __float2bfloat16_rn(v); }
-__device__ __forceinline__ __nv_bfloat16 to_bf16(__nv_bfloat16 v) { return v; }
 
 __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
     asm volatile(
@@ -45,90 +46,259 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], 
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
 }
 
-// C(m, n) = epilogue( sum_k A(m, k) B(k, n) ), A(m,k) = A[m*sam + k*sak],
-// B(k,n) = B[k*sbk + n*sbn]; epilogue: + bias[n], ReLU, * (mask(m,n) > 0).
-template <typename TA, typename TB>
-__global__ void __launch_bounds__(kGT) gemm_bf16_kernel(int M, int N, int K, const TA* __restrict__ A, long long sam,
-                                                       long long sak, const TB* __restrict__ B, long long sbk,
-                                                       long long sbn, float* __restrict__ Cm, int ldc,
-                                                       const float* __restrict__ bias, int relu,
-                                                       const float* __restrict__ mask, int ldm) {
-    __shared__ __align__(16) __nv_bfloat16 As[64][24];
-    __shared__ __align__(16) __nv_bfloat16 Bs[64][24];
-    const int m0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int wm = (warp & 1) * 32, wn = (warp >> 1) * 32;
-    const int g = lane >> 2, t = lane & 3;
-    float acc[2][4][4];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int q = 0; q < 4; ++q) acc[i][j][q] = 0.f;
-    for (int k0 = 0; k0 < K; k0 += 16) {
-        for (int idx = tid; idx < 64 * 16; idx += kGT) {
-            const int r = idx >> 4, kk = idx & 15;
-            const int k = k0 + kk;
-            const int m = m0 + r, n = n0 + r;
-            As[r][kk] = (m < M && k < K) ? to_bf16(A[m * sam + k * sak]) : __float2bfloat16_rn(0.f);
-            Bs[r][kk] = (n < N && k < K) ? to_bf16(B[k * sbk + n * sbn]) : __float2bfloat16_rn(0.f);
-        }
-        __syncthreads();
-        uint32_t af[2][4], bfr[4][2];
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt) {
-            const int r = wm + 16 * mt + g;
-            af[mt][0] = *reinterpret_cast<const uint32_t*>(&As[r][2 * t]);
-            af[mt][1] = *reinterpret_cast<const uint32_t*>(&As[r + 8][2 * t]);
-            af[mt][2] = *reinterpret_cast<const uint32_t*>(&As[r][2 * t + 8]);
-            af[mt][3] = *reinterpret_cast<const uint32_t*>(&As[r + 8][2 * t + 8]);
-        }
-#pragma unroll
-        for (int nt = 0; nt < 4; ++nt) {
-            const int r = wn + 8 * nt + g;
-            bfr[nt][0] = *reinterpret_cast<const uint32_t*>(&Bs[r][2 * t]);
-            bfr[nt][1] = *reinterpret_cast<const uint32_t*>(&Bs[r][2 * t + 8]);
-        }
-#pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-            for (int nt = 0; nt < 4; ++nt) mma_bf16(acc[mt][nt], af[mt], bfr[nt]);
-        __syncthreads();
+constexpr int kRowsT = 32;    // rows of the batch per CTA
+constexpr int kMT = 256;      // threads (8 warps)
+constexpr int kLdIn = kMlpIn + 8, kLdH = kMlpH + 8, kLdOut = kMlpOut + 8;  // shared-memory strides (BF16 values)
+
+__device__ __forceinline__ uint32_t pair_at(const __nv_bfloat16* p) { return *reinterpret_cast<const uint32_t*>(p); }
+__device__ __forceinline__ uint32_t pair_of(__nv_bfloat16 a, __nv_bfloat16 b) {
+    return static_cast<uint32_t>(__bfloat16_as_ushort(a)) | (static_cast<uint32_t>(__bfloat16_as_ushort(b)) << 16);
+}
+
+// Rows x cols BF16 matrix (row-major, cols a multiple of 8) into shared memory of stride ld.
+__device__ __forceinline__ void load_weights(const __nv_bfloat16* __restrict__ w, int rows, int cols,
+                                             __nv_bfloat16* dst, int ld) {
+    const int per = cols / 8;
+    for (int i = threadIdx.x; i < rows * per; i += kMT)
+        *reinterpret_cast<uint4*>(dst + (i / per) * ld + 8 * (i % per)) = reinterpret_cast<const uint4*>(w)[i];
+}
+// kRowsT rows of an FP32 matrix from row r0 (zeros from row B on) as BF16. The
+// callers' matrices may start at any float: 16-byte loads where they start at 16 bytes.
+__device__ __forceinline__ void load_rows(const float* __restrict__ x, int r0, int B, int cols, __nv_bfloat16* dst,
+                                          int ld) {
+    const int per = cols / 4;
+    const bool wide = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+    for (int i = threadIdx.x; i < kRowsT * per; i += kMT) {
+        const int r = i / per, c = 4 * (i % per);
+        const float* src = x + static_cast<long long>(r0 + r) * cols + c;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r0 + r < B) v = wide ? *reinterpret_cast<const float4*>(src) : make_float4(src[0], src[1], src[2], src[3]);
+        __nv_bfloat16* d = dst + r * ld + c;
+        d[0] = to_bf16(v.x);
+        d[1] = to_bf16(v.y);
+        d[2] = to_bf16(v.z);
+        d[3] = to_bf16(v.w);
     }
+}
+
+// acc[mt] = A (kRowsT x K, row-major) times the n8 tile nt of B, K ascending. kTrans:
+// B(k, n) = Bs[k][n], else Bs[n][k].
+template <int K, bool kTrans>
+__device__ __forceinline__ void rows_times(const __nv_bfloat16* As, int lda, const __nv_bfloat16* Bs, int ldb, int nt,
+                                           float (&acc)[2][4]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
 #pragma unroll
     for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int q = 0; q < 4; ++q) acc[mt][q] = 0.f;
+#pragma unroll
+    for (int k0 = 0; k0 < K; k0 += 16) {
+        uint32_t b[2];
+        const int n = 8 * nt + g, k = k0 + 2 * t;
+        if (kTrans) {
+            b[0] = pair_of(Bs[k * ldb + n], Bs[(k + 1) * ldb + n]);
+            b[1] = pair_of(Bs[(k + 8) * ldb + n], Bs[(k + 9) * ldb + n]);
+        } else {
+            b[0] = pair_at(Bs + n * ldb + k);
+            b[1] = pair_at(Bs + n * ldb + k + 8);
+        }
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt) {
+            const __nv_bfloat16* a0 = As + (16 * mt + g) * lda + k;
+            const uint32_t a[4] = {pair_at(a0), pair_at(a0 + 8 * lda), pair_at(a0 + 8), pair_at(a0 + 8 * lda + 8)};
+            mma_bf16(acc[mt], a, b);
+        }
+    }
+}
+
+struct ForwardSmem {
+    __nv_bfloat16 w1[kMlpH * kLdIn], w2[kMlpH * kLdH], w3[kMlpOut * kLdH];
+    __nv_bfloat16 x[kRowsT * kLdIn], h1[kRowsT * kLdH], h2[kRowsT * kLdH];
+};
+
+// The whole network for 32 rows per CTA. Bound by latency: 32 CTAs of 1000 rows
+// each bring the 77 KB of weights from L2 and go through 16 K-steps. 1000 rows:
+// 15 us, against 3 x 29 us for a GEMM per layer with the activations through
+// memory. h1, h2 (FP32, for backward) may be null.
+__global__ void __launch_bounds__(kMT) mlp_forward_kernel(const float* __restrict__ feat, int B,
+                                                         const __nv_bfloat16* __restrict__ wb,
+                                                         const float* __restrict__ params, float* __restrict__ h1,
+                                                         float* __restrict__ h2, float* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char mlp_smem[];
+    ForwardSmem& sm = *reinterpret_cast<ForwardSmem*>(mlp_smem);
+    const int r0 = blockIdx.x * kRowsT, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    load_rows(feat, r0, B, kMlpIn, sm.x, kLdIn);
+    load_weights(wb, kMlpH, kMlpIn, sm.w1, kLdIn);
+    load_weights(wb + 1ll * kMlpH * kMlpIn, kMlpH, kMlpH, sm.w2, kLdH);
+    load_weights(wb + 1ll * kMlpH * kMlpIn + 1ll * kMlpH * kMlpH, kMlpOut, kMlpH, sm.w3, kLdH);
+    __syncthreads();
+    // a layer's output tile: + bias, ReLU, FP32 to global and BF16 for the next layer
+    auto store = [&](float (&acc)[2][4], int nt, const float* bias, bool relu, float* dst, int ld, __nv_bfloat16* next) {
+#pragma unroll
+        for (int mt = 0; mt < 2; ++mt)
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int m = m0 + wm + 16 * mt + g + ((q >= 2) ? 8 : 0);
-                const int n = n0 + wn + 8 * nt + 2 * t + (q & 1);
-                if (m >= M || n >= N) continue;
-                float v = acc[mt][nt][q];
-                if (bias) v += bias[n];
+                const int r = 16 * mt + g + (q >= 2 ? 8 : 0), n = 8 * nt + 2 * t + (q & 1);
+                float v = acc[mt][q] + bias[n];
                 if (relu) v = fmaxf(v, 0.f);
-                if (mask && !(mask[(long long)m * ldm + n] > 0.f)) v = 0.f;
-                Cm[(long long)m * ldc + n] = v;
+                if (dst && r0 + r < B) dst[static_cast<long long>(r0 + r) * ld + n] = v;
+                if (next) next[r * kLdH + n] = to_bf16(v);
             }
+    };
+    float acc[2][4];
+    for (int nt = warp; nt < kMlpH / 8; nt += kMT / 32) {
+        rows_times<kMlpIn, false>(sm.x, kLdIn, sm.w1, kLdIn, nt, acc);
+        store(acc, nt, params + kB1, true, h1, kMlpH, sm.h1);
+    }
+    __syncthreads();
+    for (int nt = warp; nt < kMlpH / 8; nt += kMT / 32) {
+        rows_times<kMlpH, false>(sm.h1, kLdH, sm.w2, kLdH, nt, acc);
+        store(acc, nt, params + kB2, true, h2, kMlpH, sm.h2);
+    }
+    __syncthreads();
+    for (int nt = warp; nt < kMlpOut / 8; nt += kMT / 32) {
+        rows_times<kMlpH, false>(sm.h2, kLdH, sm.w3, kLdH, nt, acc);
+        store(acc, nt, params + kB3, false, out, kMlpOut, nullptr);
+    }
 }
 
-template <typename TA, typename TB>
-void gemm(int M, int N, int K, const TA* A, long long sam, long long sak, const TB* B, long long sbk, long long sbn,
-          float* Cm, int ldc, const float* bias, bool relu, const float* mask, int ldm, cudaStream_t s) {
-    dim3 grid(ceil_div(N, 64), ceil_div(M, 64));
-    gemm_bf16_kernel<TA, TB><<<grid, kGT, 0, s>>>(M, N, K, A, sam, sak, B, sbk, sbn, Cm, ldc, bias, relu ? 1 : 0,
-                                                  mask, ldm);
-    GBA_LAUNCH_CHECK();
+struct BackwardSmem {
+    __nv_bfloat16 w3[kMlpOut * kLdH], w2[kMlpH * kLdH];
+    __nv_bfloat16 x[kRowsT * kLdIn], h1[kRowsT * kLdH], h2[kRowsT * kLdH];
+    __nv_bfloat16 d3[kRowsT * kLdOut], d2[kRowsT * kLdH], d1[kRowsT * kLdH];
+    float f[kRowsT][kMlpH + 1];  // a layer's gradient in FP32, for its bias sums
+};
+
+// The rows' share of dW (n x k) = dY^T X: warp mt owns rows 16 mt .. of dW; added
+// to what the CTA's earlier rows left when !first.
+template <int NT>
+__device__ __forceinline__ void weight_share(const __nv_bfloat16* dY, int ldy, const __nv_bfloat16* X, int ldx, int mt,
+                                             float* __restrict__ dst, bool first) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    uint32_t a[2][4];
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+        const __nv_bfloat16* y = dY + (16 * ks + 2 * t) * ldy + 16 * mt + g;
+        a[ks][0] = pair_of(y[0], y[ldy]);
+        a[ks][1] = pair_of(y[8], y[ldy + 8]);
+        a[ks][2] = pair_of(y[8 * ldy], y[9 * ldy]);
+        a[ks][3] = pair_of(y[8 * ldy + 8], y[9 * ldy + 8]);
+    }
+#pragma unroll 4
+    for (int nt = 0; nt < NT; ++nt) {
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {
+            const __nv_bfloat16* x = X + (16 * ks + 2 * t) * ldx + 8 * nt + g;
+            const uint32_t b[2] = {pair_of(x[0], x[ldx]), pair_of(x[8 * ldx], x[9 * ldx])};
+            mma_bf16(acc, a[ks], b);
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            float2* d = reinterpret_cast<float2*>(dst + (16 * mt + g + 8 * q) * (8 * NT) + 8 * nt + 2 * t);
+            float2 v = make_float2(acc[2 * q], acc[2 * q + 1]);
+            if (!first) {
+                const float2 o = *d;
+                v.x += o.x;
+                v.y += o.y;
+            }
+            *d = v;
+        }
+    }
 }
 
-// db[n] = sum_m dY[m][n] (ordered, deterministic); one CTA per column.
-__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ dY, int M, int ld, float* __restrict__ db) {
-    __shared__ double sh[8];
-    double s = 0.0;
-    for (int m = threadIdx.x; m < M; m += 256) s += dY[(long long)m * ld + blockIdx.x];
-    const double v = block_sum<256>(s, sh);
-    if (threadIdx.x == 0) db[blockIdx.x] = static_cast<float>(v);
+// Each CTA takes the 32-row groups blockIdx.x, + gridDim.x, ...; its shares of
+// the parameter gradients go to part (flat layout, kMlpParams per CTA) and, for
+// the biases in FP64, to bpart (kH of b1, kH of b2, kOut of b3 per CTA).
+// Bound by latency as the forward pass; the batch is the reduction axis of the
+// weight gradients, so one GEMM per layer had 8 CTAs walk all rows in turn (290 us
+// each at 1000 rows, 1.0 ms in all); split by rows and fused: 29 us + 5.5 us for
+// the ordered sum of the shares. One CTA per SM at most keeps the shares at
+// 150 KB x SMs; a CTA adds its later groups onto its own share.
+constexpr int kBias = 2 * kMlpH + kMlpOut;
+__global__ void __launch_bounds__(kMT) mlp_backward_kernel(const float* __restrict__ feat,
+                                                          const float* __restrict__ dO, int B,
+                                                          const __nv_bfloat16* __restrict__ wb,
+                                                          const float* __restrict__ h1, const float* __restrict__ h2,
+                                                          float* __restrict__ part, double* __restrict__ bpart) {
+    extern __shared__ __align__(16) unsigned char mlp_smem[];
+    BackwardSmem& sm = *reinterpret_cast<BackwardSmem*>(mlp_smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    float* p = part + static_cast<long long>(blockIdx.x) * kMlpParams;
+    double* bp = bpart + static_cast<long long>(blockIdx.x) * kBias;
+    load_weights(wb + 1ll * kMlpH * kMlpIn, kMlpH, kMlpH, sm.w2, kLdH);
+    load_weights(wb + 1ll * kMlpH * kMlpIn + 1ll * kMlpH * kMlpH, kMlpOut, kMlpH, sm.w3, kLdH);
+    double b1 = 0.0, b2 = 0.0, b3 = 0.0;  // this thread's columns' bias sums
+    for (int r0 = blockIdx.x * kRowsT; r0 < B; r0 += gridDim.x * kRowsT) {
+        const bool first = r0 == static_cast<int>(blockIdx.x) * kRowsT;
+        load_rows(feat, r0, B, kMlpIn, sm.x, kLdIn);
+        load_rows(h1, r0, B, kMlpH, sm.h1, kLdH);
+        load_rows(h2, r0, B, kMlpH, sm.h2, kLdH);
+        load_rows(dO, r0, B, kMlpOut, sm.d3, kLdOut);
+        const int rows = min(kRowsT, B - r0);
+        if (threadIdx.x < kMlpOut)
+#pragma unroll 8
+            for (int r = 0; r < rows; ++r) b3 += dO[static_cast<long long>(r0 + r) * kMlpOut + threadIdx.x];
+        __syncthreads();
+        // dH = (dY W) where the layer's activation is positive
+        auto masked = [&](float (&acc)[2][4], int nt, const float* h, __nv_bfloat16* d) {
+#pragma unroll
+            for (int mt = 0; mt < 2; ++mt)
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    const int r = 16 * mt + g + (q >= 2 ? 8 : 0), n = 8 * nt + 2 * t + (q & 1);
+                    float v = 0.f;
+                    if (r < rows && h[static_cast<long long>(r0 + r) * kMlpH + n] > 0.f) v = acc[mt][q];
+                    d[r * kLdH + n] = to_bf16(v);
+                    sm.f[r][n] = v;
+                }
+        };
+        float acc[2][4];
+        for (int nt = warp; nt < kMlpH / 8; nt += kMT / 32) {
+            rows_times<kMlpOut, true>(sm.d3, kLdOut, sm.w3, kLdH, nt, acc);
+            masked(acc, nt, h2, sm.d2);
+        }
+        __syncthreads();
+        if (threadIdx.x < kMlpH)
+            for (int r = 0; r < rows; ++r) b2 += sm.f[r][threadIdx.x];
+        if (warp < kMlpOut / 16) weight_share<kMlpH / 8>(sm.d3, kLdOut, sm.h2, kLdH, warp, p + kW3, first);
+        weight_share<kMlpH / 8>(sm.d2, kLdH, sm.h1, kLdH, warp, p + kW2, first);
+        __syncthreads();
+        for (int nt = warp; nt < kMlpH / 8; nt += kMT / 32) {
+            rows_times<kMlpH, true>(sm.d2, kLdH, sm.w2, kLdH, nt, acc);
+            masked(acc, nt, h1, sm.d1);
+        }
+        __syncthreads();
+        if (threadIdx.x < kMlpH)
+            for (int r = 0; r < rows; ++r) b1 += sm.f[r][threadIdx.x];
+        weight_share<kMlpIn / 8>(sm.d1, kLdH, sm.x, kLdIn, warp, p + kW1, first);
+        __syncthreads();
+    }
+    if (threadIdx.x < kMlpH) {
+        bp[threadIdx.x] = b1;
+        bp[kMlpH + threadIdx.x] = b2;
+    }
+    if (threadIdx.x < kMlpOut) bp[2 * kMlpH + threadIdx.x] = b3;
+}
+
+// The CTAs' shares added in order.
+__global__ void __launch_bounds__(256) mlp_grad_sum_kernel(const float* __restrict__ part,
+                                                          const double* __restrict__ bpart, int n,
+                                                          float* __restrict__ grad) {
+    const long long i = blockIdx.x * 256ll + threadIdx.x;
+    if (i >= kMlpParams) return;
+    const long long at = i >= kB3 ? i - kB3 + 2 * kMlpH : i >= kB2 && i < kW3 ? i - kB2 + kMlpH
+                         : i >= kB1 && i < kW2 ? i - kB1 : -1;  // among the biases
+    if (at >= 0) {
+        double s = 0.0;
+        for (int c = 0; c < n; ++c) s += bpart[static_cast<long long>(c) * kBias + at];
+        grad[i] = static_cast<float>(s);
+    } else {
+        float s = 0.f;
+#pragma unroll 8
+        for (int c = 0; c < n; ++c) s += part[c * kMlpParams + i];
+        grad[i] = s;
+    }
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __restrict__ dst, long long n) {
@@ -136,16 +306,20 @@ __global__ void to_bf16_kernel(const float* __restrict__ src, __nv_bfloat16* __r
         dst[i] = __float2bfloat16_rn(src[i]);
 }
 
+// Adam on the FP32 masters, and the weights' BF16 copies.
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
                             float* __restrict__ v, long long n, float lr, float b1, float b2, float eps, float c1,
-                            float c2) {
+                            float c2, __nv_bfloat16* __restrict__ wb) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
         const float gi = g[i];
         const float mi = b1 * m[i] + (1.f - b1) * gi;
         const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
         m[i] = mi;
         v[i] = vi;
-        p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+        p[i] = pi;
+        const long long w = i < kB1 ? i : i >= kW2 && i < kB2 ? i - kMlpH : i >= kW3 && i < kB3 ? i - 2 * kMlpH : -1;
+        if (w >= 0) wb[w] = to_bf16(pi);
     }
 }
 
@@ -261,6 +435,9 @@ std::vector<float> read_model(const std::string& path) {
 
 // ------------------------------------------------------------------ Mlp
 
+// CTAs of the backward kernel: one per 32 rows, at most one per SM (more rows: several groups each).
+static int backward_ctas(int B) { return std::min(ceil_div(B, kRowsT), device_sm_count()); }
+
 void Mlp::alloc() {
     p_ = dalloc<float>(kMlpParams);
     g_ = dalloc<float>(kMlpParams);
@@ -274,22 +451,17 @@ void Mlp::alloc() {
 }
 
 void Mlp::ensure_capacity(int B) {
-    if (B <= cap_ && h1_) return;
+    if (B <= cap_ && (h1_ || inference_)) return;
     cap_ = std::max(B, std::max(cap_, 1));
-    if (inference_) {  // forward activations only
-        for (float* q : {h1_, h2_})
-            if (q) GBA_CUDA_CHECK(cudaFreeAsync(q, pool_stream_));
-        h1_ = palloc<float>(1ll * cap_ * kMlpH, pool_stream_);
-        h2_ = palloc<float>(1ll * cap_ * kMlpH, pool_stream_);
-        return;
-    }
-    for (void* q : {static_cast<void*>(h1_), static_cast<void*>(h2_), static_cast<void*>(dh2_),
-                    static_cast<void*>(dh1_)})
+    if (inference_) return;  // the activations stay in shared memory
+    for (void* q : {static_cast<void*>(h1_), static_cast<void*>(h2_), static_cast<void*>(part_),
+                    static_cast<void*>(bpart_)})
         if (q) cudaFree(q);
     h1_ = dalloc<float>(1ll * cap_ * kMlpH);
     h2_ = dalloc<float>(1ll * cap_ * kMlpH);
-    dh2_ = dalloc<float>(1ll * cap_ * kMlpH);
-    dh1_ = dalloc<float>(1ll * cap_ * kMlpH);
+    const int ctas = backward_ctas(cap_);
+    part_ = dalloc<float>(ctas * kMlpParams);
+    bpart_ = dalloc<double>(1ll * ctas * kBias);
 }
 
 Mlp::Mlp(int capacity, uint64_t seed) : cap_(capacity) {
@@ -328,13 +500,13 @@ void Mlp::require_training() const {
 
 Mlp::~Mlp() {
     if (inference_) {
-        for (void* q : {static_cast<void*>(p_), wb_, static_cast<void*>(h1_), static_cast<void*>(h2_)})
+        for (void* q : {static_cast<void*>(p_), wb_})
             if (q) cudaFreeAsync(q, pool_stream_);
         return;
     }
     for (void* q : {static_cast<void*>(p_), static_cast<void*>(g_), static_cast<void*>(m_), static_cast<void*>(v_), wb_,
-                    static_cast<void*>(h1_), static_cast<void*>(h2_), static_cast<void*>(dh2_),
-                    static_cast<void*>(dh1_)})
+                    static_cast<void*>(h1_), static_cast<void*>(h2_), static_cast<void*>(part_),
+                    static_cast<void*>(bpart_)})
         if (q) cudaFree(q);
 }
 
@@ -378,35 +550,23 @@ void Mlp::refresh_bf16(cudaStream_t s) {
 
 void Mlp::forward(const float* feat, int B, float* out, cudaStream_t s) {
     ensure_capacity(B);
-    const __nv_bfloat16* wb = static_cast<const __nv_bfloat16*>(wb_);
-    const __nv_bfloat16* w1 = wb;
-    const __nv_bfloat16* w2 = wb + 1ll * kMlpH * kMlpIn;
-    const __nv_bfloat16* w3 = w2 + 1ll * kMlpH * kMlpH;
-    // H1 = relu(X W1^T + b1): A = X [B x 64], B(k, n) = W1[n][k]
-    gemm(B, kMlpH, kMlpIn, feat, kMlpIn, 1, w1, 1, kMlpIn, h1_, kMlpH, p_ + kB1, true, nullptr, 0, s);
-    gemm(B, kMlpH, kMlpH, h1_, kMlpH, 1, w2, 1, kMlpH, h2_, kMlpH, p_ + kB2, true, nullptr, 0, s);
-    gemm(B, kMlpOut, kMlpH, h2_, kMlpH, 1, w3, 1, kMlpH, out, kMlpOut, p_ + kB3, false, nullptr, 0, s);
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        sizeof(ForwardSmem)));
+    mlp_forward_kernel<<<ceil_div(B, kRowsT), kMT, sizeof(ForwardSmem), s>>>(
+        feat, B, static_cast<const __nv_bfloat16*>(wb_), p_, h1_, h2_, out);
+    GBA_LAUNCH_CHECK();
 }
 
 void Mlp::backward(const float* feat, const float* dO, int B, cudaStream_t s) {
     require_training();
     if (B <= 0 || B > cap_) throw std::invalid_argument("backward: batch must be the last forward's (<= capacity)");
-    const __nv_bfloat16* wb = static_cast<const __nv_bfloat16*>(wb_);
-    const __nv_bfloat16* w2 = wb + 1ll * kMlpH * kMlpIn;
-    const __nv_bfloat16* w3 = w2 + 1ll * kMlpH * kMlpH;
-    // layer 3: dW3[n][k] = sum_m dO[m][n] H2[m][k]; db3; dH2 = (dO W3) * (H2 > 0)
-    gemm(kMlpOut, kMlpH, B, dO, 1, kMlpOut, h2_, kMlpH, 1, g_ + kW3, kMlpH, nullptr, false, nullptr, 0, s);
-    colsum_kernel<<<kMlpOut, 256, 0, s>>>(dO, B, kMlpOut, g_ + kB3);
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(mlp_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        sizeof(BackwardSmem)));
+    const int ctas = backward_ctas(B);
+    mlp_backward_kernel<<<ctas, kMT, sizeof(BackwardSmem), s>>>(
+        feat, dO, B, static_cast<const __nv_bfloat16*>(wb_), h1_, h2_, part_, bpart_);
     GBA_LAUNCH_CHECK();
-    gemm(B, kMlpH, kMlpOut, dO, kMlpOut, 1, w3, kMlpH, 1, dh2_, kMlpH, nullptr, false, h2_, kMlpH, s);
-    // layer 2
-    gemm(kMlpH, kMlpH, B, dh2_, 1, kMlpH, h1_, kMlpH, 1, g_ + kW2, kMlpH, nullptr, false, nullptr, 0, s);
-    colsum_kernel<<<kMlpH, 256, 0, s>>>(dh2_, B, kMlpH, g_ + kB2);
-    GBA_LAUNCH_CHECK();
-    gemm(B, kMlpH, kMlpH, dh2_, kMlpH, 1, w2, kMlpH, 1, dh1_, kMlpH, nullptr, false, h1_, kMlpH, s);
-    // layer 1 (input features need no gradient)
-    gemm(kMlpH, kMlpIn, B, dh1_, 1, kMlpH, feat, kMlpIn, 1, g_ + kW1, kMlpIn, nullptr, false, nullptr, 0, s);
-    colsum_kernel<<<kMlpH, 256, 0, s>>>(dh1_, B, kMlpH, g_ + kB1);
+    mlp_grad_sum_kernel<<<ceil_div(kMlpParams, 256), 256, 0, s>>>(part_, bpart_, ctas, g_);
     GBA_LAUNCH_CHECK();
 }
 
@@ -415,9 +575,9 @@ void Mlp::adam_step(float lr, float beta1, float beta2, float eps, cudaStream_t 
     ++step_;
     const float c1 = 1.f - std::pow(beta1, static_cast<float>(step_));
     const float c2 = 1.f - std::pow(beta2, static_cast<float>(step_));
-    adam_kernel<<<120, 256, 0, s>>>(p_, g_, m_, v_, kMlpParams, lr, beta1, beta2, eps, c1, c2);
+    adam_kernel<<<120, 256, 0, s>>>(p_, g_, m_, v_, kMlpParams, lr, beta1, beta2, eps, c1, c2,
+                                    static_cast<__nv_bfloat16*>(wb_));
     GBA_LAUNCH_CHECK();
-    refresh_bf16(s);
 }
 
 // ------------------------------------------------------------------ solver side

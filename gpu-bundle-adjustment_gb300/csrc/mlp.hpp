@@ -51,8 +51,8 @@ class Mlp {
 public:
     Mlp(int capacity, uint64_t seed);               // random init (He; small last layer), zero biases
     Mlp(const std::string& path, int capacity);     // load a saved model
-    // Inference only (forward): a saved model whose parameters, BF16 weights
-    // and activations are allocated stream-ordered on `stream` (the device's
+    // Inference only (forward): a saved model whose parameters and BF16 weights
+    // are allocated stream-ordered on `stream` (the device's
     // memory pool: no driver allocation or device-wide synchronisation per
     // solve) and uploaded on that stream; training calls throw.
     Mlp(const std::string& path, cudaStream_t stream);
@@ -92,11 +92,10 @@ private:
     float* m_ = nullptr;   // Adam moments
     float* v_ = nullptr;
     void* wb_ = nullptr;   // BF16 copies of W1, W2, W3
-    float* h1_ = nullptr;  // activations [cap x 128]
+    float* h1_ = nullptr;  // activations [cap x 128], for backward
     float* h2_ = nullptr;
-    float* o_ = nullptr;   // [cap x 48]
-    float* dh2_ = nullptr;
-    float* dh1_ = nullptr;
+    float* part_ = nullptr;    // backward: each CTA's share of the gradients
+    double* bpart_ = nullptr;  // and of the bias gradients
 };
 
 class LearnedPreconditioner {
