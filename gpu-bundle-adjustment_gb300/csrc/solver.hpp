@@ -255,6 +255,7 @@ public:
     DevBuf<int> acc_id_, acc_off_;
     DevBuf<float> y_acc_;
     void set_matvec(int mode);  // 0 auto (one pass), 1 two-pass (deterministic), 2 one-pass
+    DevBuf<double> cam_rec_;  // plain: per-camera constants of the FP64 Jacobians (28 per camera)
     DevBuf<double> cam_pre_;  // per-camera rotation matrix, translation, intrinsics (16 per camera)
     DevBuf<float> cam_pre_ff_;  // mixed: the same as float-float pairs (32 floats per camera)
     DevBuf<float> pts_ff_;      // mixed: float-float copy of the points being costed (6 floats per point)

@@ -389,6 +389,7 @@ Solver::Solver(int C, int P, int E, const double* cams, const double* pts, const
     if (form_ == SolverForm::Plain) {
         W_.alloc(27ull * E);
         JcR_.alloc(20ull * E);
+        cam_rec_.alloc(28ull * C);
         T_.alloc(27ull * E);
         n_pad_ = ((9 * C + 63) / 64) * 64;  // S itself is allocated at the first dense Schur step
         rhs_.alloc(n_pad_);
