@@ -49,6 +49,7 @@ namespace gba {
 namespace {
 
 constexpr int kPT = 256;
+constexpr int kLongPts = 8;  // entries of a list of long points (kPT / 33 used)
 constexpr int kCT = 128;
 constexpr int kVT = 256;  // vector-kernel threads
 constexpr int kCB = 32;   // thread-per-camera kernels: one warp per block spreads C cameras over the SMs
@@ -612,176 +613,228 @@ __global__ void __launch_bounds__(kCT) schur_camera_pass(const int* __restrict__
 // warp gives each point's sum z at its last lane, which applies V'^-1 (loaded
 // by every lane of the point up front: one request per point), and every lane
 // takes its point's w from that lane (match + shuffle); then Jc^T (Jp w) goes
-// into the slot's accumulator. No shared memory and no barrier: a warp's
-// chain is loads -> shuffles -> atomics, and 64 warps per SM hide it. Points
-// with more than 32 observations go through the chunked point pass.
+// into the slot's accumulator. Points with more than 32 observations go through
+// schur_matvec_long.
+// Bound by the memory system: 108 bytes per slot and 24 per point from DRAM, and
+// one request to L1 and L2 per gathered or accumulated record. A warp used to
+// wait for the flag, its descriptor, its indices and its records one after the
+// other; now warps stay (three CTAs per SM: more of them crowd L1, and 64
+// registers spill) and fetch the indices of their next run and the descriptor of
+// the one after it while the records of this one arrive. With schur_matvec_long,
+// 8.8 million slots: 250 -> 216 us (1.2 GB from DRAM, 5.7 TB/s).
 constexpr int kMWarps = 8;  // warps per CTA
-__global__ void __launch_bounds__(32 * kMWarps) schur_matvec_warp(
+constexpr int kMCtas = 3;   // CTAs per SM of the persistent grids
+
+// Adds each lane's q[9] into its accumulator aid of y (kX32 floats per accumulator).
+// Three lanes write one accumulator's 48 bytes (through shared memory), ten to
+// eleven accumulators per instruction, so that the reductions reach L2 as two
+// sectors per slot in few requests instead of three requests per slot. n lanes are in use.
+__device__ __forceinline__ void scatter_add(float4 (*stage)[3], const float (&q)[9], int aid, int n, float* __restrict__ y) {
+    const int lane = threadIdx.x & 31;
+    float4* st = stage[threadIdx.x];
+    st[0] = make_float4(q[0], q[1], q[2], q[3]);
+    st[1] = make_float4(q[4], q[5], q[6], q[7]);
+    st[2] = make_float4(q[8], 0.f, 0.f, 0.f);
+    __syncwarp();
+    const float4* wst = stage[threadIdx.x & ~31];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const int t = 32 * i + lane, slot = t / 3, part = t - 3 * slot;
+        const int a = __shfl_sync(0xffffffffu, aid, slot);
+        if (t < 3 * n) atomicAdd(reinterpret_cast<float4*>(y + static_cast<long long>(kX32) * a) + part, wst[t]);
+    }
+    __syncwarp();
+}
+// Inclusive sums of v over the lanes with this lane's key up to this lane (equal keys are neighbours).
+__device__ __forceinline__ void segment_scan(int key, float& v0, float& v1, float& v2) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const float u0 = __shfl_up_sync(0xffffffffu, v0, d);
+        const float u1 = __shfl_up_sync(0xffffffffu, v1, d);
+        const float u2 = __shfl_up_sync(0xffffffffu, v2, d);
+        const int kd = __shfl_up_sync(0xffffffffu, key, d);
+        if (lane >= d && kd == key) {
+            v0 += u0;
+            v1 += u1;
+            v2 += u2;
+        }
+    }
+}
+// v = Jp^T (Jc x) of a slot, J = [Jc(18), Jp(6)].
+__device__ __forceinline__ void slot_product(const float (&J)[24], const float (&xv)[9], float& v0, float& v1, float& v2) {
+    float t0 = 0.f, t1 = 0.f;
+#pragma unroll
+    for (int c = 0; c < 9; ++c) {
+        t0 = fmaf(J[c], xv[c], t0);
+        t1 = fmaf(J[9 + c], xv[c], t1);
+    }
+    v0 = fmaf(J[18], t0, J[21] * t1);
+    v1 = fmaf(J[19], t0, J[22] * t1);
+    v2 = fmaf(J[20], t0, J[23] * t1);
+}
+// A flag the PCG kernels keep as a double (0.0 = all bits zero), without the FP64 pipe.
+__device__ __forceinline__ bool flag_set(const double* f) { return f && *reinterpret_cast<const long long*>(f) != 0; }
+
+__global__ void __launch_bounds__(32 * kMWarps, kMCtas) schur_matvec_warp(
     const int2* __restrict__ wchunk, int n_wchunk, const int* __restrict__ s_cam, const int* __restrict__ s_pt,
     const int* __restrict__ acc_id, const float* __restrict__ Jc32, const float* __restrict__ Jp32, long long js,
     const float* __restrict__ vinv, const float* __restrict__ x, float* __restrict__ y,
     const double* __restrict__ done) {
+    __shared__ float4 stage[32 * kMWarps][3];
+    const int lane = threadIdx.x & 31, step = gridDim.x * kMWarps;
+    int wid = blockIdx.x * kMWarps + (threadIdx.x >> 5);
+    auto chunk = [&](int w) { return w < n_wchunk ? wchunk[w] : make_int2(0, 0); };
+    int2 r = chunk(wid), r1 = chunk(wid + step);
+    int key = -1, cam = 0, aid = 0;
+    if (r.x + lane < r.y) {
+        key = s_pt[r.x + lane];
+        cam = s_cam[r.x + lane];
+        aid = acc_id[r.x + lane];
+    }
     pdl_wait();  // x: the previous kernel's direction
-    if (done && *done != 0.0) return;
-    const int wid = blockIdx.x * kMWarps + (threadIdx.x >> 5);
-    if (wid >= n_wchunk) return;  // whole warps leave together
-    const int lane = threadIdx.x & 31;
-    const int2 r = wchunk[wid];
-    const int s = r.x + lane;
-    const bool has = s < r.y;
-    int key = -1, aid = 0;
-    float J[24], vi[6];
-    float v0 = 0.f, v1 = 0.f, v2 = 0.f;
-    if (has) {
-        key = s_pt[s];
-        aid = acc_id[s];
-        float xv[9];
-        load_x(x, s_cam[s], xv);
-        load_vinv(vinv, nullptr, key, vi);
-        load_j(Jc32, Jp32, js, s, J);
-        float t0 = 0.f, t1 = 0.f;
-#pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            t0 = fmaf(J[c], xv[c], t0);
-            t1 = fmaf(J[9 + c], xv[c], t1);
+    pdl_trigger();
+    if (flag_set(done)) return;
+    for (; wid < n_wchunk; wid += step) {
+        const int s = r.x + lane;
+        const bool has = s < r.y;
+        float J[24], vi[6], xv[9];
+        if (has) {
+            load_x(x, cam, xv);
+            load_vinv(vinv, nullptr, key, vi);
+            load_j(Jc32, Jp32, js, s, J);
         }
-        v0 = fmaf(J[18], t0, J[21] * t1);
-        v1 = fmaf(J[19], t0, J[22] * t1);
-        v2 = fmaf(J[20], t0, J[23] * t1);
-    }
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const float u0 = __shfl_up_sync(0xffffffffu, v0, d);
-        const float u1 = __shfl_up_sync(0xffffffffu, v1, d);
-        const float u2 = __shfl_up_sync(0xffffffffu, v2, d);
-        const int kd = __shfl_up_sync(0xffffffffu, key, d);
-        if (lane >= d && kd == key) {
-            v0 += u0;
-            v1 += u1;
-            v2 += u2;
+        // the next run's indices and the descriptor after it
+        int nkey = -1, ncam = 0, naid = 0;
+        if (r1.x + lane < r1.y) {
+            nkey = s_pt[r1.x + lane];
+            ncam = s_cam[r1.x + lane];
+            naid = acc_id[r1.x + lane];
         }
-    }
-    float w0 = 0.f, w1 = 0.f, w2 = 0.f;
-    if (has) apply_vinv(vi, v0, v1, v2, w0, w1, w2);  // meaningful at the point's last lane
-    const unsigned grp = __match_any_sync(0xffffffffu, key);
-    const int last = 31 - __clz(grp);
-    w0 = __shfl_sync(0xffffffffu, w0, last);
-    w1 = __shfl_sync(0xffffffffu, w1, last);
-    w2 = __shfl_sync(0xffffffffu, w2, last);
-    if (has) {
-        float u0, u1;
-        jp_times(J + 18, w0, w1, w2, u0, u1);
+        const int2 r2 = chunk(wid + 2 * step);
+        float v0 = 0.f, v1 = 0.f, v2 = 0.f;
+        if (has) slot_product(J, xv, v0, v1, v2);
+        segment_scan(key, v0, v1, v2);
+        float w0 = 0.f, w1 = 0.f, w2 = 0.f;
+        if (has) apply_vinv(vi, v0, v1, v2, w0, w1, w2);  // meaningful at the point's last lane
+        const unsigned grp = __match_any_sync(0xffffffffu, key);
+        const int last = 31 - __clz(grp);
+        w0 = __shfl_sync(0xffffffffu, w0, last);
+        w1 = __shfl_sync(0xffffffffu, w1, last);
+        w2 = __shfl_sync(0xffffffffu, w2, last);
         float q[9];
 #pragma unroll
-        for (int c = 0; c < 9; ++c) q[c] = fmaf(J[c], u0, J[9 + c] * u1);
-        float* ya = y + static_cast<long long>(kX32) * aid;
-        atomicAdd(reinterpret_cast<float4*>(ya), make_float4(q[0], q[1], q[2], q[3]));
-        atomicAdd(reinterpret_cast<float4*>(ya) + 1, make_float4(q[4], q[5], q[6], q[7]));
-        atomicAdd(ya + 8, q[8]);
+        for (int c = 0; c < 9; ++c) q[c] = 0.f;
+        if (has) {
+            float u0, u1;
+            jp_times(J + 18, w0, w1, w2, u0, u1);
+#pragma unroll
+            for (int c = 0; c < 9; ++c) q[c] = fmaf(J[c], u0, J[9 + c] * u1);
+        }
+        scatter_add(stage, q, aid, r.y - r.x, y);
+        r = r1;
+        r1 = r2;
+        key = nkey;
+        cam = ncam;
+        aid = naid;
     }
 }
 
-// The one-pass product for points with 33 to 256 observations: a CTA takes
-// a list of such points (not consecutive) whose slots total at most 256 and
-// lays them out as one virtual chunk (thread t: the t-th slot of the list);
-// the point pass of schur_point_pass follows, then Jc^T u into the slot's
-// accumulator. lchunk[k] = {first entry in lpts, entries}.
-__global__ void __launch_bounds__(kPT) schur_matvec_long(
-    const int2* __restrict__ lchunk, const int* __restrict__ lpts, const int* __restrict__ pt_off,
-    const int* __restrict__ s_cam, const int* __restrict__ acc_id, const float* __restrict__ Jc32,
-    const float* __restrict__ Jp32, long long js, const float* __restrict__ vinv, const float* __restrict__ x,
-    float* __restrict__ y, const double* __restrict__ done) {
-    constexpr int kMaxPts = kPT / 33 + 1;  // points of more than 32 slots in 256
-    __shared__ int pb[kMaxPts + 1], ps[kMaxPts], pid[kMaxPts];  // virtual begin, first real slot, point
+// The one-pass product for points with 33 to 256 observations: a CTA takes a list
+// of such points (not consecutive) whose slots total at most 256 and lays them out
+// as one virtual chunk (thread t: the t-th slot of the list); each warp's sums per
+// point are combined by the point's owner thread, which applies V'^-1, then
+// Jc^T u goes into the slot's accumulator. ldesc holds 8 entries per list, {first
+// virtual slot, first slot, point, end of the virtual slots}, empty ones {n, 0, 0, n}.
+// Bound and pipelined as schur_matvec_warp: lanes 0-7 of every warp hold the next
+// list's entries, every thread its next camera and accumulator.
+__global__ void __launch_bounds__(kPT, kMCtas) schur_matvec_long(
+    const int4* __restrict__ ldesc, int n_lchunk, const int* __restrict__ s_cam, const int* __restrict__ acc_id,
+    const float* __restrict__ Jc32, const float* __restrict__ Jp32, long long js, const float* __restrict__ vinv,
+    const float* __restrict__ x, float* __restrict__ y, const double* __restrict__ done) {
+    static_assert(kLongPts >= kPT / 33, "points of more than 32 slots in 256");
     __shared__ float seg[kPT][3];
-    __shared__ float wsh[kMaxPts][3];
-    pdl_wait();
-    if (done && *done != 0.0) return;
-    const int2 lc = lchunk[blockIdx.x];
+    __shared__ float wsh[kLongPts][3];
+    __shared__ float4 stage[kPT][3];
     const int tid = threadIdx.x, lane = tid & 31;
-    if (tid < lc.y) {  // the list's points in parallel, then their prefix
-        const int p = lpts[lc.x + tid];
-        const int o0 = pt_off[p], o1 = pt_off[p + 1];
-        pid[tid] = p;
-        ps[tid] = o0;
-        pb[tid + 1] = o1 - o0;
-    }
-    __syncwarp();
-    if (tid == 0) {
-        pb[0] = 0;
-        for (int j = 1; j <= lc.y; ++j) pb[j] += pb[j - 1];
-    }
-    __syncthreads();
-    const int n = pb[lc.y];
-    int key = -1, aid = 0;
-    long long sl = 0;
-    float J[24];
-    float v0 = 0.f, v1 = 0.f, v2 = 0.f;
-    if (tid < n) {
+    auto entry = [&](int k) {
+        return k < n_lchunk && lane < kLongPts ? ldesc[kLongPts * k + lane] : make_int4(0, 0, 0, 0);
+    };
+    // this thread's entry, slot (-1: none), camera and accumulator of the list in e
+    auto place = [&](const int4& e, int& key, int& sl, int& cam, int& aid) {
+        const int n = __shfl_sync(0xffffffffu, e.w, kLongPts - 1);
         int j = 0;
-        while (tid >= pb[j + 1]) ++j;
-        key = j;
-        sl = ps[j] + (tid - pb[j]);
-        aid = acc_id[sl];
-        float xv[9];
-        load_x(x, s_cam[sl], xv);
-        load_j(Jc32, Jp32, js, sl, J);
-        float t0 = 0.f, t1 = 0.f;
 #pragma unroll
-        for (int c = 0; c < 9; ++c) {
-            t0 = fmaf(J[c], xv[c], t0);
-            t1 = fmaf(J[9 + c], xv[c], t1);
+        for (int i = 1; i < kLongPts; ++i) j += tid >= __shfl_sync(0xffffffffu, e.x, i);
+        const int b = __shfl_sync(0xffffffffu, e.x, j), s0 = __shfl_sync(0xffffffffu, e.y, j);
+        key = sl = -1;
+        cam = aid = 0;
+        if (tid < n) {
+            key = j;
+            sl = s0 + (tid - b);
+            cam = s_cam[sl];
+            aid = acc_id[sl];
         }
-        v0 = fmaf(J[18], t0, J[21] * t1);
-        v1 = fmaf(J[19], t0, J[22] * t1);
-        v2 = fmaf(J[20], t0, J[23] * t1);
-    }
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const float u0 = __shfl_up_sync(0xffffffffu, v0, d);
-        const float u1 = __shfl_up_sync(0xffffffffu, v1, d);
-        const float u2 = __shfl_up_sync(0xffffffffu, v2, d);
-        const int kd = __shfl_up_sync(0xffffffffu, key, d);
-        if (lane >= d && kd == key) {
-            v0 += u0;
-            v1 += u1;
-            v2 += u2;
+    };
+    int k = blockIdx.x;
+    int4 e = entry(k), e1 = entry(k + gridDim.x);
+    int key, sl, cam, aid;
+    place(e, key, sl, cam, aid);
+    pdl_wait();
+    pdl_trigger();
+    if (flag_set(done)) return;
+    for (; k < n_lchunk; k += gridDim.x) {
+        float J[24], xv[9], vi[6];
+        if (sl >= 0) {
+            load_x(x, cam, xv);
+            load_j(Jc32, Jp32, js, sl, J);
         }
-    }
-    const int knext = __shfl_down_sync(0xffffffffu, key, 1);
-    if (lane == 31 || knext != key) {
-        seg[tid][0] = v0;
-        seg[tid][1] = v1;
-        seg[tid][2] = v2;
-    }
-    __syncthreads();
-    if (tid < lc.y) {  // owner of point entry tid: its warp segments in order
-        const int b = pb[tid], e = pb[tid + 1];
-        float z0 = 0.f, z1 = 0.f, z2 = 0.f;
-        for (int w = b >> 5; w <= (e - 1) >> 5; ++w) {
-            const int q = min(e - 1, 32 * w + 31);
-            z0 += seg[q][0];
-            z1 += seg[q][1];
-            z2 += seg[q][2];
+        const bool owner = tid < kLongPts && e.w > e.x;
+        if (owner) load_vinv(vinv, nullptr, e.z, vi);
+        int nkey, nsl, ncam, naid;
+        place(e1, nkey, nsl, ncam, naid);
+        const int4 e2 = entry(k + 2 * gridDim.x);
+        float v0 = 0.f, v1 = 0.f, v2 = 0.f;
+        if (sl >= 0) slot_product(J, xv, v0, v1, v2);
+        segment_scan(key, v0, v1, v2);
+        const int knext = __shfl_down_sync(0xffffffffu, key, 1);
+        if (lane == 31 || knext != key) {
+            seg[tid][0] = v0;
+            seg[tid][1] = v1;
+            seg[tid][2] = v2;
         }
-        float vi[6], w0, w1, w2;
-        load_vinv(vinv, nullptr, pid[tid], vi);
-        apply_vinv(vi, z0, z1, z2, w0, w1, w2);
-        wsh[tid][0] = w0;
-        wsh[tid][1] = w1;
-        wsh[tid][2] = w2;
-    }
-    __syncthreads();
-    if (tid < n) {
-        float u0, u1;
-        jp_times(J + 18, wsh[key][0], wsh[key][1], wsh[key][2], u0, u1);
+        __syncthreads();
+        if (owner) {  // the point's warp segments in order
+            float z0 = 0.f, z1 = 0.f, z2 = 0.f;
+            for (int w = e.x >> 5; w <= (e.w - 1) >> 5; ++w) {
+                const int q = min(e.w - 1, 32 * w + 31);
+                z0 += seg[q][0];
+                z1 += seg[q][1];
+                z2 += seg[q][2];
+            }
+            float w0, w1, w2;
+            apply_vinv(vi, z0, z1, z2, w0, w1, w2);
+            wsh[tid][0] = w0;
+            wsh[tid][1] = w1;
+            wsh[tid][2] = w2;
+        }
+        __syncthreads();
         float q[9];
 #pragma unroll
-        for (int c = 0; c < 9; ++c) q[c] = fmaf(J[c], u0, J[9 + c] * u1);
-        float* ya = y + static_cast<long long>(kX32) * aid;
-        atomicAdd(reinterpret_cast<float4*>(ya), make_float4(q[0], q[1], q[2], q[3]));
-        atomicAdd(reinterpret_cast<float4*>(ya) + 1, make_float4(q[4], q[5], q[6], q[7]));
-        atomicAdd(ya + 8, q[8]);
+        for (int c = 0; c < 9; ++c) q[c] = 0.f;
+        if (sl >= 0) {
+            float u0, u1;
+            jp_times(J + 18, wsh[key][0], wsh[key][1], wsh[key][2], u0, u1);
+#pragma unroll
+            for (int c = 0; c < 9; ++c) q[c] = fmaf(J[c], u0, J[9 + c] * u1);
+        }
+        scatter_add(stage, q, aid, __popc(__ballot_sync(0xffffffffu, sl >= 0)), y);
+        e = e1;
+        e1 = e2;
+        key = nkey;
+        sl = nsl;
+        cam = ncam;
+        aid = naid;
     }
 }
 
@@ -1805,6 +1858,335 @@ __global__ void __launch_bounds__(kVT) pcg_direction(float* __restrict__ p32, co
     if (i < n) *pp = fmaf(static_cast<float>(beta), pv, zv);
 }
 
+// ---- what follows the product of a PCG iteration in one kernel: p.q, alpha, x and
+// r, the preconditioner, the convergence test, beta and the next direction
+// (pcg_update, coarse_w, coarse_z and pcg_direction do it in up to four launches).
+// Each of those is bound by its launch and two memory round trips, for a few
+// 9-vectors per camera; between them stand only sums over all cameras. One
+// cluster of CTAs (16, or 8 where 16 do not fit a device) owns all cameras, `per`
+// consecutive ones per CTA, and takes those sums through distributed shared
+// memory: every CTA sends its partial to every other, one cluster barrier, and
+// all add the partials in the same order. FP64 instructions hold their warp's
+// scheduler for 64 cycles on this chip, so only single warps take the FP64
+// sums, and one thread the scalars.
+constexpr int kTailMaxT = 1024;
+constexpr int kTailMinT = 128;   // four warps: the sums' roles below
+constexpr int kTailMaxCtas = 16;
+// Two 9-vectors of a CTA's cameras in shared memory, also with 8 CTAs. Below, an
+// iteration (with its product) takes, separate kernels -> this one, block-Jacobi and
+// learned: 60 cameras 15.9 -> 12.5 and 10.6 -> 7.9 us; 500 18.3 -> 14.1, 19.4 -> 14.1;
+// 5,000 38 -> 29, 51 -> 37; 24,000 80 -> 69, 128 -> 99 us.
+constexpr int kTailMaxC = 24000;
+
+struct TailShared {
+    double slot[4][10][kTailMaxCtas];  // partials of each CTA, for the four sums
+    double tot[10];
+    float wp[10][33];                  // warp sums
+    float cf[kCoarse];                 // coarse coefficients
+    double c1[kCoarse];
+    float scalar;                      // alpha, then beta
+    int done;                          // the S_DONE value of this iteration
+};
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Store v at `local`'s place in the shared memory of CTA `rank` of the cluster.
+__device__ __forceinline__ void cluster_store(double* local, int rank, double v) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(local))), "r"(rank));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+
+// Totals over the cluster of NS <= 2 scalars (v[0 .. NS)) and, with kNine, of nine
+// coarse sums (v[NS .. NS + 9), into sm.tot). fin(t0, t1) runs in thread 0 with
+// the scalars' totals; what it writes to sm is visible to every thread on return.
+// Warp sums in FP32; then FP64: a scalar's warps on one warp (warp j for scalar
+// j), the nine sums on four lanes each of warps 2 and 3 (runs of eight warps
+// added in FP32 first), then the CTAs' partials the same way.
+template <int NS, bool kNine, class Fin>
+__device__ __forceinline__ void cluster_totals(const float* v, TailShared& sm, int which, int rank, int nctas, Fin fin) {
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
+    double(&slot)[10][kTailMaxCtas] = sm.slot[which];
+#pragma unroll
+    for (int j = 0; j < NS; ++j) {
+        const float t = warp_sum(v[j]);
+        if (lane == 0) sm.wp[j][warp] = t;
+    }
+    if constexpr (kNine) {
+        // halve the values and the lanes that hold them: lane l ends with sum l / 2
+        float a[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) a[j] = j < kCoarse ? v[NS + j] : 0.f;
+#pragma unroll
+        for (int o = 16, h = 8; h >= 1; o >>= 1, h >>= 1) {
+            const bool up = lane & o;
+#pragma unroll
+            for (int j = 0; j < h; ++j) {
+                const float keep = up ? a[j + h] : a[j], send = up ? a[j] : a[j + h];
+                a[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+        }
+        a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
+        if (!(lane & 1) && lane < 2 * kCoarse) sm.wp[NS + (lane >> 1)][warp] = a[0];
+    }
+    __syncthreads();
+    if (warp < NS) {
+        double d = lane < nw ? static_cast<double>(sm.wp[warp][lane]) : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        if (lane < nctas) cluster_store(&slot[warp][rank], lane, d);
+    }
+    const int j9 = NS + ((tid - 64) >> 2), g = tid & 3;
+    const bool nine = kNine && (warp == 2 || warp == 3);
+    if (nine) {
+        float f = 0.f;
+        if (j9 < NS + kCoarse)
+            for (int w = 8 * g; w < min(8 * g + 8, nw); ++w) f += sm.wp[j9][w];
+        double d = static_cast<double>(f);
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        d += __shfl_xor_sync(0xffffffffu, d, 2);
+        if (j9 < NS + kCoarse)
+            for (int c = g; c < nctas; c += 4) cluster_store(&slot[j9][rank], c, d);
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (NS > 0 && warp == 0) {  // scalar 0 on the lower lanes, scalar 1 on the upper ones
+        const int c = lane & 15;
+        double d = c < nctas && (NS == 2 || lane < 16) ? slot[lane >> 4][c] : 0.0;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+        const double d1 = NS == 2 ? __shfl_sync(0xffffffffu, d, 16) : 0.0;
+        if (lane == 0) fin(d, d1);
+    }
+    if (nine) {
+        double d = 0.0;
+        if (j9 < NS + kCoarse)
+            for (int c = g; c < nctas; c += 4) d += slot[j9][c];
+        d += __shfl_xor_sync(0xffffffffu, d, 1);
+        d += __shfl_xor_sync(0xffffffffu, d, 2);
+        if (g == 0 && j9 < NS + kCoarse) sm.tot[j9 - NS] = d;
+    }
+    __syncthreads();
+}
+
+// E^-1 t by warps 2 and 3, four lanes per row; e: the lane's entries of its row
+// (columns g, g + 4, 8 of g = 0). Result in every lane of the row.
+__device__ __forceinline__ double coarse_solve4(const double (&e)[3], const double* t) {
+    const int g = threadIdx.x & 3;
+    double d = e[0] * t[g] + e[1] * t[g + 4];
+    if (g == 0) d += e[2] * t[8];
+    d += __shfl_xor_sync(0xffffffffu, d, 1);
+    d += __shfl_xor_sync(0xffffffffu, d, 2);
+    return d;
+}
+
+// kOne: a CTA's cameras fit its threads (nine per camera), which hold their rows
+// of M, SZ and Z in registers from before the first sum; otherwise the threads
+// go over the cameras in rounds and read the rows where they use them.
+template <bool kZ, bool kOne>
+__global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ q, float* __restrict__ x,
+                                                     float* __restrict__ r, float* __restrict__ p32,
+                                                     const float* __restrict__ Minv, const float* __restrict__ Zc,
+                                                     const float* __restrict__ SZ, const double* __restrict__ einv,
+                                                     int C, int per, int max_iters, double* __restrict__ sc) {
+    extern __shared__ float tail_vec[];
+    __shared__ TailShared sm;
+    float* zs = tail_vec;            // w, then z (9 per camera of the CTA)
+    float* rs = tail_vec + 9 * per;  // r, then r - SZ c1
+    cluster_arrive();
+    const int tid = threadIdx.x, warp = tid >> 5;
+    const int rank = blockIdx.x, nctas = gridDim.x;
+    const int c0 = min(rank * per, C), m = min(per, C - c0);  // this CTA's cameras
+    const long long n = 9ll * C, i0 = 9ll * c0;
+    const int rows = 9 * m, step = kOne ? blockDim.x : 9 * (blockDim.x / 9);
+    const int first = tid < step ? tid : rows;  // this thread's first row
+    auto load9 = [&](float (&d)[9], const float* src, long long stride) {
+#pragma unroll
+        for (int j = 0; j < 9; ++j) d[j] = src[j * stride];
+    };
+    auto p_at = [&](int i) { return p32 + static_cast<long long>(kX32) * (c0 + i / 9) + i % 9; };
+    // the rows do not change during a solve's iterations
+    float mrow[9], sz[kCoarse], zc[kCoarse], xv = 0.f, rv = 0.f, pv = 0.f, qv = 0.f;
+    if (kOne) {
+#pragma unroll
+        for (int j = 0; j < 9; ++j) mrow[j] = sz[j] = zc[j] = 0.f;
+        if (first < rows) {
+            load9(mrow, Minv + 9 * (i0 + first), 1);
+            if (kZ) {
+                load9(zc, Zc + i0 + first, n);
+                load9(sz, SZ + i0 + first, n);
+            }
+        }
+    }
+    double e[3] = {0.0, 0.0, 0.0};
+    if (kZ && (warp == 2 || warp == 3)) {
+        const int row = (tid - 64) >> 2, g = tid & 3;
+        if (row < kCoarse && einv[kCoarse * kCoarse] != 0.0) {
+            e[0] = einv[row * kCoarse + g];
+            e[1] = einv[row * kCoarse + g + 4];
+            if (g == 0) e[2] = einv[row * kCoarse + 8];
+        }
+    }
+    pdl_wait();
+    pdl_trigger();
+    cluster_wait();  // every CTA of the cluster runs
+    if (flag_set(sc + S_DONE)) return;
+    double rz_old = 0.0, tol2bb = 0.0, iters = 0.0, alpha = 0.0, rr = 0.0;  // thread 0
+    if (tid == 0) {
+        rz_old = sc[S_RZ];
+        tol2bb = sc[S_TOL2] * sc[S_BB];
+        iters = sc[S_ITERS] + 1.0;
+    }
+
+    float v[10];
+#pragma unroll
+    for (int j = 0; j < 10; ++j) v[j] = 0.f;
+    for (int i = first; i < rows; i += step) {
+        pv = *p_at(i);
+        qv = q[i0 + i];
+        v[0] = fmaf(pv, qv, v[0]);
+        if (kOne) {
+            xv = x[i0 + i];
+            rv = r[i0 + i];
+        }
+    }
+    cluster_totals<1, false>(v, sm, 0, rank, nctas, [&](double pq, double) {
+        const bool ok = pq > 0.0 && isfinite(pq);
+        alpha = ok ? rz_old / pq : 0.0;
+        sm.scalar = static_cast<float>(alpha);
+        sm.done = ok ? 0 : 2;
+    });
+    if (sm.done) {
+        if (rank == 0 && tid == 0) sc[S_DONE] = 2.0;  // breakdown: keep the current iterate
+        return;
+    }
+    const float af = sm.scalar;
+
+    // x, r; r.r and Z^T r, or z = M r and r.z
+    v[0] = 0.f;
+    for (int i = first; i < rows; i += step) {
+        if (!kOne) {
+            xv = x[i0 + i];
+            rv = r[i0 + i];
+            pv = *p_at(i);
+            qv = q[i0 + i];
+            if (kZ) load9(zc, Zc + i0 + i, n);
+        }
+        x[i0 + i] = fmaf(af, pv, xv);
+        rv = fmaf(-af, qv, rv);
+        r[i0 + i] = rv;
+        rs[i] = rv;
+        v[0] = fmaf(rv, rv, v[0]);
+        if (kZ) {
+#pragma unroll
+            for (int j = 0; j < kCoarse; ++j) v[1 + j] = fmaf(zc[j], rv, v[1 + j]);
+        }
+    }
+    // the convergence test, and beta
+    auto test = [&](double rr_t) { return rr_t <= tol2bb || iters >= max_iters ? 1 : 0; };
+    auto direction = [&](double rz) {
+        if (sm.done == 0 && (!(rz > 0.0) || !isfinite(rz))) sm.done = 2;
+        const double beta = rz / rz_old;
+        sm.scalar = static_cast<float>(beta);
+        if (rank != 0) return;
+        sc[S_ALPHA] = alpha;
+        sc[S_RZPREV] = rz_old;
+        sc[S_ITERS] = iters;
+        sc[S_RR] = rr;
+        if (sm.done) {
+            sc[S_DONE] = sm.done;
+        } else {
+            sc[S_BETA] = beta;
+            sc[S_RZ] = rz;
+        }
+    };
+    if constexpr (!kZ) {
+        __syncthreads();
+        for (int i = first; i < rows; i += step) {
+            if (!kOne) load9(mrow, Minv + 9 * (i0 + i), 1);
+            const float* r9 = rs + i - i % 9;
+            float z = 0.f;
+#pragma unroll
+            for (int j = 0; j < 9; ++j) z = fmaf(mrow[j], r9[j], z);
+            zs[i] = z;
+            v[1] = fmaf(rs[i], z, v[1]);
+        }
+        cluster_totals<2, false>(v, sm, 1, rank, nctas, [&](double rr_t, double rz_t) {
+            rr = rr_t;
+            sm.done = test(rr_t);
+            direction(rz_t);
+        });
+    } else {
+        cluster_totals<1, true>(v, sm, 1, rank, nctas, [&](double rr_t, double) {
+            rr = rr_t;
+            sm.done = test(rr_t);
+            if (sm.done) direction(1.0);
+        });
+        if (sm.done) return;
+        // w = M (r - SZ c1) and SZ^T w
+        const int row = (tid - 64) >> 2;
+        const bool coeff = (warp == 2 || warp == 3) && row < kCoarse && (tid & 3) == 0;
+        if (warp == 2 || warp == 3) {
+            const double c = coarse_solve4(e, sm.tot);
+            if (coeff) {
+                sm.c1[row] = c;
+                sm.cf[row] = static_cast<float>(c);
+            }
+        }
+        __syncthreads();
+        for (int i = first; i < rows; i += step) {
+            if (!kOne) load9(sz, SZ + i0 + i, n);
+            float yi = rs[i];
+#pragma unroll
+            for (int j = 0; j < kCoarse; ++j) yi = fmaf(-sz[j], sm.cf[j], yi);
+            rs[i] = yi;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < kCoarse; ++j) v[j] = 0.f;
+        for (int i = first; i < rows; i += step) {
+            if (!kOne) {
+                load9(mrow, Minv + 9 * (i0 + i), 1);
+                load9(sz, SZ + i0 + i, n);
+            }
+            const float* y9 = rs + i - i % 9;
+            float w = 0.f;
+#pragma unroll
+            for (int j = 0; j < 9; ++j) w = fmaf(mrow[j], y9[j], w);
+            zs[i] = w;
+#pragma unroll
+            for (int j = 0; j < kCoarse; ++j) v[j] = fmaf(sz[j], w, v[j]);
+        }
+        cluster_totals<0, true>(v, sm, 2, rank, nctas, [](double, double) {});
+        // z = w + Z (c1 - c2) and r.z
+        if (warp == 2 || warp == 3) {
+            const double c = coarse_solve4(e, sm.tot);
+            if (coeff) sm.cf[row] = static_cast<float>(sm.c1[row] - c);
+        }
+        __syncthreads();
+        v[0] = 0.f;
+        for (int i = first; i < rows; i += step) {
+            if (!kOne) {
+                load9(zc, Zc + i0 + i, n);
+                rv = r[i0 + i];
+            }
+            float z = zs[i];
+#pragma unroll
+            for (int j = 0; j < kCoarse; ++j) z = fmaf(zc[j], sm.cf[j], z);
+            zs[i] = z;
+            v[0] = fmaf(rv, z, v[0]);
+        }
+        cluster_totals<1, false>(v, sm, 3, rank, nctas, [&](double rz_t, double) { direction(rz_t); });
+    }
+    if (sm.done) return;
+    const float bf = sm.scalar;
+    for (int i = first; i < rows; i += step) {
+        float* pp = p_at(i);
+        *pp = fmaf(bf, kOne ? pv : *pp, zs[i]);
+    }
+}
+
 // x = 0, r = b (rounded to FP32), z = M r, p = z; partials b.b and r.z. Nine
 // threads per camera. With a coarse basis (Zc non-null): x = 0, r = b and the
 // partials b.b and Z^T b; coarse_w / coarse_z then form z = p and the r.z partials.
@@ -2080,17 +2462,17 @@ static void camera_parts_ff(Solver& s) {
 // Jc^T u, accumulated in device memory (acc_id_: the slot's accumulator).
 static void implicit_parts_acc(Solver& s, const float* x, const double* done) {
     cudaEvent_t ev = s.prof_start();
+    const int resident = kMCtas * device_sm_count();
     if (s.n_wchunk_ > 0) {
-        launch_pdl(schur_matvec_warp, ceil_div(s.n_wchunk_, kMWarps), 32 * kMWarps, 0, s.stream_,
+        launch_pdl(schur_matvec_warp, std::min(ceil_div(s.n_wchunk_, kMWarps), resident), 32 * kMWarps, 0, s.stream_,
                        reinterpret_cast<const int2*>(s.wchunk_.get()), s.n_wchunk_, s.s_cam_.get(), s.s_pt_.get(),
                        s.acc_id_.get(), s.Jc32_.get(), s.Jp32_.get(), s.js_, s.Vinv32_.get(), x, s.y_acc_.get(),
                        done);
     }
     if (s.n_lchunk_ > 0) {  // points with 33 to 256 observations, packed per CTA
-        launch_pdl(schur_matvec_long, s.n_lchunk_, kPT, 0, s.stream_,
-                       reinterpret_cast<const int2*>(s.lchunk_.get()), s.lpts_.get(), s.pt_off_.get(),
-                       s.s_cam_.get(), s.acc_id_.get(), s.Jc32_.get(), s.Jp32_.get(), s.js_, s.Vinv32_.get(), x,
-                       s.y_acc_.get(), done);
+        launch_pdl(schur_matvec_long, std::min(s.n_lchunk_, resident), kPT, 0, s.stream_,
+                       reinterpret_cast<const int4*>(s.ldesc_.get()), s.n_lchunk_, s.s_cam_.get(), s.acc_id_.get(),
+                       s.Jc32_.get(), s.Jp32_.get(), s.js_, s.Vinv32_.get(), x, s.y_acc_.get(), done);
     }
     if (s.n_huge_ > 0) {  // points with more than 256 observations, one range each
         schur_point_pass<float, false, false, true><<<s.n_huge_, kPT, 0, s.stream_>>>(
@@ -2106,6 +2488,76 @@ void launch_split_ff(const double* x, long long n, float* out, cudaStream_t s) {
     if (n <= 0) return;
     split_kernel<<<ceil_div(n, kVT), kVT, 0, s>>>(x, n, out);
     GBA_LAUNCH_CHECK();
+}
+
+// The tail's cluster. ctas 0: the separate kernels.
+struct TailPlan {
+    int ctas = 0, per = 0, threads = 0;
+    bool one_round = false;  // every camera row has a thread
+    size_t smem = 0;
+};
+static cudaLaunchConfig_t tail_config(const TailPlan& t, cudaStream_t stream, cudaLaunchAttribute* at) {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = t.ctas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(static_cast<unsigned>(t.ctas));
+    cfg.blockDim = dim3(static_cast<unsigned>(t.threads));
+    cfg.dynamicSmemBytes = t.smem;
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    return cfg;
+}
+// What a cluster of t needs beyond the defaults.
+template <bool kZ, bool kOne>
+static void allow_tail(const TailPlan& t) {
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(pcg_tail<kZ, kOne>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(pcg_tail<kZ, kOne>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(t.smem)));
+}
+template <bool kZ, bool kOne>
+static void launch_tail_as(Solver& s, const TailPlan& t, int max_iters) {
+    cudaLaunchAttribute at[2];
+    const cudaLaunchConfig_t cfg = tail_config(t, s.stream_, at);
+    allow_tail<kZ, kOne>(t);
+    GBA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, pcg_tail<kZ, kOne>,
+                                      static_cast<const float*>(s.pcg_q_.get()), s.pcg_e_.get(), s.pcg_r_.get(),
+                                      s.pcg_p32_.get(), static_cast<const float*>(s.Pinv_.get()),
+                                      static_cast<const float*>(s.cz32_.get()),
+                                      static_cast<const float*>(s.csz32_.get()),
+                                      static_cast<const double*>(s.ceinv_.get()), s.C_, t.per, max_iters,
+                                      s.pcg_s_.get()));
+    count_launch();
+}
+static void launch_tail(Solver& s, const TailPlan& t, bool coarse, int max_iters) {
+    cudaEvent_t ev = s.prof_start();
+    if (coarse)
+        t.one_round ? launch_tail_as<true, true>(s, t, max_iters) : launch_tail_as<true, false>(s, t, max_iters);
+    else
+        t.one_round ? launch_tail_as<false, true>(s, t, max_iters) : launch_tail_as<false, false>(s, t, max_iters);
+    s.prof_stop("pcg_tail", ev);
+}
+static TailPlan plan_tail(const Solver& s) {
+    TailPlan t;
+    if (s.C_ > kTailMaxC) return t;
+    for (int ctas : {kTailMaxCtas, kTailMaxCtas / 2}) {  // 16 CTAs per cluster are an opt-in the device may refuse
+        t.ctas = ctas;
+        t.per = ceil_div(s.C_, ctas);
+        t.one_round = 9 * t.per <= kTailMaxT;
+        t.threads = t.one_round ? std::max(kTailMinT, 32 * ceil_div(9 * t.per, 32)) : kTailMaxT;
+        t.smem = 2 * 9 * sizeof(float) * t.per;
+        if (ctas == kTailMaxCtas / 2) return t;
+        cudaLaunchAttribute at[2];
+        const cudaLaunchConfig_t cfg = tail_config(t, s.stream_, at);
+        int fit = 0;
+        allow_tail<true, true>(t);
+        if (cudaOccupancyMaxActiveClusters(&fit, pcg_tail<true, true>, &cfg) == cudaSuccess && fit > 0) return t;
+        cudaGetLastError();
+    }
+    return t;
 }
 
 // Mixed-form back-substitution: the point pass in back-substitution mode (dp,
@@ -2199,6 +2651,7 @@ PcgStats Solver::schur_pcg(double lambda, const LMOptions& opts, bool learned, u
     // The learned coarse space (basis, S Z, E^-1) is formed once per trial, when
     // an inner solve first needs it.
     bool coarse_ready = false;
+    const TailPlan tail = plan_tail(*this);
     // Inner PCG on the FP32 operator, S32 e = r (e in pcg_e_, FP32), preconditioned by
     // block-Jacobi, or by the balancing two-level form with the learned coarse
     // basis (coarse). Returns the iteration count; *ok = reached the inner
@@ -2242,17 +2695,22 @@ PcgStats Solver::schur_pcg(double lambda, const LMOptions& opts, bool learned, u
             for (int j = 0; j < batch; ++j) {
                 if (one_pass_) {
                     implicit_parts_acc(*this, pcg_p32_.get(), done);
-                    cudaEvent_t fev = prof_start();
-                    launch_pdl(pcg_q_finalize_acc, npq, kVT, 0, stream_, y_acc_.get(), acc_off_.get(),
-                                   ul32_.get(), pcg_p32_.get(), C_, pcg_q_.get(), red_pq, sc);
-                    prof_stop("pcg_q_finalize", fev);
                 } else {
                     implicit_parts<float>(*this, pcg_p32_.get(), 0.0, done);
-                    cudaEvent_t fev = prof_start();
+                }
+                cudaEvent_t fev = prof_start();
+                if (one_pass_) {
+                    launch_pdl(pcg_q_finalize_acc, npq, kVT, 0, stream_, y_acc_.get(), acc_off_.get(), ul32_.get(),
+                                   pcg_p32_.get(), C_, pcg_q_.get(), red_pq, sc);
+                } else {
                     pcg_q_finalize<<<nvb, kVT, 0, stream_>>>(cam_chunk_off_.get(), cam_part_.get(), ul32_.get(),
                                                              pcg_p32_.get(), C_, pcg_q_.get(), red_pq, sc);
                     GBA_LAUNCH_CHECK();
-                    prof_stop("pcg_q_finalize", fev);
+                }
+                prof_stop("pcg_q_finalize", fev);
+                if (tail.ctas) {
+                    launch_tail(*this, tail, coarse, max_iters);
+                    continue;
                 }
                 launch_pdl(pcg_update, nub, kUT, 0, stream_, pcg_e_.get(), pcg_r_.get(), pcg_z_.get(),
                                pcg_p32_.get(), pcg_q_.get(), Pinv_.get(), C_, red_pq, npq, red, red2, sc, Zc, red_zr);
@@ -2533,7 +2991,20 @@ void Solver::build_point_groups() {
     if (!wc.empty())
         GBA_CUDA_CHECK(cudaMemcpyAsync(wchunk_.get(), wc.data(), wc.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                        stream_));
+    std::vector<int4> ld(kLongPts * std::max<size_t>(lc.size(), 1));
+    for (size_t k = 0; k < lc.size(); ++k) {  // schur_matvec_long's form of the lists
+        int v = 0;
+        for (int j = 0; j < lc[k].y; ++j) {
+            const int p = lp[lc[k].x + j], n = off[p + 1] - off[p];
+            ld[kLongPts * k + j] = make_int4(v, off[p], p, v + n);
+            v += n;
+        }
+        for (int j = lc[k].y; j < kLongPts; ++j) ld[kLongPts * k + j] = make_int4(v, 0, 0, v);
+    }
+    ldesc_.alloc(4 * ld.size());
     if (!lc.empty()) {
+        GBA_CUDA_CHECK(cudaMemcpyAsync(ldesc_.get(), ld.data(), ld.size() * sizeof(int4), cudaMemcpyHostToDevice,
+                                       stream_));
         GBA_CUDA_CHECK(cudaMemcpyAsync(lchunk_.get(), lc.data(), lc.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                        stream_));
         GBA_CUDA_CHECK(cudaMemcpyAsync(lpts_.get(), lp.data(), lp.size() * sizeof(int), cudaMemcpyHostToDevice,

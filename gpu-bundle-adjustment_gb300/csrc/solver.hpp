@@ -250,7 +250,7 @@ public:
     // entries}); longer points as ranges (int4 {p, p + 1, first slot, end
     // slot}) for the chunked point passes
     int n_wchunk_ = 0, n_lchunk_ = 0, n_huge_ = 0;
-    DevBuf<int> wchunk_, lchunk_, lpts_, huge_range_;
+    DevBuf<int> wchunk_, lchunk_, lpts_, ldesc_, huge_range_;
     void build_point_groups();  // pcg.cu
     DevBuf<int> acc_id_, acc_off_;
     DevBuf<float> y_acc_;
