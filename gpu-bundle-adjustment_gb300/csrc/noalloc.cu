@@ -33,10 +33,14 @@
 namespace gba {
 namespace {
 
-constexpr int kCostThreads = 256;
-constexpr int kCostPerThread = 8;
+// Bound by the FP64 pipe (67 instructions an observation), so the CTAs have to be
+// many enough to spread evenly: with 2048 observations each, 800,000 made 391 CTAs
+// on 152 SMs, three on some and two on others: 137 -> 124 us (214 with sine, cosine
+// and root instead of the series).
+constexpr int kCostThreads = 128;
+constexpr int kCostPerThread = 4;
 constexpr int kCostChunk = kCostThreads * kCostPerThread;  // observations per CTA
-constexpr int kCostScratchChunks = 32768;                  // -> at most 67,108,864 observations
+constexpr int kCostScratchChunks = 131072;                 // -> at most 67,108,864 observations
 
 // [0, kCostScratchChunks): per-chunk SSE; [kCostScratchChunks, 2 kCostScratchChunks):
 // per-chunk count of non-finite residuals (exact in FP64 below 2^53).
@@ -48,8 +52,10 @@ __global__ void __launch_bounds__(kCostThreads) cost_chunk_kernel(const double* 
                                                                  const double* __restrict__ px, int E,
                                                                  double* __restrict__ scratch) {
     __shared__ double red[kCostThreads / 32];
+    __shared__ int badw[kCostThreads / 32];
     const long long base = static_cast<long long>(blockIdx.x) * kCostChunk;
-    double sse = 0.0, bad = 0.0;
+    double sse = 0.0;
+    int bad = 0;
 #pragma unroll 1
     for (int k = 0; k < kCostPerThread; ++k) {
         const long long e = base + k * kCostThreads + threadIdx.x;
@@ -67,12 +73,16 @@ __global__ void __launch_bounds__(kCostThreads) cost_chunk_kernel(const double* 
         if (isfinite(r[0]) && isfinite(r[1]))
             sse += r[0] * r[0] + r[1] * r[1];
         else
-            bad += 1.0;
+            ++bad;
     }
     const double s = block_sum<kCostThreads>(sse, red);
-    const double b = block_sum<kCostThreads>(bad, red);
+    bad = __reduce_add_sync(0xffffffffu, bad);
+    if ((threadIdx.x & 31) == 0) badw[threadIdx.x >> 5] = bad;
+    __syncthreads();
     if (threadIdx.x == 0) {
         scratch[blockIdx.x] = s;
+        int b = 0;
+        for (int w = 0; w < kCostThreads / 32; ++w) b += badw[w];
         scratch[kCostScratchChunks + blockIdx.x] = b;
     }
 }
@@ -82,6 +92,7 @@ __global__ void __launch_bounds__(256) cost_chunk_finalize(const double* __restr
                                                           unsigned long long* __restrict__ out_bad) {
     __shared__ double red[8];
     double s = 0.0, b = 0.0;
+#pragma unroll 4
     for (int i = threadIdx.x; i < nchunks; i += 256) {
         s += scratch[i];
         b += scratch[kCostScratchChunks + i];
