@@ -32,7 +32,7 @@ __global__ void __launch_bounds__(kTB) damp_invert_v_kernel(const double* __rest
         a[2] += lambda * (a[2] > 0.0 ? a[2] : 1e-12);
         a[5] += lambda * (a[5] > 0.0 ? a[5] : 1e-12);
         double inv[6];
-        if (!blk::inverse3_packed(a, inv)) {
+        if (!blk::inverse3_ldl(a, inv) && !blk::inverse3_packed(a, inv)) {
             ++bad;
 #pragma unroll
             for (int k = 0; k < 6; ++k) inv[k] = 0.0;
@@ -116,38 +116,85 @@ __global__ void __launch_bounds__(kTB) damp_invert_v_ff_kernel(const double* __r
     if (threadIdx.x == 0 && nb) atomicAdd(nonspd, nb);
 }
 
-__global__ void batch_chol9_kernel(const double* __restrict__ A, const double* __restrict__ b, double* __restrict__ x,
-                                   int* __restrict__ ok, int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double L[45];
-    const bool good = blk::chol9_factor(A + 81ll * i, L);
-    ok[i] = good ? 1 : 0;
-    if (good) {
-        double xi[9], bi[9];
+// Batched blocks, one per thread. The arrays are row-major per block, so a warp
+// brings its 32 blocks through shared memory: a column of them touches a sector
+// per lane. What is left is the FP64 chain of a block (64 cycles an instruction,
+// whether one lane or 32 use it).
+template <int N, int kLd>
+__device__ __forceinline__ void load_blocks(const double* __restrict__ src, double* stage, int rows) {
+    const int lane = threadIdx.x & 31;
 #pragma unroll
-        for (int k = 0; k < 9; ++k) bi[k] = b[9ll * i + k];
-        blk::chol9_solve(L, bi, xi);
+    for (int k = 0; k < N; ++k) {
+        const int i = 32 * k + lane;
+        if (i < N * rows) stage[kLd * (i / N) + i % N] = src[i];
+    }
+    __syncwarp();
+}
+// Rows of stage whose bit is set in good to dst.
+template <int N, int kLd>
+__device__ __forceinline__ void store_blocks(const double* stage, unsigned good, double* __restrict__ dst) {
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
 #pragma unroll
-        for (int k = 0; k < 9; ++k) x[9ll * i + k] = xi[k];
+    for (int k = 0; k < N; ++k) {
+        const int i = 32 * k + lane;
+        if (good >> (i / N) & 1) dst[i] = stage[kLd * (i / N) + i % N];
     }
 }
 
-__global__ void batch_inverse3_kernel(const double* __restrict__ A, double* __restrict__ Ainv, int* __restrict__ ok,
-                                      int n) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const double* a = A + 9ll * i;
-    const double pk[6] = {a[0], a[3], a[4], a[6], a[7], a[8]};  // lower triangle, row-major
-    double inv[6];
-    const bool good = blk::inverse3_packed(pk, inv);
-    ok[i] = good ? 1 : 0;
-    if (good) {
-        double* o = Ainv + 9ll * i;
-        o[0] = inv[0]; o[1] = inv[1]; o[2] = inv[3];
-        o[3] = inv[1]; o[4] = inv[2]; o[5] = inv[4];
-        o[6] = inv[3]; o[7] = inv[4]; o[8] = inv[5];
+constexpr int kChol9T = 32;
+__global__ void __launch_bounds__(kChol9T) batch_chol9_kernel(const double* __restrict__ A, const double* __restrict__ b,
+                                                             double* __restrict__ x, int* __restrict__ ok, int n) {
+    __shared__ double As[32 * 81], bs[32 * 9];
+    const int base = blockIdx.x * kChol9T, rows = min(32, n - base), lane = threadIdx.x;
+    load_blocks<9, 9>(b + 9ll * base, bs, rows);
+    load_blocks<81, 81>(A + 81ll * base, As, rows);
+    bool good = false;
+    if (lane < rows) {
+        const double* a = As + 81 * lane;
+        double t[45], xi[9];
+#pragma unroll
+        for (int i = 0; i < 9; ++i)
+#pragma unroll
+            for (int j = 0; j <= i; ++j) t[blk::tri(i, j)] = a[9 * i + j];
+        good = blk::solve9_ldl(t, bs + 9 * lane, xi);
+        if (!good) {
+            good = blk::chol9_factor(a, t);
+            if (good) blk::chol9_solve(t, bs + 9 * lane, xi);
+        }
+        ok[base + lane] = good ? 1 : 0;
+        if (good) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) bs[9 * lane + k] = xi[k];
+        }
     }
+    store_blocks<9, 9>(bs, __ballot_sync(0xffffffffu, good), x + 9ll * base);
+}
+
+constexpr int kInv3T = 128;
+__global__ void __launch_bounds__(kInv3T) batch_inverse3_kernel(const double* __restrict__ A,
+                                                               double* __restrict__ Ainv, int* __restrict__ ok,
+                                                               int n) {
+    __shared__ double stages[kInv3T / 32][32 * 9];
+    double* stage = stages[threadIdx.x >> 5];
+    const int base = blockIdx.x * kInv3T + (threadIdx.x & ~31), lane = threadIdx.x & 31;
+    if (base >= n) return;  // whole warps
+    const int rows = min(32, n - base);
+    load_blocks<9, 9>(A + 9ll * base, stage, rows);
+    bool good = false;
+    if (lane < rows) {
+        double* o = stage + 9 * lane;
+        const double pk[6] = {o[0], o[3], o[4], o[6], o[7], o[8]};  // lower triangle, row-major
+        double inv[6];
+        good = blk::inverse3_ldl(pk, inv) || blk::inverse3_packed(pk, inv);
+        ok[base + lane] = good ? 1 : 0;
+        if (good) {
+            o[0] = inv[0]; o[1] = inv[1]; o[2] = inv[3];
+            o[3] = inv[1]; o[4] = inv[2]; o[5] = inv[4];
+            o[6] = inv[3]; o[7] = inv[4]; o[8] = inv[5];
+        }
+    }
+    store_blocks<9, 9>(stage, __ballot_sync(0xffffffffu, good), Ainv + 9ll * base);
 }
 
 // Plain-form point back-substitution, one CTA per point chunk (slots sorted by
@@ -330,13 +377,13 @@ void Solver::backsub_launch(double lambda, bool reuse) {
 
 void launch_batch_chol9_factor_solve(const double* A, const double* b, double* x, int* ok, int n, cudaStream_t s) {
     if (n <= 0) return;
-    batch_chol9_kernel<<<ceil_div(n, 128), 128, 0, s>>>(A, b, x, ok, n);
+    batch_chol9_kernel<<<ceil_div(n, kChol9T), kChol9T, 0, s>>>(A, b, x, ok, n);
     GBA_LAUNCH_CHECK();
 }
 
 void launch_batch_inverse3_spd(const double* A, double* Ainv, int* ok, int n, cudaStream_t s) {
     if (n <= 0) return;
-    batch_inverse3_kernel<<<ceil_div(n, 128), 128, 0, s>>>(A, Ainv, ok, n);
+    batch_inverse3_kernel<<<ceil_div(n, kInv3T), kInv3T, 0, s>>>(A, Ainv, ok, n);
     GBA_LAUNCH_CHECK();
 }
 

@@ -38,27 +38,6 @@ __device__ __forceinline__ bool chol9_factor(const T* A, T* L) {
     return true;
 }
 
-// Same, from a packed symmetric lower triangle (45).
-template <typename T>
-__device__ __forceinline__ bool chol9_factor_packed(const T* A, T* L) {
-#pragma unroll
-    for (int i = 0; i < 9; ++i) {
-#pragma unroll
-        for (int j = 0; j <= i; ++j) {
-            T s = A[tri(i, j)];
-#pragma unroll
-            for (int k = 0; k < j; ++k) s -= L[tri(i, k)] * L[tri(j, k)];
-            if (i == j) {
-                if (!(s > T(0))) return false;
-                L[tri(i, i)] = bsqrt(s);
-            } else {
-                L[tri(i, j)] = s / L[tri(j, j)];
-            }
-        }
-    }
-    return true;
-}
-
 // Solve L L^T x = b.
 template <typename T>
 __device__ __forceinline__ void chol9_solve(const T* L, const T* b, T* x) {
@@ -102,6 +81,76 @@ __device__ __forceinline__ bool inverse3_packed(const T* a, T* inv) {
     inv[3] = m20 * m22;
     inv[4] = m21 * m22;
     inv[5] = m22 * m22;
+    return true;
+}
+
+// The root-free forms A = L D L^T, L unit lower: one reciprocal per pivot instead
+// of a root and the divisions by it (an FP64 reciprocal, root or division holds
+// its warp for 350 to 690 cycles on this chip, a multiplication for 64). They
+// stand for the routines above where every pivot is clearly positive (clear: more
+// than kClear of its diagonal entry, and with a finite reciprocal); otherwise they
+// return false and the caller asks the Cholesky form, which decides what is SPD.
+constexpr double kClear = 1e-10;
+__device__ __forceinline__ bool clear_pivot(double d, double diag) { return d > kClear * diag && d > 1e-280 && d < 1e280; }
+
+__device__ __forceinline__ bool inverse3_ldl(const double* a, double* inv) {
+    if (!clear_pivot(a[0], a[0])) return false;
+    const double r0 = 1.0 / a[0];
+    const double l10 = a[1] * r0, l20 = a[3] * r0;
+    const double d1 = a[2] - l10 * a[1];
+    if (!clear_pivot(d1, a[2])) return false;
+    const double u21 = a[4] - l20 * a[1], r1 = 1.0 / d1;
+    const double l21 = u21 * r1;
+    const double d2 = a[5] - l20 * a[3] - l21 * u21;
+    if (!clear_pivot(d2, a[5])) return false;
+    const double r2 = 1.0 / d2;
+    const double m20 = l10 * l21 - l20;  // L^-1 = [1; -l10 1; m20 -l21 1]
+    inv[5] = r2;
+    inv[4] = -l21 * r2;
+    inv[3] = m20 * r2;
+    inv[2] = r1 - l21 * inv[4];
+    const double q = l10 * r1;
+    inv[1] = -q - l21 * inv[3];
+    inv[0] = r0 + l10 * q + m20 * inv[3];
+    return true;
+}
+
+// x = A^-1 b, A: packed lower triangle (45), overwritten by L and D.
+__device__ __forceinline__ bool solve9_ldl(double* a, const double* b, double* x) {
+    double r[9], diag[9];
+#pragma unroll
+    for (int i = 0; i < 9; ++i) diag[i] = a[tri(i, i)];
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        ok = ok && clear_pivot(a[tri(k, k)], diag[k]);
+        r[k] = 1.0 / a[tri(k, k)];
+        double u[9];
+#pragma unroll
+        for (int i = k + 1; i < 9; ++i) {
+            u[i] = a[tri(i, k)];
+            a[tri(i, k)] = u[i] * r[k];
+        }
+#pragma unroll
+        for (int i = k + 1; i < 9; ++i)
+#pragma unroll
+            for (int j = k + 1; j <= i; ++j) a[tri(i, j)] -= a[tri(i, k)] * u[j];
+    }
+    if (!ok) return false;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) {
+        double s = b[i];
+#pragma unroll
+        for (int k = 0; k < i; ++k) s -= a[tri(i, k)] * x[k];
+        x[i] = s;
+    }
+#pragma unroll
+    for (int i = 8; i >= 0; --i) {
+        double s = x[i] * r[i];
+#pragma unroll
+        for (int k = i + 1; k < 9; ++k) s -= a[tri(k, i)] * x[k];
+        x[i] = s;
+    }
     return true;
 }
 
