@@ -932,21 +932,20 @@ __global__ void __launch_bounds__(kVT) pcg_q_finalize(const int* __restrict__ ca
 // (the grid has ceil(C / 8) blocks of 8 warps): lanes take the accumulators in
 // turn as float4 runs, two per lane per round with both loads issued before
 // the stores, then a warp reduction; one p.q partial per block. The loads that
-// do not depend on the product (offsets, U_lambda row, p) go out with the done
-// flag's, so that a warp waits for two memory round trips, not five. All FP32
-// but the block partial.
+// do not depend on the product (offsets, U_lambda row, p, the done flag) go out
+// before the wait for it: the product's blocks let this kernel start only after
+// they have waited for the kernel that wrote p and the flag. All FP32 but the
+// block partial.
 __global__ void __launch_bounds__(kVT) pcg_q_finalize_acc(float* __restrict__ y, const int* __restrict__ acc_off,
                                                          const float* __restrict__ Ul,
                                                          const float* __restrict__ p32, int C,
                                                          float* __restrict__ q, double* __restrict__ red,
                                                          const double* __restrict__ sc) {
     __shared__ double sh[kVT / 32];
-    pdl_wait();
-    pdl_trigger();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x * (kVT / 32) + warp;
     const bool cam = c < C;
-    const double done = sc[S_DONE];
+    const bool done = flag_set(sc + S_DONE);
     int r0 = 0, r1 = 0;
     float u[9], pc[9], pown = 0.f;
 #pragma unroll
@@ -965,7 +964,9 @@ __global__ void __launch_bounds__(kVT) pcg_q_finalize_acc(float* __restrict__ y,
             pown = pr[lane];
         }
     }
-    if (done != 0.0) return;  // the same value in every thread of the grid
+    pdl_wait();
+    pdl_trigger();
+    if (done) return;  // the same value in every thread of the grid
     float a[9];
 #pragma unroll
     for (int t = 0; t < 9; ++t) a[t] = 0.f;
@@ -1581,11 +1582,15 @@ __global__ void __launch_bounds__(kC9) coarse_camera_pass9(const int* __restrict
     float acc[9];
 #pragma unroll
     for (int i = 0; i < 9; ++i) acc[i] = 0.f;
+#pragma unroll 4
     for (int q = b + g; q < e; q += 16) {
-        const float* rec = J32c + 20ll * q;
+        const float4* rec = reinterpret_cast<const float4*>(J32c + 20ll * q);  // 80-byte records
         const float2 u = reinterpret_cast<const float2*>(u9 + static_cast<long long>(kU9) * q)[j];
+        float Jc[20];
 #pragma unroll
-        for (int i = 0; i < 9; ++i) acc[i] = fmaf(__ldg(rec + i), u.x, fmaf(__ldg(rec + 9 + i), u.y, acc[i]));
+        for (int t = 0; t < 5; ++t) reinterpret_cast<float4*>(Jc)[t] = __ldg(rec + t);
+#pragma unroll
+        for (int i = 0; i < 9; ++i) acc[i] = fmaf(Jc[i], u.x, fmaf(Jc[9 + i], u.y, acc[i]));
     }
 #pragma unroll
     for (int i = 0; i < 9; ++i) sh[g][9 * i + j] = acc[i];
@@ -1616,103 +1621,90 @@ __global__ void __launch_bounds__(kVT) coarse_sz_finalize(const int* __restrict_
     SZ32[j * n + 9ll * c + i] = static_cast<float>(v);
 }
 
-// Block partials of E = Z^T SZ: red[block * kCoarse^2 + a kCoarse + b] over the
-// block's entries (one per thread): warp shuffle sums per pair, then the warps'
-// sums in warp order (one barrier).
-__global__ void __launch_bounds__(kVT) coarse_gram_partials(const double* __restrict__ Zc,
-                                                           const double* __restrict__ SZ, long long n,
-                                                           double* __restrict__ red) {
+// Block partials of E = Z^T S Z (81 per block, red[81 block + 9 a + b]), `rows` rows
+// per block: thread (g, a, b) takes every third row from shared memory. Bound by the
+// FP64 pipe of few SMs: 43 -> 8 us at 257 cameras against 81 warp sums per warp.
+constexpr int kGramRows = 64;               // rows per pass of a block
+constexpr int kGramT = 3 * kCoarse * kCoarse;
+__global__ void __launch_bounds__(kGramT) coarse_gram_partials(const double* __restrict__ Zc,
+                                                              const double* __restrict__ SZ, long long n, int rows,
+                                                              double* __restrict__ red) {
     constexpr int KK = kCoarse * kCoarse;
-    __shared__ double wsum[kVT / 32][KK];
-    const long long i = static_cast<long long>(blockIdx.x) * kVT + threadIdx.x;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double zv[kCoarse], sv[kCoarse];
-#pragma unroll
-    for (int j = 0; j < kCoarse; ++j) {
-        zv[j] = i < n ? Zc[j * n + i] : 0.0;
-        sv[j] = i < n ? SZ[j * n + i] : 0.0;
-    }
-#pragma unroll
-    for (int a = 0; a < kCoarse; ++a)
-#pragma unroll
-        for (int b = 0; b < kCoarse; ++b) {
-            const double t = warp_sum(zv[a] * sv[b]);
-            if (lane == 0) wsum[warp][a * kCoarse + b] = t;
+    __shared__ double zs[kCoarse][kGramRows], ss[kCoarse][kGramRows], sum[3][KK];
+    const long long i0 = static_cast<long long>(blockIdx.x) * rows, i1 = min(i0 + rows, n);
+    const int g = threadIdx.x / KK, t = threadIdx.x - KK * g, a = t / kCoarse, b = t - kCoarse * a;
+    double acc = 0.0;
+    for (long long base = i0; base < i1; base += kGramRows) {
+        const int m = static_cast<int>(min(static_cast<long long>(kGramRows), i1 - base));
+        for (int k = threadIdx.x; k < kCoarse * kGramRows; k += kGramT) {
+            const int j = k / kGramRows, r = k % kGramRows;
+            zs[j][r] = r < m ? Zc[j * n + base + r] : 0.0;
+            ss[j][r] = r < m ? SZ[j * n + base + r] : 0.0;
         }
-    __syncthreads();
-    if (threadIdx.x < KK) {
-        double v = 0.0;
-#pragma unroll
-        for (int w = 0; w < kVT / 32; ++w) v += wsum[w][threadIdx.x];
-        red[static_cast<long long>(blockIdx.x) * KK + threadIdx.x] = v;
+        __syncthreads();
+        for (int r = g; r < m; r += 3) acc += zs[a][r] * ss[b][r];
+        __syncthreads();
     }
+    sum[g][t] = acc;
+    __syncthreads();
+    if (g == 0) red[static_cast<long long>(blockIdx.x) * KK + t] = sum[0][t] + sum[1][t] + sum[2][t];
+}
+// Rows per block: 64, or what makes one block per SM.
+static int gram_rows(long long n) {
+    return std::max(kGramRows, kGramRows * ceil_div(static_cast<int>(ceil_div(n, device_sm_count())), kGramRows));
 }
 
-// E from the partials (fixed order), symmetrised; FP64 Cholesky and inverse by
-// one thread. einv[kCoarse^2] = 1 if E is SPD (relative pivot floor 1e-13), else 0.
-constexpr int kEinvT = 1024;
+// E from the partials (fixed order), symmetrised; its FP64 inverse by Gauss-Jordan
+// steps without exchanges (E is SPD, or flagged), one thread per entry.
+// einv[kCoarse^2] = 1 if E is SPD (relative pivot floor 1e-13, the pivots of its
+// Cholesky factor), else 0. One CTA, bound by its FP64 chain: 46 -> 10 us at 257
+// cameras against one thread's factorisation and a thread per column.
+constexpr int kEinvG = 12;  // groups of partials
+constexpr int kEinvT = kEinvG * kCoarse * kCoarse;
 __global__ void __launch_bounds__(kEinvT) coarse_einv_kernel(const double* __restrict__ red, int nb,
                                                             double* __restrict__ einv) {
     constexpr int K = kCoarse, KK = kCoarse * kCoarse;
-    __shared__ double E[KK], L[KK];
-    __shared__ int ok;
-    // entry t of E: one warp sums the nb block partials (lanes strided, then a shuffle tree)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int t = warp; t < KK; t += kEinvT / 32) {
-        double v = 0.0;
-        for (int b = lane; b < nb; b += 32) v += red[static_cast<long long>(b) * KK + t];
-        v = warp_sum(v);
-        if (lane == 0) E[t] = v;
+    __shared__ double part[kEinvG][KK], M[KK], dmax;
+    const int g = threadIdx.x / KK, t = threadIdx.x - KK * g, a = t / K, b = t - K * a;
+    double v = 0.0;
+#pragma unroll 4
+    for (int k = g; k < nb; k += kEinvG) v += red[static_cast<long long>(k) * KK + t];
+    part[g][t] = v;
+    __syncthreads();
+    const bool own = g == 0;
+    if (own) {
+        v = 0.0;
+#pragma unroll
+        for (int k = 0; k < kEinvG; ++k) v += part[k][t];
+        part[0][t] = v;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {  // Cholesky of the symmetrised E (9 x 9)
-        double dmax = 0.0;
-        for (int a = 0; a < K; ++a)
-            for (int b = 0; b < K; ++b) L[a * K + b] = 0.5 * (E[a * K + b] + E[b * K + a]);
-        for (int a = 0; a < K; ++a) dmax = fmax(dmax, L[a * K + a]);
-        bool good = dmax > 0.0 && isfinite(dmax);
-        for (int k = 0; k < K && good; ++k) {
-            double d = L[k * K + k];
-            for (int m = 0; m < k; ++m) d -= L[k * K + m] * L[k * K + m];
-            if (!(d > 1e-13 * dmax)) {
-                good = false;
-                break;
-            }
-            const double l = sqrt(d);
-            L[k * K + k] = l;
-            for (int a = k + 1; a < K; ++a) {
-                double v = L[a * K + k];
-                for (int m = 0; m < k; ++m) v -= L[a * K + m] * L[k * K + m];
-                L[a * K + k] = v / l;
-            }
-        }
-        ok = good;
+    if (own) M[t] = v = 0.5 * (v + part[0][K * b + a]);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double d = 0.0;
+        for (int k = 0; k < K; ++k) d = fmax(d, M[k * K + k]);
+        dmax = d;
     }
     __syncthreads();
-    if (!ok) {
-        for (int t = threadIdx.x; t <= KK; t += kEinvT) einv[t] = 0.0;
-        return;
-    }
-    // E^-1 = L^-T L^-1, one column of the identity per thread
-    if (threadIdx.x < K) {
-        const int col = threadIdx.x;
-        double y[K];
-#pragma unroll
-        for (int a = 0; a < K; ++a) {
-            double v = a == col ? 1.0 : 0.0;
-            for (int m = 0; m < a; ++m) v -= L[a * K + m] * y[m];
-            y[a] = v / L[a * K + a];
+    bool good = dmax > 0.0 && isfinite(dmax);
+    const double floor_ = 1e-13 * dmax;
+    for (int k = 0; k < K && good; ++k) {  // good: the same in every thread
+        const double d = M[k * K + k];
+        good = d > floor_;
+        if (own && good) {
+            const double r = 1.0 / d, mk = M[K * a + k], kb = M[K * k + b];
+            if (a == k)
+                v = b == k ? r : kb * r;
+            else
+                v = b == k ? -mk * r : v - mk * r * kb;
         }
-#pragma unroll
-        for (int a = K - 1; a >= 0; --a) {
-            double v = y[a];
-            for (int m = a + 1; m < K; ++m) v -= L[m * K + a] * y[m];
-            y[a] = v / L[a * K + a];
-        }
-#pragma unroll
-        for (int a = 0; a < K; ++a) einv[a * K + col] = y[a];
+        __syncthreads();
+        if (own && good) M[t] = v;
+        __syncthreads();
     }
-    if (threadIdx.x == 0) einv[KK] = 1.0;
+    if (own) einv[t] = good ? v : 0.0;
+    if (threadIdx.x == 0) einv[KK] = good ? 1.0 : 0.0;
 }
 
 // Block partials of a . b, a FP64 and b FP32 (b . x of the inner solution).
@@ -2006,7 +1998,9 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
         for (int j = 0; j < 9; ++j) d[j] = src[j * stride];
     };
     auto p_at = [&](int i) { return p32 + static_cast<long long>(kX32) * (c0 + i / 9) + i % 9; };
-    // the rows do not change during a solve's iterations
+    // What the wait is for is q: the rows do not change during a solve's iterations,
+    // and x, r, p and the scalars are this kernel's own from the iteration before,
+    // for which the product has waited before it let its successors start.
     float mrow[9], sz[kCoarse], zc[kCoarse], xv = 0.f, rv = 0.f, pv = 0.f, qv = 0.f;
     if (kOne) {
 #pragma unroll
@@ -2017,7 +2011,17 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
                 load9(zc, Zc + i0 + first, n);
                 load9(sz, SZ + i0 + first, n);
             }
+            pv = *p_at(first);
+            xv = x[i0 + first];
+            rv = r[i0 + first];
         }
+    }
+    const bool over = flag_set(sc + S_DONE);
+    double rz_old = 0.0, tol2bb = 0.0, iters = 0.0, alpha = 0.0, rr = 0.0;  // thread 0
+    if (tid == 0) {
+        rz_old = sc[S_RZ];
+        tol2bb = sc[S_TOL2] * sc[S_BB];
+        iters = sc[S_ITERS] + 1.0;
     }
     double e[3] = {0.0, 0.0, 0.0};
     if (kZ && (warp == 2 || warp == 3)) {
@@ -2031,25 +2035,15 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
     pdl_wait();
     pdl_trigger();
     cluster_wait();  // every CTA of the cluster runs
-    if (flag_set(sc + S_DONE)) return;
-    double rz_old = 0.0, tol2bb = 0.0, iters = 0.0, alpha = 0.0, rr = 0.0;  // thread 0
-    if (tid == 0) {
-        rz_old = sc[S_RZ];
-        tol2bb = sc[S_TOL2] * sc[S_BB];
-        iters = sc[S_ITERS] + 1.0;
-    }
+    if (over) return;
 
     float v[10];
 #pragma unroll
     for (int j = 0; j < 10; ++j) v[j] = 0.f;
     for (int i = first; i < rows; i += step) {
-        pv = *p_at(i);
+        if (!kOne) pv = *p_at(i);
         qv = q[i0 + i];
         v[0] = fmaf(pv, qv, v[0]);
-        if (kOne) {
-            xv = x[i0 + i];
-            rv = r[i0 + i];
-        }
     }
     cluster_totals<1, false>(v, sm, 0, rank, nctas, [&](double pq, double) {
         const bool ok = pq > 0.0 && isfinite(pq);
@@ -2869,7 +2863,7 @@ void Solver::coarse_prepare(double lambda) {
     const int n = 9 * C_;
     const int nvb = ceil_div(n, kVT);
     const int nub = ceil_div(C_, kUC);
-    const size_t need_red = 2ull * nub * kCoarse + kCoarse + 1ull * nvb * kCoarse * kCoarse;
+    const size_t need_red = 2ull * nub * kCoarse + kCoarse + 1ull * ceil_div(n, gram_rows(n)) * kCoarse * kCoarse;
     if (!cz_.get()) {
         StreamAllocScope scope(stream_);
         cz_.alloc(1ull * kCoarse * n);
@@ -2922,9 +2916,10 @@ void Solver::coarse_prepare(double lambda) {
                                                                       csz32_.get());
     GBA_LAUNCH_CHECK();
     double* gram = cred_.get() + 2ll * nub * kCoarse + kCoarse;
-    coarse_gram_partials<<<nvb, kVT, 0, stream_>>>(cz_.get(), csz_.get(), n, gram);
+    const int rows = gram_rows(n), ngram = ceil_div(n, rows);
+    coarse_gram_partials<<<ngram, kGramT, 0, stream_>>>(cz_.get(), csz_.get(), n, rows, gram);
     GBA_LAUNCH_CHECK();
-    coarse_einv_kernel<<<1, kEinvT, 0, stream_>>>(gram, nvb, ceinv_.get());
+    coarse_einv_kernel<<<1, kEinvT, 0, stream_>>>(gram, ngram, ceinv_.get());
     GBA_LAUNCH_CHECK();
     prof_stop("coarse_gram", ev1);
     prof_stop("coarse_prepare", ev);
