@@ -515,11 +515,14 @@ constexpr int kSolT = 256;
 constexpr int kSolRows = 16;  // rows (columns) of L per pass of a block
 
 // Forward step j: y_j = L_jj^-1 b_j, b[j0 + 64 : r_end) -= L[.., j] y_j.
-__global__ void __launch_bounds__(kSolT) forward_step(const double* __restrict__ L, int j0, int r_end, int lda,
+// blockIdx.y = 1: the second chain's tile, dj rows further on.
+__global__ void __launch_bounds__(kSolT) forward_step(const double* __restrict__ L, int j0, int r_end, int dj, int lda,
                                                      const double* __restrict__ inv, double* __restrict__ b,
                                                      double* __restrict__ y, const int* __restrict__ info) {
     __shared__ double part[4][NB], bs[NB], x[NB], red[kSolRows][kSolT / kSolRows + 1];
     const int lr = threadIdx.x & (kSolRows - 1), kg = threadIdx.x / kSolRows;  // row, group of four columns
+    j0 += blockIdx.y * dj;
+    r_end += blockIdx.y * dj;
     double m[16], l[4] = {0.0, 0.0, 0.0, 0.0};
     load_tile_cols<true>(inv + static_cast<long long>(j0) * NB, m);
     int r = j0 + NB + blockIdx.x * kSolRows + lr;
@@ -552,37 +555,70 @@ __global__ void __launch_bounds__(kSolT) forward_step(const double* __restrict__
     }
 }
 
-// Backward step j: x_j = L_jj^-T y_j (into b), y[i0 : j0) -= L[j, ..]^T x_j.
-__global__ void __launch_bounds__(kSolT) backward_step(const double* __restrict__ L, int i0, int j0, int lda,
-                                                      const double* __restrict__ invt, double* __restrict__ y,
+// Backward step j: x_j = L_jj^-T y_j (into b), y[i0 : i1) -= L[j, ..]^T x_j.
+// known >= 0: x_j is there already, as b[known], b[known - 1], ...
+struct BackwardTile {
+    int j0, i0, i1, known;
+};
+__global__ void __launch_bounds__(kSolT) backward_step(const double* __restrict__ L, BackwardTile t0, BackwardTile t1,
+                                                      int lda, const double* __restrict__ invt, double* __restrict__ y,
                                                       double* __restrict__ b, const int* __restrict__ info) {
     __shared__ double part[4][NB], bs[NB], x[NB];
     const int kg = threadIdx.x & 15, lc = threadIdx.x >> 4;  // group of four rows, column
+    const BackwardTile t = blockIdx.y ? t1 : t0;
+    const int j0 = t.j0;
     double m[16], l[4] = {0.0, 0.0, 0.0, 0.0};
-    load_tile_cols<false>(invt + static_cast<long long>(j0) * NB, m);
-    int c = i0 + blockIdx.x * kSolRows + lc;
-    if (c < j0) {
+    if (t.known < 0) load_tile_cols<false>(invt + static_cast<long long>(j0) * NB, m);
+    int c = t.i0 + blockIdx.x * kSolRows + lc;
+    if (c < t.i1) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) l[i] = L[j0 + 4 * kg + i + static_cast<long long>(c) * lda];
     }
     pdl_wait();
     pdl_trigger();
     if (*info) return;
-    if (threadIdx.x < NB) bs[threadIdx.x] = y[j0 + threadIdx.x];
-    __syncthreads();
-    tile_product<false>(m, bs, part, x);
-    if (blockIdx.x == 0 && threadIdx.x < NB) b[j0 + threadIdx.x] = x[threadIdx.x];
-    for (; c - lc < j0; c += gridDim.x * kSolRows) {
+    if (t.known >= 0) {
+        if (threadIdx.x < NB) x[threadIdx.x] = b[t.known - threadIdx.x];
+        __syncthreads();
+    } else {
+        if (threadIdx.x < NB) bs[threadIdx.x] = y[j0 + threadIdx.x];
+        __syncthreads();
+        tile_product<false>(m, bs, part, x);
+        if (blockIdx.x == 0 && threadIdx.x < NB) b[j0 + threadIdx.x] = x[threadIdx.x];
+    }
+    for (; c - lc < t.i1; c += gridDim.x * kSolRows) {
         double v = fma(l[0], x[4 * kg], l[1] * x[4 * kg + 1]) + fma(l[2], x[4 * kg + 2], l[3] * x[4 * kg + 3]);
         const int nc = c + gridDim.x * kSolRows;
-        if (nc < j0) {
+        if (nc < t.i1) {
 #pragma unroll
             for (int i = 0; i < 4; ++i) l[i] = L[j0 + 4 * kg + i + static_cast<long long>(nc) * lda];
         }
 #pragma unroll
         for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o, 16);
-        if (kg == 0 && c < j0) y[c] -= v;
+        if (kg == 0 && c < t.i1) y[c] -= v;
     }
+}
+
+// The right-hand side of the two chains of band_potrf_twisted, and the solution back
+// in the band's order. base: the second chain's first row, its last s rows copies.
+__global__ void twist_rhs(const double* __restrict__ b, int n, int base, int s, double* __restrict__ bt) {
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n + s) bt[i] = i < base ? b[i] : i < n ? b[n - 1 - (i - base)] : 0.0;
+}
+__global__ void twist_merge_rhs(int n, int base, int s, double* __restrict__ bt) {
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;  // row base - s + i of the band
+    if (i < s) bt[base - s + i] += bt[n + s - 1 - i];
+}
+__global__ void twist_solution(const double* __restrict__ bt, int n, int base, const int* __restrict__ info,
+                               double* __restrict__ b) {
+    pdl_wait();
+    pdl_trigger();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n && *info == 0) b[i] = bt[i < base ? i : base + n - 1 - i];
 }
 
 }  // namespace
@@ -620,6 +656,18 @@ static void dense_potrf_fp64(double* A, int n, int lda, int* info, cudaStream_t 
 
 size_t dense_potrs_workspace(int n) { return (2ull * NB + 1) * n * sizeof(double); }
 
+static void invert_tiles(const double* L, int nt, int lda, double* inv, double* invt, const int* info, cudaStream_t s) {
+    const int xsm = NB * (NB + 1) * sizeof(double);
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(tile_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, xsm));
+    launch_pdl(tile_inverse, nt, kInvT, xsm, s, L, lda, inv, invt, info);
+}
+// Blocks of a step over `rows` rows (columns) of each chain. Two passes of a block at
+// most where the rows allow it: a further pass costs a block less than a further block
+// costs the launch.
+static dim3 step_grid(int rows, int chains) {
+    return dim3(std::max(1, std::min(2 * device_sm_count(), ceil_div(rows, kSolRows))), chains);
+}
+
 void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* info, void* workspace,
                  cudaStream_t s) {
     if (n % NB != 0 || bt < 0 || (bt < n / NB - 1 ? lda + 1 < (bt + 2) * NB : lda < n))
@@ -628,23 +676,63 @@ void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* 
     double* inv = static_cast<double*>(workspace);
     double* invt = inv + static_cast<size_t>(NB) * n;
     double* y = invt + static_cast<size_t>(NB) * n;
-    const int xsm = NB * (NB + 1) * sizeof(double);
-    GBA_CUDA_CHECK(cudaFuncSetAttribute(tile_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, xsm));
-    launch_pdl(tile_inverse, nt, kInvT, xsm, s, L, lda, inv, invt, info);
-    // Two passes of a block at most where the rows allow it: a further pass costs
-    // a block less than a further block costs the launch.
-    const int most = 2 * device_sm_count();
+    invert_tiles(L, nt, lda, inv, invt, info, s);
     for (int jb = 0; jb < nt; ++jb) {
         const int j0 = jb * NB;
         const int r_end = static_cast<int>(std::min<long long>(n, j0 + NB + (long long)bt * NB));
-        const int grid = std::max(1, std::min(most, ceil_div(r_end - j0 - NB, kSolRows)));
-        launch_pdl(forward_step, grid, kSolT, 0, s, L, j0, r_end, lda, inv, b, y, info);
+        launch_pdl(forward_step, step_grid(r_end - j0 - NB, 1), kSolT, 0, s, L, j0, r_end, 0, lda, inv, b, y, info);
     }
     for (int jb = nt - 1; jb >= 0; --jb) {
         const int j0 = jb * NB, i0 = std::max(0, j0 - bt * NB);
-        const int grid = std::max(1, std::min(most, ceil_div(j0 - i0, kSolRows)));
-        launch_pdl(backward_step, grid, kSolT, 0, s, L, i0, j0, lda, invt, y, b, info);
+        const BackwardTile t{j0, i0, j0, -1};
+        launch_pdl(backward_step, step_grid(j0 - i0, 1), kSolT, 0, s, L, t, t, lda, invt, y, b, info);
     }
+}
+
+size_t band_twist_solve_workspace(int n, int bt) {
+    return dense_potrs_workspace(n + NB * bt) + sizeof(double) * (n + static_cast<size_t>(NB) * bt);
+}
+
+void band_potrs_twisted(const double* F, int n, int lda, int bt, int ta, double* b, const int* info, void* workspace,
+                        cudaStream_t s) {
+    const int np = n + bt * NB, sep = bt * NB, a = ta * NB, base = a + sep, tb = n / NB - ta - bt;
+    double* inv = static_cast<double*>(workspace);
+    double* invt = inv + static_cast<size_t>(NB) * np;
+    double* y = invt + static_cast<size_t>(NB) * np;
+    double* x = y + np;
+    launch_pdl(twist_rhs, ceil_div(np, 256), 256, 0, s, b, n, base, sep, x);
+    invert_tiles(F, n / NB, lda, inv, invt, info, s);  // not those of the copies
+    for (int k = 0; k < std::max(ta, tb); ++k) {
+        const int chains = k < ta && k < tb ? 2 : 1, j0 = k * NB + (k < ta ? 0 : base);
+        launch_pdl(forward_step, step_grid(sep, chains), kSolT, 0, s, F, j0, j0 + NB + sep, base, lda, inv, x, y, info);
+    }
+    launch_pdl(twist_merge_rhs, ceil_div(sep, 256), 256, 0, s, n, base, sep, x);
+    for (int k = 0; k < bt; ++k) {
+        const int j0 = a + k * NB;
+        launch_pdl(forward_step, step_grid(base - j0 - NB, 1), kSolT, 0, s, F, j0, base, 0, lda, inv, x, y, info);
+    }
+    auto columns = [&](int j0, int first) { return std::max(first, j0 - sep); };
+    for (int k = bt - 1; k >= 0; --k) {
+        const int j0 = a + k * NB, i0 = columns(j0, 0);
+        const BackwardTile t{j0, i0, j0, -1};
+        launch_pdl(backward_step, step_grid(j0 - i0, 1), kSolT, 0, s, F, t, t, lda, invt, y, x, info);
+    }
+    // chain 0's tiles above, beside chain 1's: the rows between (known now), then its own
+    for (int k = 0; k < std::max(ta, tb + bt); ++k) {
+        BackwardTile t[2];
+        int m = 0;
+        if (k < ta) {
+            const int j0 = a - (k + 1) * NB;
+            t[m++] = {j0, columns(j0, 0), j0, -1};
+        }
+        if (k < tb + bt) {
+            const int j0 = np - (k + 1) * NB;
+            // row j0 + i of chain 1 is row base + n - 1 - j0 - i of the band
+            t[m++] = {j0, columns(j0, base), std::min(j0, n), k < bt ? base + n - 1 - j0 : -1};
+        }
+        launch_pdl(backward_step, step_grid(sep, m), kSolT, 0, s, F, t[0], t[m - 1], lda, invt, y, x, info);
+    }
+    launch_pdl(twist_solution, ceil_div(n, 256), 256, 0, s, x, n, base, info, b);
 }
 
 void Solver::ensure_schur_storage() {
@@ -661,7 +749,20 @@ void Solver::ensure_schur_storage() {
     band_mode_ = band;
     S_.release();
     S_.alloc(static_cast<size_t>(n_pad_) * (band ? band_ldb_ : n_pad_));
-    if (!chol_ws_.get()) chol_ws_.alloc(std::max(dense_potrf_workspace(n_pad_), dense_potrs_workspace(n_pad_)));
+    // A band that pays is factored from both ends (an explicitly chosen one leaves its
+    // factor in S): 3 (bt + 2) <= nt, so at least bt + 3 of the nt panels run beside others.
+    const int nt = n_pad_ / NB;
+    twist_ta_ = band && want == 0 ? (nt - band_bt_ + 1) / 2 : 0;
+    twist_.release();
+    size_t ws = std::max(dense_potrf_workspace(n_pad_), dense_potrs_workspace(n_pad_));
+    if (twist_ta_) {
+        twist_.alloc(static_cast<size_t>(n_pad_ + NB * band_bt_) * band_ldb_);
+        ws = std::max(ws, std::max(band_twist_workspace(n_pad_, band_bt_), band_twist_solve_workspace(n_pad_, band_bt_)));
+    }
+    if (chol_ws_.size() < ws) {
+        chol_ws_.release();
+        chol_ws_.alloc(ws);
+    }
     schur_layout_planned_ = want;
 }
 
@@ -716,13 +817,15 @@ int Solver::schur_dense(double lambda) {
     cudaEvent_t ev = prof_start();
     if (schur_layout_ == 1)
         dense_potrf_fp64(S_.get(), n_pad_, lda, info_.get(), stream_);
+    else if (twist_ta_)
+        band_potrf_twisted(S_.get(), n_pad_, lda, bt, twist_ta_, twist_.get(), info_.get(), chol_ws_.get(), stream_);
     else
         dense_potrf(S_.get(), n_pad_, lda, bt, info_.get(), chol_ws_.get(), stream_);
     prof_stop("dense_potrf", ev);
     int info = 0;
     read_back({{&info, info_.get(), sizeof info}});
     if (info < 0) throw std::runtime_error("dense_potrf: a wait of the trailing update ran out");
-    if (info != 0) return info;
+    if (info != 0) return twist_ta_ ? band_twist_row(info - 1, n_pad_, bt, twist_ta_) + 1 : info;
     // solve in a copy so rhs stays the assembled right-hand side (in the band
     // layout the copy is in the renumbered camera order; the padding stays 0)
     if (band_mode_) {
@@ -733,7 +836,10 @@ int Solver::schur_dense(double lambda) {
         GBA_CUDA_CHECK(cudaMemcpyAsync(pcg_x_.get(), rhs_.get(), n_pad_ * sizeof(double), cudaMemcpyDeviceToDevice,
                                        stream_));
     }
-    dense_potrs(S_.get(), n_pad_, lda, bt, pcg_x_.get(), info_.get(), chol_ws_.get(), stream_);
+    if (twist_ta_)
+        band_potrs_twisted(twist_.get(), n_pad_, lda, bt, twist_ta_, pcg_x_.get(), info_.get(), chol_ws_.get(), stream_);
+    else
+        dense_potrs(S_.get(), n_pad_, lda, bt, pcg_x_.get(), info_.get(), chol_ws_.get(), stream_);
     if (band_mode_) {
         permute_cameras<<<ceil_div(9 * C_, 256), 256, 0, stream_>>>(perm, C_, false, pcg_x_.get(), dc_.get());
         GBA_LAUNCH_CHECK();

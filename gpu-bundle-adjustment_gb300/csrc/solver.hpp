@@ -335,6 +335,8 @@ public:
     bool band_beneficial_ = false;
     int band_ldb_ = 0, band_bt_ = 0;
     DevBuf<int> cam_perm_;
+    int twist_ta_ = 0;         // > 0: the band is factored from both ends, this many tiles from the top
+    DevBuf<double> twist_;     // the two chains' factor (S_ keeps the assembled band then)
     void set_schur_layout(int layout) { schur_layout_ = layout; }
     void plan_schur_band();       // structure.cu: ordering and band size from the block list
     void ensure_schur_storage();  // dense.cu: allocates S for the chosen layout
@@ -385,6 +387,16 @@ void dense_potrf(double* A, int n, int lda, int bt, int* info, void* workspace, 
 // (nothing is done where *info != 0). workspace: dense_potrs_workspace(n) bytes of
 // device memory, the call's own until the stream has passed it.
 size_t dense_potrs_workspace(int n);
+// The same for a band S from both ends (chol.cu): ta tiles from the top, the bt tiles
+// after them last; S stays, F ((n + 64 bt) columns of lda + 1) holds the factor.
+// band_twist_row: the band row of a row of F (*info counts F's).
+size_t band_twist_workspace(int n, int bt);
+size_t band_twist_solve_workspace(int n, int bt);
+int band_twist_row(int i, int n, int bt, int ta);
+void band_potrf_twisted(const double* S, int n, int lda, int bt, int ta, double* F, int* info, void* workspace,
+                        cudaStream_t s);
+void band_potrs_twisted(const double* F, int n, int lda, int bt, int ta, double* b, const int* info, void* workspace,
+                        cudaStream_t s);
 void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* info, void* workspace,
                  cudaStream_t s);
 // Residual + Jacobian for E independent observations (device pointers, original
