@@ -754,8 +754,6 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
             const bool in = rloc < 64 * nt;
             long long* p = F + (j1 + rloc) + static_cast<long long>(j1 + cloc) * lda;
             long long c[16];
-#pragma unroll
-            for (int k = 0; k < 16; ++k) c[k] = in && rloc >= cloc + k ? p[static_cast<long long>(k) * lda] : 0;
             if (!mbar_wait(bar(B_LOFULL), i & 1, &gave_up)) break;
             tc_fence_after();
 #pragma unroll
@@ -767,8 +765,8 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
                 tmem_wait_load();
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    c[k0 + k] -= static_cast<long long>(__float2int_rn(g4[k])) * 256 +
-                                 __float2int_rn(0.5f * fmaf(g6[k], 0x1p-9f, g5[k]));
+                    c[k0 + k] = static_cast<long long>(__float2int_rn(g4[k])) * 256 +
+                                __float2int_rn(0.5f * fmaf(g6[k], 0x1p-9f, g5[k]));
             }
             tc_fence_before();
             __syncwarp();
@@ -786,7 +784,7 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
                     const int top = small_int(g0[k]) * 512 + small_int(g1[k]);  // 2^35
-                    c[k0 + k] -= (static_cast<long long>(top) << 35) +
+                    c[k0 + k] += (static_cast<long long>(top) << 35) +
                                  static_cast<long long>(__float2int_rn(g2[k])) * (1 << 26) +
                                  static_cast<long long>(__float2int_rn(g3[k])) * (1 << 17);
                 }
@@ -794,10 +792,12 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(B_HIEMPTY));
-            asm volatile("" : "+l"(p));  // the sixteen addresses are formed again, not held across the recombination
+            // subtracted at L2: the entries are not waited for
 #pragma unroll
             for (int k = 0; k < 16; ++k)
-                if (in && rloc >= cloc + k) p[static_cast<long long>(k) * lda] = c[k];
+                if (in && rloc >= cloc + k)
+                    atomicAdd(reinterpret_cast<unsigned long long*>(p + static_cast<long long>(k) * lda),
+                              static_cast<unsigned long long>(-c[k]));
         }
     }
     __syncwarp();

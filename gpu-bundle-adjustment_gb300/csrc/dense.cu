@@ -444,44 +444,38 @@ __global__ void __launch_bounds__(256) syrk_update_quad_kernel(double* __restric
 // product at 1.7 FMA per cycle, and the update; the operands (constant during the
 // solve) are loaded before the previous step has ended.
 
-// L_jj^-1 of every tile, column-major (inv) and transposed (invt): rows of X
-// in order, X_k = (e_k - sum_m L_km X_m) / L_kk, as rank-1 updates of the rows below.
-constexpr int kInvT = 256;
+// L_jj^-1 of every tile, column-major (inv) and transposed (invt): kInvCols columns
+// of X per block, X_k = (e_k - sum_m L_km X_m) / L_kk as rank-1 updates of the rows
+// below, one entry per thread. Bound by the 64 dependent steps (a product, a barrier
+// and the update, whose FP64 instructions the warps of a sub-partition take in
+// turn): one tile per block with its rows and columns in turn took 60 us, 12 us so.
+constexpr int kInvCols = 8;
+constexpr int kInvT = NB * kInvCols;
 __global__ void __launch_bounds__(kInvT) tile_inverse(const double* __restrict__ L, int lda, double* __restrict__ inv,
                                                      double* __restrict__ invt, const int* __restrict__ info) {
-    __shared__ double t[NB][NB + 1];  // t[col][row] of L
-    extern __shared__ double xs[];    // X, row-major, stride NB + 1
-    __shared__ double rinv[NB];
+    extern __shared__ double t[];         // t[column NB + row] of L
+    __shared__ double x[NB][kInvCols], rinv[NB];
     pdl_wait();  // no early trigger: the first step reads the inverses before its own wait
     if (*info) return;
     const long long j0 = static_cast<long long>(blockIdx.x) * NB;
-    for (int i = threadIdx.x; i < NB * NB; i += kInvT) {
-        const int r = i & 63, c = i >> 6;
-        const double v = r >= c ? L[(j0 + r) + (j0 + c) * lda] : 0.0;
-        t[c][r] = v;
-        if (r == c) rinv[r] = 1.0 / v;
-        xs[r * (NB + 1) + c] = r == c ? 1.0 : 0.0;
-    }
+    const int r = threadIdx.x & 63, cl = threadIdx.x >> 6, first = blockIdx.y * kInvCols, c = first + cl;
+    for (int k = first + cl; k < NB; k += kInvCols) t[NB * k + r] = r >= k ? L[(j0 + r) + (j0 + k) * lda] : 0.0;
+    if (cl == 0 && r >= first) rinv[r] = 1.0 / L[(j0 + r) + (j0 + r) * lda];
     __syncthreads();
-    for (int k = 0; k < NB; ++k) {
-        // row k is complete but for its pivot: columns 0 .. k
-        if (threadIdx.x <= k) xs[k * (NB + 1) + threadIdx.x] *= rinv[k];
+    double v = r == c ? 1.0 : 0.0;
+    for (int k = first; k < NB; ++k) {  // (columns right of k: zeros)
+        if (r == k) x[k][cl] = v = v * rinv[k];
         __syncthreads();
-        // rows below, columns 0 .. k: a warp takes a row and 32 columns
-        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, halves = (k >> 5) + 1;
-        for (int w = warp; w < (NB - 1 - k) * halves; w += kInvT / 32) {
-            const int r = k + 1 + w / halves, c = 32 * (w % halves) + lane;
-            if (c <= k) xs[r * (NB + 1) + c] -= t[k][r] * xs[k * (NB + 1) + c];
-        }
-        __syncthreads();
+        if ((r | 31) > k && r > k) v -= t[NB * k + r] * x[k][cl];
     }
-    double* o = inv + j0 * NB;
-    double* ot = invt + j0 * NB;
-    for (int i = threadIdx.x; i < NB * NB; i += kInvT) {
-        const int r = i & 63, c = i >> 6;
-        o[i] = xs[r * (NB + 1) + c];
-        ot[i] = xs[c * (NB + 1) + r];
-    }
+    if (r < first) v = 0.0;
+    inv[j0 * NB + NB * c + r] = v;
+    __syncthreads();
+    // transposed: row c of invt's tile is column c of the inverse
+    x[r][cl] = v;
+    __syncthreads();
+    const int cc = threadIdx.x & (kInvCols - 1), rr = threadIdx.x / kInvCols;
+    invt[j0 * NB + NB * rr + first + cc] = x[rr][cc];
 }
 
 // x = M b for a 64 x 64 tile M (column-major, 0 outside the triangle): 256
@@ -657,9 +651,7 @@ static void dense_potrf_fp64(double* A, int n, int lda, int* info, cudaStream_t 
 size_t dense_potrs_workspace(int n) { return (2ull * NB + 1) * n * sizeof(double); }
 
 static void invert_tiles(const double* L, int nt, int lda, double* inv, double* invt, const int* info, cudaStream_t s) {
-    const int xsm = NB * (NB + 1) * sizeof(double);
-    GBA_CUDA_CHECK(cudaFuncSetAttribute(tile_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, xsm));
-    launch_pdl(tile_inverse, nt, kInvT, xsm, s, L, lda, inv, invt, info);
+    launch_pdl(tile_inverse, dim3(nt, NB / kInvCols), kInvT, NB * NB * sizeof(double), s, L, lda, inv, invt, info);
 }
 // Blocks of a step over `rows` rows (columns) of each chain. Two passes of a block at
 // most where the rows allow it: a further pass costs a block less than a further block
