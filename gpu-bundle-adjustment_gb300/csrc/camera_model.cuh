@@ -113,36 +113,20 @@ GBA_HD void residual(const double* cam, const double* X, const double* obs, doub
     r[1] = fd * v - obs[1];
 }
 
-// Residual + analytic Jacobian. Jc: 2x9 row-major (a[3], t[3], f, k1, k2);
-// Jp: 2x3 row-major.
-GBA_HD void residual_jacobian(const double* cam, const double* X, const double* obs, double* r, double* Jc, double* Jp) {
-    const double* a = cam;
-    const double t = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
-    const bool first_order = !(t > 1e-24);
-    // the branch's R = I + [a]x for the point, J_l = I, dX_c/dX = I and dRX/da = -[X]x
-    double A = 1.0, B = 0.0, C = 0.0, c = 1.0;
-    if (!first_order) rotation_terms(t, A, B, C, c);
-    const double A0 = A * a[0], A1 = A * a[1], A2 = A * a[2];
-    const double B0 = B * a[0], B1 = B * a[1], B2 = B * a[2];
-    const double C0 = C * a[0], C1 = C * a[1], C2 = C * a[2];
-    const double R[9] = {c + B0 * a[0],  B0 * a[1] - A2, B0 * a[2] + A1,
-                    B1 * a[0] + A2, c + B1 * a[1],  B1 * a[2] - A0,
-                    B2 * a[0] - A1, B2 * a[1] + A0, c + B2 * a[2]};
-    const double Jl[9] = {A + C0 * a[0],  C0 * a[1] - B2, C0 * a[2] + B1,
-                     C1 * a[0] + B2, A + C1 * a[1],  C1 * a[2] - B0,
-                     C2 * a[0] - B1, C2 * a[1] + B0, A + C2 * a[2]};
-    double RX[3];
-    for (int i = 0; i < 3; ++i) RX[i] = R[3 * i] * X[0] + R[3 * i + 1] * X[1] + R[3 * i + 2] * X[2];
-    const double iz = 1.0 / (RX[2] + cam[5]);
-    const double u = -(RX[0] + cam[3]) * iz, v = -(RX[1] + cam[4]) * iz;
+// Residual and Jacobian rows from the rotation R, its left Jacobian J_l, R X and
+// tf = (t, f, k1, k2).
+GBA_HD void jacobian_rows(const double* R, const double* Jl, const double* RX, bool first_order, const double* tf,
+                          const double* X, const double* obs, double* r, double* Jc, double* Jp) {
+    const double iz = 1.0 / (RX[2] + tf[2]);
+    const double u = -(RX[0] + tf[0]) * iz, v = -(RX[1] + tf[1]) * iz;
     const double r2 = u * u + v * v;
-    const double f = cam[6], k1 = cam[7], k2r2 = cam[8] * r2;
+    const double f = tf[3], k1 = tf[4], k2r2 = tf[5] * r2;
     const double d = 1.0 + r2 * (k1 + k2r2);
     const double fd = f * d;
     r[0] = fd * u - obs[0];
     r[1] = fd * v - obs[1];
 
-    // D = f (d I + 2 L [u v]^double [u v]), L = k1 + 2 k2 r2, and
+    // D = f (d I + 2 L [u v]^T [u v]), L = k1 + 2 k2 r2, and
     // M = d(u,v)/dX_c = [[-iz, 0, -u iz], [0, -iz, -v iz]]; g = rows of D M
     const double fL2 = 2.0 * f * (k1 + 2.0 * k2r2);
     const double fu = fL2 * u;
@@ -172,6 +156,29 @@ GBA_HD void residual_jacobian(const double* cam, const double* X, const double* 
         Jc[row * 9 + 7] = fr2 * p;
         Jc[row * 9 + 8] = fr2 * r2 * p;
     }
+}
+
+// Residual + analytic Jacobian. Jc: 2x9 row-major (a[3], t[3], f, k1, k2);
+// Jp: 2x3 row-major.
+GBA_HD void residual_jacobian(const double* cam, const double* X, const double* obs, double* r, double* Jc, double* Jp) {
+    const double* a = cam;
+    const double t = a[0] * a[0] + a[1] * a[1] + a[2] * a[2];
+    const bool first_order = !(t > 1e-24);
+    // the branch's R = I + [a]x for the point, J_l = I, dX_c/dX = I and dRX/da = -[X]x
+    double A = 1.0, B = 0.0, C = 0.0, c = 1.0;
+    if (!first_order) rotation_terms(t, A, B, C, c);
+    const double A0 = A * a[0], A1 = A * a[1], A2 = A * a[2];
+    const double B0 = B * a[0], B1 = B * a[1], B2 = B * a[2];
+    const double C0 = C * a[0], C1 = C * a[1], C2 = C * a[2];
+    const double R[9] = {c + B0 * a[0],  B0 * a[1] - A2, B0 * a[2] + A1,
+                    B1 * a[0] + A2, c + B1 * a[1],  B1 * a[2] - A0,
+                    B2 * a[0] - A1, B2 * a[1] + A0, c + B2 * a[2]};
+    const double Jl[9] = {A + C0 * a[0],  C0 * a[1] - B2, C0 * a[2] + B1,
+                     C1 * a[0] + B2, A + C1 * a[1],  C1 * a[2] - B0,
+                     C2 * a[0] - B1, C2 * a[1] + B0, A + C2 * a[2]};
+    double RX[3];
+    for (int i = 0; i < 3; ++i) RX[i] = R[3 * i] * X[0] + R[3 * i + 1] * X[1] + R[3 * i + 2] * X[2];
+    jacobian_rows(R, Jl, RX, first_order, cam + 3, X, obs, r, Jc, Jp);
 }
 
 // Rotated point R(a) X (without translation) and the pieces the Jacobian needs.
@@ -321,6 +328,17 @@ GBA_HD void residual_jacobian_pre(const T* pre, const T* X, const T* obs, T* r, 
             Jp[row * 3 + j] = first_order ? DM[row * 3 + j]
                                           : g0 * R[j] + g1 * R[3 + j] + g2 * R[6 + j];
     }
+}
+
+// The same in FP64 with the common factors taken once: the FP64 kernels are bound by these instructions.
+GBA_HD void residual_jacobian_pre(const double* pre, const double* X, const double* obs, double* r, double* Jc,
+                                  double* Jp) {
+    const double* R = pre;
+    const double* Jl = pre + 9;
+    const bool first_order = pre[24] != 0.0;
+    double RX[3];
+    for (int i = 0; i < 3; ++i) RX[i] = R[3 * i] * X[0] + R[3 * i + 1] * X[1] + R[3 * i + 2] * X[2];
+    jacobian_rows(R, Jl, RX, first_order, pre + 18, X, obs, r, Jc, Jp);
 }
 
 // The per-camera constants of residual_jacobian_pre, in FP64 (28 slots; the

@@ -39,36 +39,55 @@ __device__ __forceinline__ bool all_finite(const T* v, int n) {
 
 // ---------------------------------------------------------------- FP64 path
 
+// Each warp's 32 x N values, one row per lane, to consecutive memory at dst (rows
+// rows of it): through shared memory, since a store of one column would touch 32
+// sectors. stage: 32 (N + 1 - N % 2) values of this warp.
+template <int N, typename T>
+__device__ __forceinline__ void store_rows(const T* v, T* stage, T* __restrict__ dst, int rows) {
+    constexpr int kLd = N + 1 - N % 2;  // odd: no bank conflicts
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < N; ++k) stage[kLd * lane + k] = v[k];
+    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const int i = 32 * k + lane;
+        if (i < N * rows) dst[i] = stage[kLd * (i / N) + i % N];
+    }
+    __syncwarp();
+}
+
 // Per-camera constants of the FP64 Jacobians (model::camera_constants: rotation,
 // left Jacobian, t, f, k1, k2), one camera per thread in warp-sized blocks: the
 // sine, cosine and square root of a camera are taken once, not once per
 // observation. The FP64 pipe bounds the point pass (a warp's FP64 instruction
-// takes 64 cycles): 605 -> 451 us at 1000 cameras and 200,000 points of about 8
-// observations, 197 -> 148 us at 257 cameras and 65,000 points.
+// takes 64 cycles): 605 -> 451 us at 1000 cameras and 800,000 observations, 197 ->
+// 148 us at 257 cameras and 225,000; with the Jacobian's common factors taken once
+// and the rows stored through shared memory 385 and 133 us.
 __global__ void camera_constants_kernel(const double* __restrict__ cams, int C, double* __restrict__ out) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c < C) model::camera_constants(cams + 9ll * c, out + static_cast<long long>(kCamRec) * c);
 }
 
-__global__ void __launch_bounds__(kPT) point_pass_f64(
+constexpr int kStage64 = 32 * 27;
+__global__ void __launch_bounds__(kPT, 2) point_pass_f64(
     const int* __restrict__ pchunk, const int* __restrict__ pt_off, const int* __restrict__ s_cam,
     const int* __restrict__ s_pt, const double2* __restrict__ s_px, const double* __restrict__ cam_rec,
     const double* __restrict__ pts, double* __restrict__ W, double* __restrict__ JcR, double* __restrict__ V,
     double* __restrict__ bp, double* __restrict__ sse_part, unsigned long long* __restrict__ counters,
     double delta) {
+    extern __shared__ double stage_f64[];  // kStage64 per warp
     __shared__ double contrib[9][kPT];
+    __shared__ int off[kPT + 1];           // the chunk's points' first slots
     __shared__ double red[kPT / 32];
     __shared__ unsigned long long redu[kPT / 32];
     const int chunk = blockIdx.x;
     const int p0 = pchunk[chunk], p1 = pchunk[chunk + 1];
     const int s0 = pt_off[p0], s1 = pt_off[p1];
-    const int my_p = p0 + threadIdx.x;
-    int my_b = 0, my_e = 0;
-    if (my_p < p1) {
-        my_b = pt_off[my_p];
-        my_e = pt_off[my_p + 1];
-    }
-    double acc[9];
+    double* stage = stage_f64 + kStage64 * (threadIdx.x >> 5);
+    const int npts = p1 - p0;  // at most kPT
+    for (int k = threadIdx.x; k <= npts; k += kPT) off[k] = pt_off[p0 + k];
+    double acc[9];  // thread t: sums t, t + kPT, ... of the chunk's 9 npts (point t / 9, value t % 9)
 #pragma unroll
     for (int k = 0; k < 9; ++k) acc[k] = 0.0;
     double sse = 0.0;
@@ -76,12 +95,16 @@ __global__ void __launch_bounds__(kPT) point_pass_f64(
 
     for (int base = s0; base < s1; base += kPT) {
         const int s = base + threadIdx.x;
-        double v[9];
+        double rec[20], Jp[6];  // [Jc(18), r(2)]; zeros without a (finite) observation
 #pragma unroll
-        for (int k = 0; k < 9; ++k) v[k] = 0.0;
+        for (int k = 0; k < 20; ++k) rec[k] = 0.0;
+#pragma unroll
+        for (int k = 0; k < 6; ++k) Jp[k] = 0.0;
+        double* const Jc = rec;
+        double* const r = rec + 18;
         if (s < s1) {
             const int c = s_cam[s], p = s_pt[s];
-            double cam[kCamRec], X[3], obs[2], r[2], Jc[18], Jp[6];
+            double cam[kCamRec], X[3], obs[2];
             const double2* c2 = reinterpret_cast<const double2*>(cam_rec + static_cast<long long>(kCamRec) * c);
 #pragma unroll
             for (int k = 0; k < 13; ++k) {  // 25 of the record's 28 values
@@ -95,61 +118,60 @@ __global__ void __launch_bounds__(kPT) point_pass_f64(
             obs[0] = o.x;
             obs[1] = o.y;
             model::residual_jacobian_pre(cam, X, obs, r, Jc, Jp);
-            const bool fin = all_finite(r, 2) && all_finite(Jc, 18) && all_finite(Jp, 6);
-            double* Ws = W + 27ll * s;
-            double* Qs = JcR + 20ll * s;
-            if (fin) {
+            if (all_finite(r, 2) && all_finite(Jc, 18) && all_finite(Jp, 6)) {
                 const double sq = r[0] * r[0] + r[1] * r[1];
                 sse += robust_rho(sq, delta);
                 if (delta > 0.0) {  // robust loss: rows scaled by sqrt(rho'(s))
                     const double sw = robust_sqrt_weight(sq, delta);
-                    r[0] *= sw;
-                    r[1] *= sw;
 #pragma unroll
-                    for (int k = 0; k < 18; ++k) Jc[k] *= sw;
+                    for (int k = 0; k < 20; ++k) rec[k] *= sw;
 #pragma unroll
                     for (int k = 0; k < 6; ++k) Jp[k] *= sw;
                 }
-#pragma unroll
-                for (int i = 0; i < 9; ++i)
-#pragma unroll
-                    for (int j = 0; j < 3; ++j) Ws[3 * i + j] = Jc[i] * Jp[j] + Jc[9 + i] * Jp[3 + j];
-#pragma unroll
-                for (int k = 0; k < 18; ++k) Qs[k] = Jc[k];
-                Qs[18] = r[0];
-                Qs[19] = r[1];
-                v[0] = Jp[0] * Jp[0] + Jp[3] * Jp[3];
-                v[1] = Jp[1] * Jp[0] + Jp[4] * Jp[3];
-                v[2] = Jp[1] * Jp[1] + Jp[4] * Jp[4];
-                v[3] = Jp[2] * Jp[0] + Jp[5] * Jp[3];
-                v[4] = Jp[2] * Jp[1] + Jp[5] * Jp[4];
-                v[5] = Jp[2] * Jp[2] + Jp[5] * Jp[5];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) v[6 + i] = -(Jp[i] * r[0] + Jp[3 + i] * r[1]);
             } else {
                 ++anom;
 #pragma unroll
-                for (int k = 0; k < 27; ++k) Ws[k] = 0.0;
+                for (int k = 0; k < 20; ++k) rec[k] = 0.0;
 #pragma unroll
-                for (int k = 0; k < 20; ++k) Qs[k] = 0.0;
+                for (int k = 0; k < 6; ++k) Jp[k] = 0.0;
             }
         }
+        const int w0 = base + (threadIdx.x & ~31), rows = max(0, min(32, s1 - w0));
+        store_rows<20>(rec, stage, JcR + 20ll * w0, rows);
+        {
+            double w[27];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) contrib[k][threadIdx.x] = v[k];
+            for (int i = 0; i < 9; ++i)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) w[3 * i + j] = Jc[i] * Jp[j] + Jc[9 + i] * Jp[3 + j];
+            store_rows<27>(w, stage, W + 27ll * w0, rows);
+        }
+        contrib[0][threadIdx.x] = Jp[0] * Jp[0] + Jp[3] * Jp[3];
+        contrib[1][threadIdx.x] = Jp[1] * Jp[0] + Jp[4] * Jp[3];
+        contrib[2][threadIdx.x] = Jp[1] * Jp[1] + Jp[4] * Jp[4];
+        contrib[3][threadIdx.x] = Jp[2] * Jp[0] + Jp[5] * Jp[3];
+        contrib[4][threadIdx.x] = Jp[2] * Jp[1] + Jp[5] * Jp[4];
+        contrib[5][threadIdx.x] = Jp[2] * Jp[2] + Jp[5] * Jp[5];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) contrib[6 + i][threadIdx.x] = -(Jp[i] * r[0] + Jp[3 + i] * r[1]);
         __syncthreads();
-        if (my_p < p1) {
-            const int b = max(my_b, base), e = min(my_e, base + kPT);
-            for (int t = b; t < e; ++t)
 #pragma unroll
-                for (int k = 0; k < 9; ++k) acc[k] += contrib[k][t - base];
+        for (int k = 0; k < 9; ++k) {
+            const int t = threadIdx.x + k * kPT, p = t / 9, q = t - 9 * p;
+            if (p >= npts) break;
+            const int b = max(off[p], base), e = min(off[p + 1], base + kPT);
+            for (int i = b; i < e; ++i) acc[k] += contrib[q][i - base];
         }
         __syncthreads();
     }
-    if (my_p < p1) {
 #pragma unroll
-        for (int k = 0; k < 6; ++k) V[6ll * my_p + k] = acc[k];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) bp[3ll * my_p + k] = acc[6 + k];
+    for (int k = 0; k < 9; ++k) {
+        const int t = threadIdx.x + k * kPT, p = t / 9, q = t - 9 * p;
+        if (p >= npts) break;
+        if (q < 6)
+            V[6ll * (p0 + p) + q] = acc[k];
+        else
+            bp[3ll * (p0 + p) + q - 6] = acc[k];
     }
     const double tot = block_sum<kPT>(sse, red);
     const unsigned long long na = block_sum_u64<kPT>(anom, redu);
@@ -177,7 +199,8 @@ __device__ __forceinline__ void halve(double (&u)[64], int bit) {
 
 // Camera pass: partials of U (lower triangle, row order) and bc per camera chunk.
 // Bound by the FP64 pipe; with the folded reduction and twice the warps per chunk
-// 380 -> 326 us at 1000 cameras, 113 -> 100 us at 257.
+// 380 -> 326 us at 1000 cameras, 113 -> 100 us at 257; with two FMAs a product pair
+// (not product, FMA and add) 222 and 69 us.
 __global__ void __launch_bounds__(kCT64) camera_pass_f64(const int* __restrict__ cchunk_begin,
                                                          const int* __restrict__ cchunk_cam,
                                                          const int* __restrict__ cam_off,
@@ -204,11 +227,11 @@ __global__ void __launch_bounds__(kCT64) camera_pass_f64(const int* __restrict__
         for (int a = 0; a < 9; ++a)
 #pragma unroll
             for (int bb = 0; bb <= a; ++bb) {
-                u[idx] += J[a] * J[bb] + J[9 + a] * J[9 + bb];
+                u[idx] = fma(J[a], J[bb], fma(J[9 + a], J[9 + bb], u[idx]));
                 ++idx;
             }
 #pragma unroll
-        for (int a = 0; a < 9; ++a) u[45 + a] -= J[a] * J[18] + J[9 + a] * J[19];
+        for (int a = 0; a < 9; ++a) u[45 + a] = fma(-J[a], J[18], fma(-J[9 + a], J[19], u[45 + a]));
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     halve<64>(u, 16);
@@ -707,24 +730,6 @@ __global__ void __launch_bounds__(kCostT, 4) cost_ff(const int* __restrict__ cch
     }
 }
 
-// Each warp's 32 x N values, one row per lane, to consecutive memory at dst (rows
-// rows of it): through shared memory, since a store of one column would touch 32
-// sectors. stage: 32 (N + 1 - N % 2) values of this warp.
-template <int N, typename T>
-__device__ __forceinline__ void store_rows(const T* v, T* stage, T* __restrict__ dst, int rows) {
-    constexpr int kLd = N + 1 - N % 2;  // odd: no bank conflicts
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 0; k < N; ++k) stage[kLd * lane + k] = v[k];
-    __syncwarp();
-#pragma unroll
-    for (int k = 0; k < N; ++k) {
-        const int i = 32 * k + lane;
-        if (i < N * rows) dst[i] = stage[kLd * (i / N) + i % N];
-    }
-    __syncwarp();
-}
-
 // One observation per thread, Jacobians to the caller's row-major arrays. In FP64
 // the FP64 pipe bounds it (about 170 instructions an observation; 800,000 of them
 // 330 -> 236 us with the rotation as series), in FP32 memory (85 -> 33 us, 128 MB,
@@ -771,7 +776,9 @@ void Solver::accumulate_launch() {
         cudaEvent_t ev = prof_start();
         camera_constants_kernel<<<ceil_div(C_, kPreT), kPreT, 0, stream_>>>(cams_.get(), C_, cam_rec_.get());
         GBA_LAUNCH_CHECK();
-        point_pass_f64<<<n_pchunk_, kPT, 0, stream_>>>(pchunk_.get(), pt_off_.get(), s_cam_.get(), s_pt_.get(),
+        const int stage_bytes = kPT / 32 * kStage64 * sizeof(double);
+        GBA_CUDA_CHECK(cudaFuncSetAttribute(point_pass_f64, cudaFuncAttributeMaxDynamicSharedMemorySize, stage_bytes));
+        point_pass_f64<<<n_pchunk_, kPT, stage_bytes, stream_>>>(pchunk_.get(), pt_off_.get(), s_cam_.get(), s_pt_.get(),
                                                        spx, cam_rec_.get(), pts_.get(), W_.get(), JcR_.get(),
                                                        V_.get(), bp_.get(), sse_part_.get(), counters_.get(),
                                                        huber_delta_);
