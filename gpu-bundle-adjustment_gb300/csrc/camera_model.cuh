@@ -97,9 +97,9 @@ GBA_HD void residual(const double* cam, const double* X, const double* obs, doub
         double A, B, C, c;
         rotation_terms(t, A, B, C, c);
         const double q = B * (a[0] * X[0] + a[1] * X[1] + a[2] * X[2]);
-        P[0] = c * X[0] + A * x0 + q * a[0] + cam[3];
-        P[1] = c * X[1] + A * x1 + q * a[1] + cam[4];
-        P[2] = c * X[2] + A * x2 + q * a[2] + cam[5];
+        P[0] = c * X[0] + (A * x0 + (q * a[0] + cam[3]));
+        P[1] = c * X[1] + (A * x1 + (q * a[1] + cam[4]));
+        P[2] = c * X[2] + (A * x2 + (q * a[2] + cam[5]));
     } else {
         P[0] = X[0] + x0 + cam[3];
         P[1] = X[1] + x1 + cam[4];

@@ -48,15 +48,18 @@ constexpr int NB = 64;                        // panel width / tile size
 constexpr int kTileB = NB * NB * 2;           // bytes of one FP16 digit tile
 constexpr int kNS = fx::kSlices;
 
-// Workspace: digit tiles (kNS per 64-row tile), row exponents, row flags.
+// Workspace: digit tiles (kNS per 64-row tile), which small updates replace by the
+// panel's rows as integers (64 per row), row exponents, row flags.
 struct Work {
     unsigned char* tiles;
+    long long* rows;
     int* e;
     int* bad;  // 1: fails at this row's pivot; 2: infinite diagonal entry
 };
 Work carve(void* ws, int n) {
     Work w;
     w.tiles = static_cast<unsigned char*>(ws);
+    w.rows = static_cast<long long*>(ws);
     w.e = reinterpret_cast<int*>(w.tiles + static_cast<size_t>(n / NB) * kNS * kTileB);
     w.bad = w.e + n;
     return w;
@@ -389,10 +392,15 @@ __device__ __forceinline__ void updating_warp(PanelSmem& sm, Acc (&a)[16], int g
 // FP64 columns and FP16 digit tiles of the rows in sm.lv[first, first + count):
 // row i of them is matrix row r0 + i.
 __device__ void panel_output(const PanelSmem& sm, int first, int count, int r0, double* __restrict__ A, int j0,
-                             int lda, const int* __restrict__ e, unsigned char* __restrict__ tiles) {
+                             int lda, const int* __restrict__ e, unsigned char* __restrict__ tiles,
+                             long long* __restrict__ rows) {
+    if (rows) {
+        for (int t = threadIdx.x; t < count * NB; t += kPanelThreads)
+            rows[static_cast<long long>(r0) * NB + t] = sm.lv[(first + (t >> 6)) * kLvS + (t & 63)];
+    }
     // digits: one thread per row and run of eight columns, a 16-byte store per digit,
     // in the 128-byte-swizzled K-major layout that the update's MMA reads
-    for (int t = threadIdx.x; t < count * 8; t += kPanelThreads) {
+    for (int t = threadIdx.x; !rows && t < count * 8; t += kPanelThreads) {
         const int i = t % count, kc = t / count;
         const int r = r0 + i, rt = r & 63;
         int q[8][kNS];
@@ -416,11 +424,13 @@ __device__ void panel_output(const PanelSmem& sm, int first, int count, int r0, 
     }
 }
 
+// rows: where the panel's rows go as integers, for chol_update_int (null: as digit tiles).
 // j0: first column of the panel; blockIdx.y = 1: of the second chain's, dj further on.
 __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restrict__ A, int j0, int dj, int lda,
                                                               int nbelow, int rpc, const int* __restrict__ e,
                                                               int* __restrict__ bad,
                                                               unsigned char* __restrict__ tiles,
+                                                              long long* __restrict__ rows,
                                                               int* __restrict__ info) {
     extern __shared__ __align__(16) unsigned char panel_smem[];
     PanelSmem& sm = *reinterpret_cast<PanelSmem*>(panel_smem);
@@ -483,7 +493,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
         return;
     }
     if (srow >= NB && rbad) bad[matrix_row(srow)] = 1;
-    if (nx > 0) panel_output(sm, NB, nx, j0 + NB + b0, A, j0, lda, e, tiles);
+    if (nx > 0) panel_output(sm, NB, nx, j0 + NB + b0, A, j0, lda, e, tiles, rows);
     if (blockIdx.x == 0) {  // the diagonal tile's factor
         for (int t = tid; t < NB * NB; t += kPanelThreads) {
             const int i = t & 63, k = t >> 6;
@@ -547,7 +557,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
             if (lv && rb && q == 0) bad[r] = 1;
         }
         __syncthreads();
-        panel_output(sm, 0, n, j0 + NB + c0, A, j0, lda, e, tiles);
+        panel_output(sm, 0, n, j0 + NB + c0, A, j0, lda, e, tiles, rows);
     }
 }
 
@@ -810,6 +820,48 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
     if (tid == 0 && gave_up) *info = INT_MIN;
 }
 
+// The update of a few tiles with integer multiply-adds, 16 x 16 entries per block, one
+// per thread: a tile of chol_update occupies one SM for the 112 MMAs of its 28 digit
+// products (77 cycles each) and its operands' way to shared memory, 10.4 us with the
+// launch, however few tiles there are; here they spread over all SMs. 576 rows
+// (9 panels) 380 -> 338 us.
+constexpr int kIntB = 16;
+__global__ void __launch_bounds__(kIntB * kIntB) chol_update_int(double* __restrict__ A, int j1, int dj, int lda,
+                                                                const long long* __restrict__ rows,
+                                                                const int* __restrict__ info) {
+    __shared__ __align__(16) Limbs L[2][kIntB][NB + 2];
+    int rb = static_cast<int>((sqrtf(8.f * blockIdx.x + 1.f) - 1.f) * 0.5f);
+    while (rb * (rb + 1) / 2 > static_cast<int>(blockIdx.x)) --rb;
+    while ((rb + 1) * (rb + 2) / 2 <= static_cast<int>(blockIdx.x)) ++rb;
+    const int cb = blockIdx.x - rb * (rb + 1) / 2;
+    j1 += blockIdx.y * dj;
+    const int i = threadIdx.x & (kIntB - 1), j = threadIdx.x / kIntB;  // row, column of the block
+    const int row = j1 + kIntB * rb + i, col = j1 + kIntB * cb + j;
+    pdl_wait();
+    pdl_trigger();
+    if (*info) return;
+    long long* p = reinterpret_cast<long long*>(A) + row + static_cast<long long>(col) * lda;
+    Acc acc = {row >= col ? *p : 0, 0};
+#pragma unroll
+    for (int t = threadIdx.x; t < 2 * kIntB * NB; t += kIntB * kIntB) {
+        const int h = t / (kIntB * NB), r = (t / NB) % kIntB, k = t % NB;
+        L[h][r][k] = fx::split(rows[static_cast<long long>(j1 + kIntB * (h ? cb : rb) + r) * NB + k]);
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < NB; k += 4) {
+        Limbs a[4], b[4];
+        load_limbs4(&L[0][i][k], a);
+        load_limbs4(&L[1][j][k], b);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) fx::fms(acc, a[q], b[q]);
+    }
+    if (row >= col) *p = fx::value(acc);
+}
+// Most tiles below the diagonal tile that it serves: of a step (panel and update) of
+// 42 us, 5 us less at up to 8 tiles, 3 at 12, none at 16, 10 more at 24.
+constexpr int kIntTiles = 12;
+
 }  // namespace
 
 size_t dense_potrf_workspace(int n) {
@@ -823,9 +875,16 @@ static void factor_panel(double* A, int j0, int dj, int chains, int below, int l
     // rows per CTA: kExtra are solved along with the diagonal tile; more only
     // where the panel has more than that for every SM
     const int rpc = kExtra * std::max(1, ceil_div(rows * chains, kExtra * sms));
+    const bool ints = below <= kIntTiles;
     launch_pdl(chol_panel, dim3(std::max(1, ceil_div(rows, rpc)), chains), kPanelThreads, sizeof(PanelSmem), s, A, j0,
-               dj, lda, rows, rpc, w.e, w.bad, w.tiles, info);
+               dj, lda, rows, rpc, w.e, w.bad, w.tiles, ints ? w.rows : nullptr, info);
     if (below == 0) return;
+    if (ints) {
+        const int blocks = rows / kIntB;
+        launch_pdl(chol_update_int, dim3(blocks * (blocks + 1) / 2, chains), kIntB * kIntB, 0, s, A, j0 + NB, dj, lda,
+                   w.rows, info);
+        return;
+    }
     const long long pairs = below / 2;
     const long long tiles = pairs * (pairs + 1) + (below % 2 ? below : 0);
     launch_pdl(chol_update, dim3(static_cast<unsigned>(std::min<long long>(tiles, std::max(1, sms / chains))), chains),

@@ -544,9 +544,9 @@ __global__ void camera_precompute_kernel(const double* __restrict__ cams, int C,
 
 __device__ __forceinline__ void residual_pre(const double* __restrict__ pc, const double* X, const double* obs,
                                              double* r) {
-    const double P0 = pc[0] * X[0] + pc[1] * X[1] + pc[2] * X[2] + pc[9];
-    const double P1 = pc[3] * X[0] + pc[4] * X[1] + pc[5] * X[2] + pc[10];
-    const double P2 = pc[6] * X[0] + pc[7] * X[1] + pc[8] * X[2] + pc[11];
+    const double P0 = pc[0] * X[0] + (pc[1] * X[1] + (pc[2] * X[2] + pc[9]));
+    const double P1 = pc[3] * X[0] + (pc[4] * X[1] + (pc[5] * X[2] + pc[10]));
+    const double P2 = pc[6] * X[0] + (pc[7] * X[1] + (pc[8] * X[2] + pc[11]));
     const double iz = 1.0 / P2;
     const double u = -P0 * iz, v = -P1 * iz;
     const double r2 = u * u + v * v;

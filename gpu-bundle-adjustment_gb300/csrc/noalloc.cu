@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(kCostThreads) cost_chunk_kernel(const double* 
         obs[1] = px[2 * e + 1];
         model::residual(cam, X, obs, r);
         if (isfinite(r[0]) && isfinite(r[1]))
-            sse += r[0] * r[0] + r[1] * r[1];
+            sse = r[0] * r[0] + (r[1] * r[1] + sse);
         else
             ++bad;
     }

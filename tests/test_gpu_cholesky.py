@@ -55,7 +55,7 @@ def test_factor_matches_long_double(gba, torch_cuda, n, lda, spread):
 
 
 # rows per CTA above the fused group (16 x 152 rows), a second pass of 128 rows
-@pytest.mark.parametrize("n", [2688, 5120])
+@pytest.mark.parametrize("n", [832, 896, 2688, 5120])  # 12 and 13 tiles: either side of the update kernels
 def test_large_factor_residual(gba, torch_cuda, n):
     torch = torch_cuda
     g = torch.Generator(device="cuda").manual_seed(n)
