@@ -92,9 +92,9 @@ __device__ __forceinline__ float norm(float a) { return a; }
 __device__ __forceinline__ float shfl_up(float a, int d) { return __shfl_up_sync(0xffffffffu, a, d); }
 __device__ __forceinline__ double as_double(float a) { return a; }
 __device__ __forceinline__ double as_double(ff a) { return ffa::to_double(a); }
-template <typename T> __device__ __forceinline__ T from_double(double d);
-template <> __device__ __forceinline__ float from_double<float>(double d) { return static_cast<float>(d); }
-template <> __device__ __forceinline__ ff from_double<ff>(double d) { return ffa::from_double(d); }
+template <typename T> __device__ __forceinline__ T from_float(float f);
+template <> __device__ __forceinline__ float from_float<float>(float f) { return f; }
+template <> __device__ __forceinline__ ff from_float<ff>(float f) { return {f, 0.f}; }
 __device__ __forceinline__ float hi_of(float x) { return x; }
 __device__ __forceinline__ float hi_of(ff x) { return x.hi; }
 __device__ __forceinline__ ff to_ff(float x) { return {x, 0.f}; }
@@ -286,7 +286,6 @@ __global__ void __launch_bounds__(kPT, sizeof(T) == 4 ? (kBack ? 6 : 8) : (kBack
     __shared__ T wsh[kPT][3];
     __shared__ __align__(16) float vsh[kPT][6];  // FP32 V'^-1 of the chunk's points
     __shared__ float bsum[kPT / 32][2];
-    __shared__ double bout[kBack ? 9 * kPT : 1];  // back-substitution outputs of the chunk's points
     if (done && *done != 0.0) return;
     const int chunk = blockIdx.x;
     // the chunk's points and slots: one 16-byte load from the range table (a
@@ -323,6 +322,27 @@ __global__ void __launch_bounds__(kPT, sizeof(T) == 4 ? (kBack ? 6 : 8) : (kBack
         for (int i = threadIdx.x; i < 3 * (p1 - p0); i += kPT) cp_async8(dst + i, src + i);
     } else {
         if (my_p < p1) load_vinv(vinv_hi, vinv_lo, my_p, vinv);
+    }
+    constexpr bool kEarlyBp = kBack || kRhs;  // (elsewhere a is 0 as a rule, and the registers are not there)
+    double bpd[3] = {0.0, 0.0, 0.0};
+    auto load_bp = [&] {
+        if (my_p < p1 && a != 0.0) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) bpd[k] = bp[3ll * my_p + k];
+        }
+    };
+    if constexpr (kEarlyBp) load_bp();
+    // back-substitution: entry i = 3 (p - p0) + k of the chunk's points per thread
+    const int n3 = 3 * (p1 - p0);
+    double pt_i = 0.0, v_i = 0.0, bp_i = 0.0;
+    auto load_entry = [&](int i) {
+        const int pp = i / 3, k = i - 3 * pp;
+        pt_i = bk.pts[3ll * p0 + i];
+        v_i = bk.V[6ll * (p0 + pp) + (k == 0 ? 0 : k == 1 ? 2 : 5)];
+        bp_i = bp[3ll * p0 + i];
+    };
+    if constexpr (kBack) {
+        if (static_cast<int>(threadIdx.x) < n3) load_entry(threadIdx.x);
     }
     // Single-pass chunks (the usual case) keep the slot's Jp, point and
     // camera-major position in registers for the u phase.
@@ -417,11 +437,12 @@ __global__ void __launch_bounds__(kPT, sizeof(T) == 4 ? (kBack ? 6 : 8) : (kBack
     }
     T w0 = zero<T>(), w1 = zero<T>(), w2 = zero<T>();
     if (my_p < p1) {
-        if (a != 0.0) {
-            z0 = add(z0, from_double<T>(a * bp[3ll * my_p]));
-            z1 = add(z1, from_double<T>(a * bp[3ll * my_p + 1]));
-            z2 = add(z2, from_double<T>(a * bp[3ll * my_p + 2]));
-        }
+        // a is 1, -1 or 0, and bp holds FP32 sums, exact in FP32
+        if constexpr (!kEarlyBp) load_bp();
+        const float fa = static_cast<float>(a);
+        z0 = add(z0, from_float<T>(fa * static_cast<float>(bpd[0])));
+        z1 = add(z1, from_float<T>(fa * static_cast<float>(bpd[1])));
+        z2 = add(z2, from_float<T>(fa * static_cast<float>(bpd[2])));
         apply_vinv(vinv, z0, z1, z2, w0, w1, w2);
         wsh[threadIdx.x][0] = w0;
         wsh[threadIdx.x][1] = w1;
@@ -433,27 +454,25 @@ __global__ void __launch_bounds__(kPT, sizeof(T) == 4 ? (kBack ? 6 : 8) : (kBack
     }
     if constexpr (kBack) {
         // dp (FP64 out), trial points (FP64 sum), and the gain denominator's
-        // point terms dp_k (lambda max(V_kk, 1e-12) dp_k + bp_k) in float-float;
-        // V and bp hold FP32 sums here, exact in FP32.
+        // point terms dp_k (lambda max(V_kk, 1e-12) dp_k + bp_k) in float-float, one
+        // entry of the chunk's points per thread (an owner's three in turn are a
+        // chain of FP64 instructions that the block waits for); V and bp hold FP32
+        // sums here, exact in FP32.
+        __syncthreads();
+        const ff lam = {bk.lambda.x, bk.lambda.y};
         ff den = {0.f, 0.f};
-        if (my_p < p1) {
-            const long long p = my_p;
-            const ff lam = {bk.lambda.x, bk.lambda.y};
-            const ff d[3] = {ffa::neg(to_ff(w0)), ffa::neg(to_ff(w1)), ffa::neg(to_ff(w2))};
-            const int diag[3] = {0, 2, 5};
-#pragma unroll
-            for (int k = 0; k < 3; ++k) {
-                const double dk = ffa::to_double(d[k]);
-                const double tp = bk.pts[3 * p + k] + dk;
-                const ff tf = ffa::from_double(tp);
-                bout[3 * threadIdx.x + k] = dk;
-                bout[3 * kPT + 3 * threadIdx.x + k] = tp;
-                reinterpret_cast<float2*>(bout + 6 * kPT)[3 * threadIdx.x + k] = make_float2(tf.hi, tf.lo);
-                const float vk = static_cast<float>(bk.V[6 * p + diag[k]]);
-                ff t = {static_cast<float>(bp[3 * p + k]), 0.f};
-                ffa::madd(t, ffa::mul(lam, ff{vk > 0.f ? vk : 1e-12f, 0.f}), d[k]);
-                ffa::madd(den, ffa::norm(t), d[k]);
-            }
+        for (int i = threadIdx.x; i < n3; i += kPT) {
+            if (i >= kPT) load_entry(i);
+            const ff d = ffa::neg(to_ff(wsh[i / 3][i % 3]));
+            const double dk = ffa::to_double(d), tp = pt_i + dk;
+            const ff tf = ffa::from_double(tp);
+            bk.dp[3ll * p0 + i] = dk;
+            bk.tpts[3ll * p0 + i] = tp;
+            bk.tpts_ff[3ll * p0 + i] = make_float2(tf.hi, tf.lo);
+            const float vk = static_cast<float>(v_i);
+            ff t = {static_cast<float>(bp_i), 0.f};
+            ffa::madd(t, ffa::mul(lam, ff{vk > 0.f ? vk : 1e-12f, 0.f}), d);
+            ffa::madd(den, ffa::norm(t), d);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) den = ffa::add(den, ffa::shfl_xor(den, o));
@@ -468,18 +487,10 @@ __global__ void __launch_bounds__(kPT, sizeof(T) == 4 ? (kBack ? 6 : 8) : (kBack
             for (int w = 0; w < kPT / 32; ++w) t += static_cast<double>(bsum[w][0]) + static_cast<double>(bsum[w][1]);
             bk.part[chunk] = t;
         }
-        // dp, trial points and their split for the chunk's contiguous points, as
-        // contiguous runs
-        const int np = p1 - p0;
-        const float2* bff = reinterpret_cast<const float2*>(bout + 6 * kPT);
-        for (int i = threadIdx.x; i < 3 * np; i += kPT) {
-            bk.dp[3ll * p0 + i] = bout[i];
-            bk.tpts[3ll * p0 + i] = bout[3 * kPT + i];
-            bk.tpts_ff[3ll * p0 + i] = bff[i];
-        }
         if (!u_cm) return;
+    } else {
+        __syncthreads();
     }
-    __syncthreads();
     // u_e = Jp_e w_p for every slot of the chunk, stored camera-major (kAcc:
     // Jc_e^T u_e added into the camera's accumulators)
     if (single) {
