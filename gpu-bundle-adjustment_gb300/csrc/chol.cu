@@ -854,7 +854,7 @@ __global__ void __launch_bounds__(kIntB * kIntB) chol_update_int(double* __restr
         load_limbs4(&L[0][i][k], a);
         load_limbs4(&L[1][j][k], b);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) fx::fms(acc, a[q], b[q]);
+        for (int q = 0; q < 4; ++q) fx::fms_full(acc, a[q], b[q]);
     }
     if (row >= col) *p = fx::value(acc);
 }

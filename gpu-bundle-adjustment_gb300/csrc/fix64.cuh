@@ -137,8 +137,10 @@ GBA_FX double to_double(long long v, int e) {
 }
 
 // Products: v = hi 2^30 + lo, lo in [-2^29, 2^29). The product of two entries,
-// in units of 2^-60, is hi hi' + (hi lo' + lo hi') 2^-30 (lo lo' 2^-60 is below
-// half a unit): sums keep the two parts in two 64-bit accumulators.
+// in units of 2^-60, is hi hi' + (hi lo' + lo hi' + lo lo' 2^-30) 2^-30: sums keep the
+// two parts in two 64-bit accumulators. lo lo' is below a quarter unit: fms leaves it
+// out (within a panel, whose rounds wait for one another: an entry takes at most 63
+// such products), fms_full takes it from the upper halves of the factors.
 struct Limbs {
     int hi, lo;
 };
@@ -156,6 +158,10 @@ GBA_FX void fms(Acc& a, Limbs x, Limbs y) {  // a -= x y
     a.c += static_cast<long long>(nh) * y.hi;
     a.m += static_cast<long long>(nh) * y.lo;
     a.m += static_cast<long long>(nl) * y.hi;
+}
+GBA_FX void fms_full(Acc& a, Limbs x, Limbs y) {
+    fms(a, x, y);
+    a.m += static_cast<long long>(-x.lo >> 15) * (y.lo >> 15);
 }
 GBA_FX long long value(const Acc& a) { return a.c + ((a.m + (1ll << 29)) >> 30); }
 
