@@ -348,18 +348,23 @@ def fp64_tensor_peak_tflops():
 
 
 def roofline_potrf(solver, C):
+    """The factorisation of S: FP16 digit products of its trailing updates (28 per
+    entry product, csrc/chol.cu) against the measured 16-bit tensor peak, and its
+    FP64-equivalent rate beside cuBLAS DGEMM."""
     n_launch, k_ms = solver.kernel_stats("dense_potrf")
     if not n_launch:
         return None
     per_launch_s = k_ms / n_launch / 1e3
     n = 9 * C
-    achieved = n ** 3 / 3.0 / per_launch_s / 1e12
-    peak = fp64_tensor_peak_tflops()
+    fp64_rate = n ** 3 / 3.0 / per_launch_s / 1e12
+    peaks, src = _peaks()
+    achieved, peak = 28 * fp64_rate, peaks["bf16_tflops"]
     return {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "traffic": None, "kernel": "dense_potrf",
             "launches": n_launch, "avg_launch_s": per_launch_s,
-            "peak_source": "measured in this run: cuBLAS DGEMM 8192^3 (FP64 tensor cores), best of 3; "
-                           "MEASURED_PEAKS.json has no FP64 entry"}
+            "fp64_equivalent_tflops": fp64_rate, "dgemm_tflops": fp64_tensor_peak_tflops(),
+            "peak_source": f"{src} 16-bit tensor peak (MEASURED_PEAKS.json bf16_tflops); 28 FP16 digit products per "
+                           "FP64 product; dgemm_tflops: cuBLAS DGEMM 8192^3 in this run"}
 
 
 # ----------------------------------------------------------------- the GPU arm
