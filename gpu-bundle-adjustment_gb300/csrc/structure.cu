@@ -36,8 +36,14 @@ cudaMemPool_t device_pool() {
 }  // namespace
 
 StreamAllocScope::StreamAllocScope(cudaStream_t s) : prev_s_(t_alloc_stream), prev_on_(t_alloc_async) {
-    unsigned long long keep = kPoolKeepBytes;  // the attribute is a 64-bit unsigned value
-    GBA_CUDA_CHECK(cudaMemPoolSetAttribute(device_pool(), cudaMemPoolAttrReleaseThreshold, &keep));
+    // (not while the stream is captured, which does not permit it: the allocations
+    // become nodes of the graph then)
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    GBA_CUDA_CHECK(cudaStreamIsCapturing(s, &capture));
+    if (capture == cudaStreamCaptureStatusNone) {
+        unsigned long long keep = kPoolKeepBytes;  // the attribute is a 64-bit unsigned value
+        GBA_CUDA_CHECK(cudaMemPoolSetAttribute(device_pool(), cudaMemPoolAttrReleaseThreshold, &keep));
+    }
     t_alloc_stream = s;
     t_alloc_async = true;
 }
