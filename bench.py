@@ -284,7 +284,7 @@ def roofline_mixed(solver, breakdown, C, P, E, workload, seed):
     unit = max(share, key=share.get)
     if share[unit] == 0.0:
         return None
-    source = "timed region (CUDA events per launch on the solver stream)"
+    source = "one further step (CUDA events per launch on the solver stream)"
     if unit == "matvec":
         solver.reset_params()
         solver.accumulate()
@@ -577,8 +577,6 @@ def run_ours(args):
     for _ in range(args.warmup):
         solver.reset_params()
         solver.run(**opts)
-    solver.profile(True)
-    solver.profile_reset()
     if world > 1:
         torch.distributed.barrier()
     torch.cuda.synchronize()
@@ -590,7 +588,13 @@ def run_ours(args):
     ms_per_step = max_over_ranks(ms_total, world) / args.steps
     if world > 1:
         torch.distributed.barrier()
-    breakdown = _breakdown(solver, args.steps)
+    # the breakdown: a step of its own, with an event pair around every stage (the
+    # events come between the chained launches of a PCG iteration)
+    solver.profile(True)
+    solver.profile_reset()
+    solver.reset_params()
+    solver.run(**opts)
+    breakdown = _breakdown(solver, 1)
     if form == "plain":
         roofline = roofline_potrf(solver, C)
     else:
