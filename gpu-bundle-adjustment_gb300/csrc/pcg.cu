@@ -71,6 +71,7 @@ constexpr int kUT = 9 * kUC;   // their block size
 // Device scalar slots (pcg_s_). Within one PCG iteration each slot is written
 // by one kernel (block 0, thread 0) and read only by later kernels, except
 // S_DONE, whose value every block of the writing kernel derives itself:
+//   pcg_tail           reads all, writes all at its end (one cluster, one thread), or, as separate kernels:
 //   pcg_update         reads S_RZ;            writes S_RZPREV, S_ITERS (and S_DONE on breakdown)
 //   pcg_direction      reads S_RZPREV, S_ITERS; writes S_RZ, S_RR, S_BETA, S_DONE
 enum { S_RZ = 0, S_ALPHA, S_BETA, S_RR, S_BB, S_DONE, S_ITERS, S_TOL2, S_NORM, S_RZPREV, S_BTX0, S_BTX1 };
@@ -846,6 +847,26 @@ __global__ void __launch_bounds__(kPT, kMCtas) schur_matvec_long(
         sl = nsl;
         cam = ncam;
         aid = naid;
+    }
+}
+
+// schur_matvec_long's form of the lists (lchunk: {first entry of lpts, entries}).
+__global__ void __launch_bounds__(kVT) long_desc_kernel(const int2* __restrict__ lchunk, int n,
+                                                       const int* __restrict__ lpts, const int* __restrict__ pt_off,
+                                                       int4* __restrict__ ldesc) {
+    const int k = blockIdx.x * kVT + threadIdx.x;
+    if (k >= n) return;
+    const int2 lc = lchunk[k];
+    int v = 0;
+    for (int j = 0; j < kLongPts; ++j) {
+        int4 d = make_int4(v, 0, 0, v);
+        if (j < lc.y) {
+            const int p = lpts[lc.x + j];
+            d.y = pt_off[p];
+            d.z = p;
+            d.w = v = v + pt_off[p + 1] - d.y;
+        }
+        ldesc[static_cast<long long>(kLongPts) * k + j] = d;
     }
 }
 
@@ -2997,24 +3018,18 @@ void Solver::build_point_groups() {
     if (!wc.empty())
         GBA_CUDA_CHECK(cudaMemcpyAsync(wchunk_.get(), wc.data(), wc.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                        stream_));
-    std::vector<int4> ld(kLongPts * std::max<size_t>(lc.size(), 1));
-    for (size_t k = 0; k < lc.size(); ++k) {  // schur_matvec_long's form of the lists
-        int v = 0;
-        for (int j = 0; j < lc[k].y; ++j) {
-            const int p = lp[lc[k].x + j], n = off[p + 1] - off[p];
-            ld[kLongPts * k + j] = make_int4(v, off[p], p, v + n);
-            v += n;
-        }
-        for (int j = lc[k].y; j < kLongPts; ++j) ld[kLongPts * k + j] = make_int4(v, 0, 0, v);
-    }
-    ldesc_.alloc(4 * ld.size());
+    ldesc_.alloc(4ull * kLongPts * std::max<size_t>(lc.size(), 1));
     if (!lc.empty()) {
-        GBA_CUDA_CHECK(cudaMemcpyAsync(ldesc_.get(), ld.data(), ld.size() * sizeof(int4), cudaMemcpyHostToDevice,
-                                       stream_));
         GBA_CUDA_CHECK(cudaMemcpyAsync(lchunk_.get(), lc.data(), lc.size() * sizeof(int2), cudaMemcpyHostToDevice,
                                        stream_));
         GBA_CUDA_CHECK(cudaMemcpyAsync(lpts_.get(), lp.data(), lp.size() * sizeof(int), cudaMemcpyHostToDevice,
                                        stream_));
+    }
+    if (n_lchunk_ > 0) {
+        long_desc_kernel<<<ceil_div(n_lchunk_, kVT), kVT, 0, stream_>>>(reinterpret_cast<const int2*>(lchunk_.get()),
+                                                                       n_lchunk_, lpts_.get(), pt_off_.get(),
+                                                                       reinterpret_cast<int4*>(ldesc_.get()));
+        GBA_LAUNCH_CHECK();
     }
     if (!hr.empty())
         GBA_CUDA_CHECK(cudaMemcpyAsync(huge_range_.get(), hr.data(), hr.size() * sizeof(int4),

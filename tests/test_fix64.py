@@ -3,7 +3,8 @@
 
 Bounds: conversions round to nearest; a reciprocal square root is good to 2^-59
 (its series' next term is below 2^-63, its operands 2^-61); an entry scaled by it
-to one unit of 2^-60 times the pivot's 2^s; a product of limbs to 1.5 units.
+to one unit of 2^-60 times the pivot's 2^s; a product of limbs to 1.5 units, with the
+low halves to half a unit and the 2^-15 that their dropped bits can weigh twice.
 """
 import shutil
 import subprocess
@@ -54,6 +55,10 @@ int main() {
         Acc acc{0, 0};
         fms(acc, a, b);
         CHECK(fabsl(static_cast<long double>(value(acc)) + ldexpl(static_cast<long double>(v) * w, -60)) <= 1.5L);
+        Acc full{0, 0};
+        fms_full(full, a, b);
+        const __int128 diff = (static_cast<__int128>(value(full)) << 60) + static_cast<__int128>(v) * w;
+        CHECK(fabsl(ldexpl(static_cast<long double>(diff), -60)) <= 0.502L);
         const int e = static_cast<int>(r() % 2100) - 1075;
         CHECK(to_double(v, e) == static_cast<double>(ldexpl(static_cast<long double>(v), e - 60)));
     }
