@@ -2537,18 +2537,19 @@ static cudaLaunchConfig_t tail_config(const TailPlan& t, cudaStream_t stream, cu
     cfg.numAttrs = 2;
     return cfg;
 }
-// What a cluster of t needs beyond the defaults.
+// What a cluster may need beyond the defaults (the same for every solver: solvers of
+// several threads share the kernels' attributes).
+constexpr int kTailMaxSmem = 2 * 9 * sizeof(float) * (kTailMaxC / (kTailMaxCtas / 2));
 template <bool kZ, bool kOne>
-static void allow_tail(const TailPlan& t) {
+static void allow_tail() {
     GBA_CUDA_CHECK(cudaFuncSetAttribute(pcg_tail<kZ, kOne>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    GBA_CUDA_CHECK(cudaFuncSetAttribute(pcg_tail<kZ, kOne>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(t.smem)));
+    GBA_CUDA_CHECK(cudaFuncSetAttribute(pcg_tail<kZ, kOne>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTailMaxSmem));
 }
 template <bool kZ, bool kOne>
 static void launch_tail_as(Solver& s, const TailPlan& t, int max_iters) {
     cudaLaunchAttribute at[2];
     const cudaLaunchConfig_t cfg = tail_config(t, s.stream_, at);
-    allow_tail<kZ, kOne>(t);
+    allow_tail<kZ, kOne>();
     GBA_CUDA_CHECK(cudaLaunchKernelEx(&cfg, pcg_tail<kZ, kOne>,
                                       static_cast<const float*>(s.pcg_q_.get()), s.pcg_e_.get(), s.pcg_r_.get(),
                                       s.pcg_p32_.get(), static_cast<const float*>(s.Pinv_.get()),
@@ -2566,23 +2567,27 @@ static void launch_tail(Solver& s, const TailPlan& t, bool coarse, int max_iters
         t.one_round ? launch_tail_as<false, true>(s, t, max_iters) : launch_tail_as<false, false>(s, t, max_iters);
     s.prof_stop("pcg_tail", ev);
 }
-static TailPlan plan_tail(const Solver& s) {
+static TailPlan plan_tail(Solver& s) {
     TailPlan t;
     if (s.C_ > kTailMaxC) return t;
-    for (int ctas : {kTailMaxCtas, kTailMaxCtas / 2}) {  // 16 CTAs per cluster are an opt-in the device may refuse
+    auto with = [&](int ctas) {
         t.ctas = ctas;
         t.per = ceil_div(s.C_, ctas);
         t.one_round = 9 * t.per <= kTailMaxT;
         t.threads = t.one_round ? std::max(kTailMinT, 32 * ceil_div(9 * t.per, 32)) : kTailMaxT;
         t.smem = 2 * 9 * sizeof(float) * t.per;
-        if (ctas == kTailMaxCtas / 2) return t;
+    };
+    if (!s.tail_ctas_) {  // 16 CTAs per cluster are an opt-in the device may refuse
+        with(kTailMaxCtas);
         cudaLaunchAttribute at[2];
         const cudaLaunchConfig_t cfg = tail_config(t, s.stream_, at);
         int fit = 0;
-        allow_tail<true, true>(t);
-        if (cudaOccupancyMaxActiveClusters(&fit, pcg_tail<true, true>, &cfg) == cudaSuccess && fit > 0) return t;
-        cudaGetLastError();
+        allow_tail<true, true>();
+        const bool ok = cudaOccupancyMaxActiveClusters(&fit, pcg_tail<true, true>, &cfg) == cudaSuccess && fit > 0;
+        if (!ok) cudaGetLastError();
+        s.tail_ctas_ = ok ? kTailMaxCtas : kTailMaxCtas / 2;
     }
+    with(s.tail_ctas_);
     return t;
 }
 

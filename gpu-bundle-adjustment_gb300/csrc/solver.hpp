@@ -244,10 +244,11 @@ public:
     static constexpr int kCamChunkSlots = 1024;  // most positions of a camera chunk
     bool one_pass_ = false;
     int n_acc_ = 0;
+    int tail_ctas_ = 0;  // cluster size of pcg_tail on this device (0: not asked yet)
     // the warp-level point passes' work: warp chunks (whole points, at most
     // 32 slots: int2 {first, end slot}); points with 33 to 256 observations in
     // lists of at most 256 slots per CTA (lchunk_: int2 {first entry of lpts_,
-    // entries}); longer points as ranges (int4 {p, p + 1, first slot, end
+    // entries}; ldesc_: the same for the product, eight int4 per list); longer points as ranges (int4 {p, p + 1, first slot, end
     // slot}) for the chunked point passes
     int n_wchunk_ = 0, n_lchunk_ = 0, n_huge_ = 0;
     DevBuf<int> wchunk_, lchunk_, lpts_, ldesc_, huge_range_;

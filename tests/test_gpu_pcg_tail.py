@@ -82,3 +82,15 @@ def test_edges_of_the_range(gba, C, mode):
         assert rr <= OPTS["refine_tol"]
         its.append(it)
     assert abs(its[0] - its[1]) <= max(its) / 4 + 3
+
+
+def test_two_sizes_in_two_threads(gba):
+    """Solvers of different sizes share the kernels (and their launch attributes)."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    probs = [gba.synthetic_custom(C, 10 * C, 2, 8, 1.3, seed=C) for C in (100, 12000)]
+    with ThreadPoolExecutor(2) as pool:
+        runs = list(pool.map(lambda p: [_solve(gba, p, "learned") for _ in range(6)], probs))
+    for run in runs:
+        for it, steps, rr in run:
+            assert rr <= OPTS["refine_tol"]
