@@ -72,7 +72,7 @@ def test_edges_at_all_angles(gba, torch_cuda, E, precision, tol):
             assert np.abs(g[e] - r.ravel()).max() <= tol * max(np.abs(r).max(), 500.0 if r.shape == (2,) else 0.0)
 
 
-@pytest.mark.parametrize("n", [1, 31, 33, 131])
+@pytest.mark.parametrize("n", [1, 31, 33, 131, 9999])  # 9,999: more than 64 per SM
 def test_blocks_on_both_paths(gba, torch_cuda, n):
     torch = torch_cuda
     rng = np.random.default_rng(n)
