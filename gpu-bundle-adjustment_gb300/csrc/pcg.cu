@@ -1305,6 +1305,32 @@ __device__ __forceinline__ void store_u9(float* __restrict__ rec, const float* j
     reinterpret_cast<float2*>(rec)[8] = make_float2(u[16], u[17]);
 }
 
+// The same for a warp whose first n lanes hold slots, lane's at camera-major position
+// q: through shared memory (kU9 floats per lane), five adjacent lanes to one record, so
+// that a store reaches six or seven records' lines instead of 32: both point passes
+// 851 -> 629 us at 8.8 million observations, bound by L1's data path. The position
+// travels in the record's padding. (The basis rows fetched the same way, eleven lanes
+// to a camera: 659 us, fewer CTAs.)
+__device__ __forceinline__ void scatter_u9(float* __restrict__ u9, float* stage, const float* jp, const float* w, int q,
+                                           int n) {
+    const int lane = threadIdx.x & 31;
+    if (lane < n) {
+        store_u9(stage + kU9 * lane, jp, w);
+        stage[kU9 * lane + 18] = __int_as_float(q);
+        stage[kU9 * lane + 19] = 0.f;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        const int t = 32 * i + lane, j = t / 5, k = t - 5 * j;
+        if (j < n) {
+            const long long at = __float_as_int(stage[kU9 * j + 18]);
+            reinterpret_cast<float4*>(u9 + kU9 * at)[k] = reinterpret_cast<const float4*>(stage + kU9 * j)[k];
+        }
+    }
+    __syncwarp();
+}
+
 // The basis is used at BF16 precision: Zb[c][i][j] = bf16(Z[j][9c + i]), the
 // per-camera rows the point pass gathers (176 B per camera), and Z itself (and
 // its FP32 copy Zc32, for the PCG) is overwritten by the same rounded values,
@@ -1476,6 +1502,7 @@ __global__ void __launch_bounds__(32 * kMWarps) coarse_point_pass9_warp(
     const int* __restrict__ cam_pos, const float* __restrict__ Jc32, const float* __restrict__ Jp32, long long js,
     const float* __restrict__ vinv, const __nv_bfloat16* __restrict__ Zb, float* __restrict__ u9) {
     constexpr int KV = 3 * kCoarse;
+    __shared__ __align__(16) float stages[kMWarps][32 * kU9];
     const int wid = blockIdx.x * kMWarps + (threadIdx.x >> 5);
     if (wid >= n_wchunk) return;  // whole warps leave together
     const int lane = threadIdx.x & 31;
@@ -1483,7 +1510,7 @@ __global__ void __launch_bounds__(32 * kMWarps) coarse_point_pass9_warp(
     const int s = r.x + lane;
     const bool has = s < r.y;
     int key = -1;
-    long long q = 0;
+    int q = 0;
     float J[24], vi[6], v[KV];
 #pragma unroll
     for (int k = 0; k < KV; ++k) v[k] = 0.f;
@@ -1512,7 +1539,7 @@ __global__ void __launch_bounds__(32 * kMWarps) coarse_point_pass9_warp(
     const int last = 31 - __clz(__match_any_sync(0xffffffffu, key));
 #pragma unroll
     for (int k = 0; k < KV; ++k) v[k] = __shfl_sync(0xffffffffu, v[k], last);
-    if (has) store_u9(u9 + kU9 * q, J + 18, v);
+    scatter_u9(u9, stages[threadIdx.x >> 5], J + 18, v, q, r.y - r.x);
 }
 
 // Point pass of S Z for points with 33 to 256 observations: a CTA takes a
@@ -1526,7 +1553,7 @@ __global__ void __launch_bounds__(kPT) coarse_point_pass9_list(
     constexpr int KV = 3 * kCoarse;
     constexpr int kMaxPts = kPT / 33 + 1;
     __shared__ int pb[kMaxPts + 1], ps[kMaxPts], pid[kMaxPts];
-    __shared__ float seg[kPT][KV + 1];
+    __shared__ __align__(16) float seg[kPT][KV + 1];
     __shared__ float wsh[kMaxPts][KV];
     const int2 lc = lchunk[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31;
@@ -1592,9 +1619,9 @@ __global__ void __launch_bounds__(kPT) coarse_point_pass9_list(
         apply_vinv(vi, w[0], w[1], w[2], w[0], w[1], w[2]);
     }
     __syncthreads();
-    if (tid < n) {
-        store_u9(u9 + static_cast<long long>(kU9) * cam_pos[sl], J + 18, wsh[key]);
-    }
+    // (seg is free again: kU9 floats per thread)
+    scatter_u9(u9, &seg[0][0] + kU9 * (tid & ~31), J + 18, wsh[max(key, 0)], tid < n ? cam_pos[sl] : 0,
+               max(0, min(32, n - (tid & ~31))));
 }
 
 // Camera pass of S Z: per camera chunk, the partials sum_e Jc_e^T u_e,j for all
