@@ -53,12 +53,15 @@ constexpr int kTileB = NB * NB * 2;           // bytes of one FP16 digit tile
 constexpr int kNS = fx::kSlices;
 
 // Workspace: digit tiles (kNS per 64-row tile), which small updates replace by the
-// panel's rows as integers (64 per row), row exponents, row flags.
+// panel's rows as integers (64 per row), row exponents, row flags, and a diagonal
+// tile of the factor per chain on its way to the matrix.
+constexpr int kMaxChains = 2;
 struct Work {
     unsigned char* tiles;
     long long* rows;
     int* e;
     int* bad;  // 1: fails at this row's pivot; 2: infinite diagonal entry
+    double* diag;
 };
 Work carve(void* ws, int n) {
     Work w;
@@ -66,6 +69,7 @@ Work carve(void* ws, int n) {
     w.rows = static_cast<long long*>(ws);
     w.e = reinterpret_cast<int*>(w.tiles + static_cast<size_t>(n / NB) * kNS * kTileB);
     w.bad = w.e + n;
+    w.diag = reinterpret_cast<double*>(w.bad + n);  // (n is a multiple of 64)
     return w;
 }
 
@@ -123,7 +127,10 @@ __global__ void __launch_bounds__(256) chol_convert(double* __restrict__ A, int 
 //
 // One CTA factors the panel's diagonal tile (every CTA of the grid does, each
 // for itself: the tile is the critical path, and the SMs would idle otherwise)
-// together with 16 rows below it, then solves the further rows it was given.
+// together with 16 rows below it, then solves the further rows it was given. No CTA
+// writes that tile of the matrix: beside other work on the GPU some CTAs start only
+// when others have ended, and read it then. Its factor goes to the workspace, and the
+// update that follows puts it in its place.
 //
 // What bounds it is the chain of 64 pivots, each a reciprocal square root and
 // three dependent 64-bit products (some 400 cycles), so one warp does nothing
@@ -429,13 +436,15 @@ __device__ void panel_output(const PanelSmem& sm, int first, int count, int r0, 
 }
 
 // rows: where the panel's rows go as integers, for chol_update_int (null: as digit tiles).
+// diag: where the diagonal tile's factor goes, column-major (null, with one CTA per
+// chain: to its place).
 // j0: first column of the panel; blockIdx.y = 1: of the second chain's, dj further on.
 __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restrict__ A, int j0, int dj, int lda,
                                                               int nbelow, int rpc, const int* __restrict__ e,
                                                               int* __restrict__ bad,
                                                               unsigned char* __restrict__ tiles,
                                                               long long* __restrict__ rows,
-                                                              int* __restrict__ info) {
+                                                              double* __restrict__ diag, int* __restrict__ info) {
     extern __shared__ __align__(16) unsigned char panel_smem[];
     PanelSmem& sm = *reinterpret_cast<PanelSmem*>(panel_smem);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -504,7 +513,10 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
             if (i < k) continue;
             double v = fx::to_double(sm.lv[i * kLvS + k], e[j0 + i]);
             if (i == k && sm.diag_bad[i] == 2) v = __longlong_as_double(0x7ff0000000000000ll);
-            A[(j0 + i) + static_cast<long long>(j0 + k) * lda] = v;
+            if (diag)
+                diag[blockIdx.y * NB * NB + t] = v;
+            else
+                A[(j0 + i) + static_cast<long long>(j0 + k) * lda] = v;
         }
     }
     // further rows, kRows2 at a time: the factor is known, four threads of a
@@ -562,6 +574,16 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
         }
         __syncthreads();
         panel_output(sm, 0, n, j0 + NB + c0, A, j0, lda, e, tiles, rows);
+    }
+}
+
+// The panel's diagonal tile from the workspace to its place at row and column j0, by
+// threads t of nthreads.
+__device__ __forceinline__ void place_diagonal(double* __restrict__ A, int j0, int lda, const double* __restrict__ diag,
+                                               int t, int nthreads) {
+    for (; t < NB * NB; t += nthreads) {
+        const int i = t & 63, k = t >> 6;
+        if (i >= k) A[(j0 + i) + static_cast<long long>(j0 + k) * lda] = diag[t];
     }
 }
 
@@ -661,7 +683,7 @@ __device__ __forceinline__ void tile_of(long long t, int* I, int* J) {
 
 __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict__ A, int j1, int dj, int nt,
                                                              long long ntiles, int lda, const unsigned char* __restrict__ tiles,
-                                                             int* __restrict__ info) {
+                                                             const double* __restrict__ diag, int* __restrict__ info) {
     extern __shared__ unsigned char upd_raw[];
     __shared__ __align__(8) unsigned long long bars[B_COUNT];
     __shared__ uint32_t tmem_base;
@@ -760,6 +782,8 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
         const int quarter = warp & 3, part = (warp - 2) >> 2;  // TMEM lanes 32 quarter .., columns 16 part ..
         const uint32_t tm = tmem + (static_cast<uint32_t>(32 * quarter) << 16) + 16 * part;
         long long* F = reinterpret_cast<long long*>(A);
+        if (blockIdx.x == 0 && !failed)  // (these warps wait for the first products)
+            place_diagonal(A, j1 - NB, lda, diag + blockIdx.y * NB * NB, tid - 64, 32 * kUpdWarps);
         for (long long t = t0; t < t1; ++t) {
             int I, J;
             tile_of(t, &I, &J);
@@ -828,17 +852,24 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
 // per thread: a tile of chol_update occupies one SM for the 112 MMAs of its 28 digit
 // products (77 cycles each) and its operands' way to shared memory, 10.4 us with the
 // launch, however few tiles there are; here they spread over all SMs. 576 rows
-// (9 panels) 380 -> 338 us.
+// (9 panels) 380 -> 338 us. One more block places the panel's diagonal tile.
 constexpr int kIntB = 16;
 __global__ void __launch_bounds__(kIntB * kIntB) chol_update_int(double* __restrict__ A, int j1, int dj, int lda,
                                                                 const long long* __restrict__ rows,
+                                                                const double* __restrict__ diag,
                                                                 const int* __restrict__ info) {
     __shared__ __align__(16) Limbs L[2][kIntB][NB + 2];
+    j1 += blockIdx.y * dj;
+    if (blockIdx.x == gridDim.x - 1) {
+        pdl_wait();
+        pdl_trigger();
+        if (!*info) place_diagonal(A, j1 - NB, lda, diag + blockIdx.y * NB * NB, threadIdx.x, kIntB * kIntB);
+        return;
+    }
     int rb = static_cast<int>((sqrtf(8.f * blockIdx.x + 1.f) - 1.f) * 0.5f);
     while (rb * (rb + 1) / 2 > static_cast<int>(blockIdx.x)) --rb;
     while ((rb + 1) * (rb + 2) / 2 <= static_cast<int>(blockIdx.x)) ++rb;
     const int cb = blockIdx.x - rb * (rb + 1) / 2;
-    j1 += blockIdx.y * dj;
     const int i = threadIdx.x & (kIntB - 1), j = threadIdx.x / kIntB;  // row, column of the block
     const int row = j1 + kIntB * rb + i, col = j1 + kIntB * cb + j;
     pdl_wait();
@@ -869,7 +900,8 @@ constexpr int kIntTiles = 12;
 }  // namespace
 
 size_t dense_potrf_workspace(int n) {
-    return static_cast<size_t>(n / NB) * kNS * kTileB + 2 * sizeof(int) * static_cast<size_t>(n);
+    return static_cast<size_t>(n / NB) * kNS * kTileB + 2 * sizeof(int) * static_cast<size_t>(n) +
+           kMaxChains * NB * NB * sizeof(double);
 }
 
 // One panel and its update for `chains` (1 or 2) chains, dj rows apart: `below` tiles below the diagonal tile of each.
@@ -881,18 +913,18 @@ static void factor_panel(double* A, int j0, int dj, int chains, int below, int l
     const int rpc = kExtra * std::max(1, ceil_div(rows * chains, kExtra * sms));
     const bool ints = below <= kIntTiles;
     launch_pdl(chol_panel, dim3(std::max(1, ceil_div(rows, rpc)), chains), kPanelThreads, sizeof(PanelSmem), s, A, j0,
-               dj, lda, rows, rpc, w.e, w.bad, w.tiles, ints ? w.rows : nullptr, info);
+               dj, lda, rows, rpc, w.e, w.bad, w.tiles, ints ? w.rows : nullptr, below ? w.diag : nullptr, info);
     if (below == 0) return;
     if (ints) {
         const int blocks = rows / kIntB;
-        launch_pdl(chol_update_int, dim3(blocks * (blocks + 1) / 2, chains), kIntB * kIntB, 0, s, A, j0 + NB, dj, lda,
-                   w.rows, info);
+        launch_pdl(chol_update_int, dim3(blocks * (blocks + 1) / 2 + 1, chains), kIntB * kIntB, 0, s, A, j0 + NB, dj,
+                   lda, w.rows, w.diag, info);
         return;
     }
     const long long pairs = below / 2;
     const long long tiles = pairs * (pairs + 1) + (below % 2 ? below : 0);
     launch_pdl(chol_update, dim3(static_cast<unsigned>(std::min<long long>(tiles, std::max(1, sms / chains))), chains),
-               kUpdThreads, kUpdSmem, s, A, j0 + NB, dj, below, tiles, lda, w.tiles, info);
+               kUpdThreads, kUpdSmem, s, A, j0 + NB, dj, below, tiles, lda, w.tiles, w.diag, info);
 }
 static void allow_smem() {
     GBA_CUDA_CHECK(cudaFuncSetAttribute(chol_panel, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(PanelSmem)));

@@ -339,7 +339,7 @@ int gba_batch_inverse3_spd(const double* A, double* Ainv, int* ok, int n, void* 
  * fixed point inside (products exact, entries rounded at 2^-60 of
  * sqrt(A_ii A_jj); closer to the exact factor than FP64 arithmetic). Replaces Eigen::LLT<MatrixXd, Lower> (reference src/lm.cu:598-603).
  * n multiple of 64, lda >= n. [device] A, info (int: 0, the failed column, or
- * negative when a bounded wait inside a kernel ran out). Workspace (0.9 n KB)
+ * negative when a bounded wait inside a kernel ran out). Workspace (0.9 n KB and 64 KB)
  * is taken from and returned to the device's memory pool on the stream. */
 int gba_dense_potrf(double* A, int n, int lda, int* info, void* stream);
 /* Solves L L^T x = b in place after gba_dense_potrf (reference src/lm.cu:604). [device] */
