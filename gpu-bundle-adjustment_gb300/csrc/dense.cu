@@ -444,7 +444,9 @@ __global__ void __launch_bounds__(256) syrk_update_quad_kernel(double* __restric
 // L_jj^-1 b_j (in every block, for itself) and the update of the block's own rows
 // (forward) or columns (backward). What bounds a step: the launch, the 64 x 64
 // product at 1.7 FMA per cycle, and the update; the operands (constant during the
-// solve) are loaded before the previous step has ended.
+// solve) are loaded before the previous step has ended. The first step is launched
+// to start when the inversion has ended: waiting inside the kernel would order only
+// the loads after the wait.
 
 // L_jj^-1 of every tile, column-major (inv) and transposed (invt): kInvCols columns
 // of X per block, X_k = (e_k - sum_m L_km X_m) / L_kk as rank-1 updates of the rows
@@ -457,7 +459,7 @@ __global__ void __launch_bounds__(kInvT) tile_inverse(const double* __restrict__
                                                      double* __restrict__ invt, const int* __restrict__ info) {
     extern __shared__ double t[];         // t[column NB + row] of L
     __shared__ double x[NB][kInvCols], rinv[NB];
-    pdl_wait();  // no early trigger: the first step reads the inverses before its own wait
+    pdl_wait();
     if (*info) return;
     const long long j0 = static_cast<long long>(blockIdx.x) * NB;
     const int r = threadIdx.x & 63, cl = threadIdx.x >> 6, first = blockIdx.y * kInvCols, c = first + cl;
@@ -650,6 +652,17 @@ static void dense_potrf_fp64(double* A, int n, int lda, int* info, cudaStream_t 
     }
 }
 
+// first: the step after tile_inverse.
+static void launch_forward(bool first, dim3 grid, const double* L, int j0, int r_end, int dj, int lda, const double* inv,
+                           double* b, double* y, const int* info, cudaStream_t s) {
+    if (first) {
+        forward_step<<<grid, kSolT, 0, s>>>(L, j0, r_end, dj, lda, inv, b, y, info);
+        GBA_LAUNCH_CHECK();
+    } else {
+        launch_pdl(forward_step, grid, kSolT, 0, s, L, j0, r_end, dj, lda, inv, b, y, info);
+    }
+}
+
 size_t dense_potrs_workspace(int n) { return (2ull * NB + 1) * n * sizeof(double); }
 
 static void invert_tiles(const double* L, int nt, int lda, double* inv, double* invt, const int* info, cudaStream_t s) {
@@ -674,7 +687,7 @@ void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* 
     for (int jb = 0; jb < nt; ++jb) {
         const int j0 = jb * NB;
         const int r_end = static_cast<int>(std::min<long long>(n, j0 + NB + (long long)bt * NB));
-        launch_pdl(forward_step, step_grid(r_end - j0 - NB, 1), kSolT, 0, s, L, j0, r_end, 0, lda, inv, b, y, info);
+        launch_forward(jb == 0, step_grid(r_end - j0 - NB, 1), L, j0, r_end, 0, lda, inv, b, y, info, s);
     }
     for (int jb = nt - 1; jb >= 0; --jb) {
         const int j0 = jb * NB, i0 = std::max(0, j0 - bt * NB);
@@ -698,12 +711,12 @@ void band_potrs_twisted(const double* F, int n, int lda, int bt, int ta, double*
     invert_tiles(F, n / NB, lda, inv, invt, info, s);  // not those of the copies
     for (int k = 0; k < std::max(ta, tb); ++k) {
         const int chains = k < ta && k < tb ? 2 : 1, j0 = k * NB + (k < ta ? 0 : base);
-        launch_pdl(forward_step, step_grid(sep, chains), kSolT, 0, s, F, j0, j0 + NB + sep, base, lda, inv, x, y, info);
+        launch_forward(k == 0, step_grid(sep, chains), F, j0, j0 + NB + sep, base, lda, inv, x, y, info, s);
     }
     launch_pdl(twist_merge_rhs, ceil_div(sep, 256), 256, 0, s, n, base, sep, x);
     for (int k = 0; k < bt; ++k) {
         const int j0 = a + k * NB;
-        launch_pdl(forward_step, step_grid(base - j0 - NB, 1), kSolT, 0, s, F, j0, base, 0, lda, inv, x, y, info);
+        launch_forward(false, step_grid(base - j0 - NB, 1), F, j0, base, 0, lda, inv, x, y, info, s);
     }
     auto columns = [&](int j0, int first) { return std::max(first, j0 - sep); };
     for (int k = bt - 1; k >= 0; --k) {

@@ -77,6 +77,31 @@ def test_two_streams_and_a_busy_gpu(gba, torch_cuda, n, bt):
         assert all(j.result() for j in jobs)
 
 
+@pytest.mark.parametrize("n", [64, 1024])
+def test_solves_with_factors_in_turn(gba, torch_cuda, n):
+    """Two factors in turn: each solve's workspace holds the inverted tiles of the other's."""
+    torch = torch_cuda
+    g = torch.Generator(device="cuda").manual_seed(n)
+    factors = []
+    for _ in range(2):
+        U = torch.triu(torch.randn(n, n, generator=g, device="cuda", dtype=torch.float64) / n**0.5)  # row j: column j
+        U.diagonal().copy_(1.0 + torch.rand(n, generator=g, device="cuda", dtype=torch.float64))
+        factors.append(U)
+    b = torch.randn(n, generator=g, device="cuda", dtype=torch.float64)
+    info = torch.zeros(1, dtype=torch.int32, device="cuda")
+    stream = torch.cuda.current_stream().cuda_stream
+    got = []
+    for k in range(100):
+        x = b.clone()
+        gba.dense_potrs(factors[k % 2].data_ptr(), n, n, x.data_ptr(), info.data_ptr(), stream)
+        got.append(x)
+    torch.cuda.synchronize()
+    assert all(torch.equal(x, got[k % 2]) for k, x in enumerate(got))
+    for U, x in zip(factors, got):
+        r = U.T @ (U @ x) - b
+        assert float(r.norm()) <= 8 * n * 2.0**-53 * float(U.norm()) ** 2 * float(x.norm())
+
+
 def test_two_solvers_in_two_threads(gba):
     """One with the dense layout, one with the band that is factored from both ends."""
     probs = [gba.synthetic_custom(200, 20000, 2, 8, 1.6, seed=4), gba.synthetic_local(400, 40000, 2, 8, 1.5, 10, seed=5)]
