@@ -29,7 +29,8 @@
 // entries count as zero, and the factorisation stops at its pivot, as FP64
 // arithmetic does at the negative or NaN pivot it meets there. An infinite
 // diagonal entry is a pivot of weight infinity: its row and column of the
-// factor are zero.
+// factor are zero (a row with an entry there that is not finite is marked, and a row of
+// infinite weight with an entry whose factor's square FP64 does not hold).
 //
 // Tile addressing: element (i, j) at A[i + j lda] in both layouts (dense.cu).
 
@@ -86,6 +87,20 @@ __global__ void chol_scale(const double* __restrict__ A, int n, int lda, int* __
     bad[i] = ok ? 0 : d > 0.0 ? 2 : 1;
 }
 
+// Entry v of a row and a column with exponents ei, ej in fixed point; inf_row, inf_col:
+// their diagonal entries are infinite.
+__device__ __forceinline__ long long convert_entry(double v, int ei, int ej, bool inf_row, bool inf_col, bool diagonal,
+                                                   bool* bad) {
+    if (!inf_row && !inf_col) return fx::to_fixed(v, ei + ej, bad);
+    if (!diagonal && v != 0.0) {
+        int x;
+        uint64_t m;
+        fx::decompose(v, &x, &m);  // x = 1024: infinite or not a number
+        *bad = x == 1024 || (!inf_col && x - ej >= 511);
+    }
+    return 0;
+}
+
 // One CTA per lower tile (ti, tj), ti - tj <= bt: FP64 -> fixed point in place.
 // The strict upper triangle of a diagonal tile is not touched.
 __global__ void __launch_bounds__(256) chol_convert(double* __restrict__ A, int nt, int lda, int bt,
@@ -104,7 +119,7 @@ __global__ void __launch_bounds__(256) chol_convert(double* __restrict__ A, int 
 #pragma unroll
     for (int k = 0; k < 16; ++k) {
         const int j = tj * NB + (threadIdx.x >> 6) + 4 * k;
-        v[k] = j <= i && bad[j] != 2 ? A[i + static_cast<long long>(j) * lda] : 0.0;
+        v[k] = j <= i ? A[i + static_cast<long long>(j) * lda] : 0.0;
         ec[k] = e[j];
     }
 #pragma unroll
@@ -112,11 +127,7 @@ __global__ void __launch_bounds__(256) chol_convert(double* __restrict__ A, int 
         const int j = tj * NB + (threadIdx.x >> 6) + 4 * k;
         if (j > i) continue;
         bool b = false;
-        long long f = fx::to_fixed(v[k], ei + ec[k], &b);
-        if (inf_row) {
-            f = 0;
-            b = false;
-        }
+        const long long f = convert_entry(v[k], ei, ec[k], inf_row, bad[j] == 2, i == j, &b);
         F[i + static_cast<long long>(j) * lda] = f;
         mine = mine || b;
     }
@@ -1010,11 +1021,7 @@ __global__ void __launch_bounds__(256) twist_convert(const double* __restrict__ 
         const int j = tj * NB + k;
         if (j > i) continue;
         bool b = false;
-        long long f = fx::to_fixed(bad[j] != 2 ? tile[k][lane_row] : 0.0, ei + e[j], &b);
-        if (inf_row) {
-            f = 0;
-            b = false;
-        }
+        const long long f = convert_entry(tile[k][lane_row], ei, e[j], inf_row, bad[j] == 2, i == j, &b);
         F[i + static_cast<long long>(j) * lda] = f;
         if (sep && i == j) dsep[i - (t.np - t.s)] = f;
         mine = mine || b;
