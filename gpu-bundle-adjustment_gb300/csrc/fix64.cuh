@@ -166,7 +166,7 @@ GBA_FX void fms_full(Acc& a, Limbs x, Limbs y) {
 GBA_FX long long value(const Acc& a) { return a.c + ((a.m + (1ll << 29)) >> 30); }
 
 // 1 / sqrt(d 2^-60) = y0 2^-24 (1 - e)^(-1/2) 2^s for d in (0, 2^60): an FP32
-// reciprocal square root, the 24-bit y0 in [2^23, 2^24) and s in [1, 30], and
+// reciprocal square root, the 24-bit y0 in [2^23, 2^24) and s in [1, 31], and
 // the deviation e = 1 - d 2^-60 (y0 2^-24 2^s)^2 (|e| < 2^-21). The series
 // 1 + e/2 + 3 e^2/8 is taken where it is applied (its next term is below
 // 2^-63): its product with the entry then waits for e alone.
@@ -214,21 +214,28 @@ GBA_FX long long mulhi_s64(long long a, long long b) {
 #endif
 }
 
-// |c| / sqrt(d) for |c| < 2^61 given rsqrt_fixed(d); *bad where the result is
-// larger than an entry of a scaled factor can be (0 is returned).
+// |c| / sqrt(d) for |c| < 2^61 given rsqrt_fixed(d), to one unit; *bad where the
+// result is larger than an entry of a scaled factor can be (0 is returned). The
+// entry is shifted by s first: of a small pivot's column, whose entries are small,
+// the product then keeps all bits.
 GBA_FX long long scale_abs(long long c, const Rsqrt& r, bool* bad) {
-    const uint64_t a = c < 0 ? 0ull - static_cast<uint64_t>(c) : static_cast<uint64_t>(c);
-    const uint64_t u = ((static_cast<uint64_t>(static_cast<uint32_t>(a >> 32)) * r.y0) << 10) +
-                       ((static_cast<uint64_t>(static_cast<uint32_t>(a)) * r.y0) >> 22);  // units of 2^-62, without 2^s
-    const long long k = mulhi_s64(static_cast<long long>(u), r.e);
-    const uint64_t k2 = (static_cast<uint64_t>(static_cast<uint32_t>(u >> 31)) * r.e2) >> 33;  // u e^2
-    const uint64_t t = u + ((3 * k2) >> 3) + static_cast<uint64_t>(k >> 1);
     const int s = r.s & 31;
-    if (t > (static_cast<uint64_t>(kBig) << 2) >> s) {
+    uint64_t a = c < 0 ? 0ull - static_cast<uint64_t>(c) : static_cast<uint64_t>(c);
+    if (a >> (61 - s)) {
         *bad = true;
         return 0;
     }
-    return static_cast<long long>(s >= 2 ? t << (s - 2) : (t + 1) >> 1);
+    a <<= s;
+    const uint64_t u = ((static_cast<uint64_t>(static_cast<uint32_t>(a >> 32)) * r.y0) << 10) +
+                       ((static_cast<uint64_t>(static_cast<uint32_t>(a)) * r.y0) >> 22);  // units of 2^-62
+    const long long k = mulhi_s64(static_cast<long long>(u), r.e);
+    const uint64_t k2 = (static_cast<uint64_t>(static_cast<uint32_t>(u >> 31)) * r.e2) >> 33;  // u e^2
+    const uint64_t t = u + ((3 * k2) >> 3) + static_cast<uint64_t>(k >> 1);
+    if (t > static_cast<uint64_t>(kBig) << 2) {
+        *bad = true;
+        return 0;
+    }
+    return static_cast<long long>((t + 3) >> 2);  // the truncations above lean by a quarter unit
 }
 GBA_FX long long scale(long long c, const Rsqrt& r, bool* bad) {
     const long long x = scale_abs(c, r, bad);
