@@ -47,7 +47,9 @@ namespace gba {
 namespace {
 
 using fx::Acc;
+using fx::Acc29;
 using fx::Limbs;
+using fx::Limbs29;
 
 constexpr int NB = 64;                        // panel width / tile size
 constexpr int kTileB = NB * NB * 2;           // bytes of one FP16 digit tile
@@ -167,10 +169,10 @@ constexpr int kLvS = NB + 1;              // stride of the row-major factor valu
 constexpr int kLS = NB + 2;               // stride of the limbs of a row (16-byte aligned)
 
 struct PanelSmem {
-    Limbs L[NB * kLS];           // [row][column] limbs of the diagonal tile's factor
-    Limbs lx[kExtra * 4];        // [row][4] limbs of the current columns, rows below the tile
-    long long xw[2][4][kWin];    // the window's columns of a round (by the round's parity)
-    long long xn[4][kOut];       // the current four columns of the other rows
+    Limbs29 L[NB * kLS];         // [row][column] limbs of the diagonal tile's factor
+    Limbs29 lx[kExtra * 4];      // [row][4] limbs of the current columns, rows below the tile
+    long long xw[2][4][kWin];    // the window's columns of a round (by the round's parity), in quarter units
+    long long xn[4][kOut];       // the current four columns of the other rows, in quarter units
     long long lv[kRows2 * kLvS]; // factor values by row, for the output
     fx::Rsqrt y[NB];             // reciprocal pivots (y0 = 0: a pivot of weight infinity)
     float rest[kWin];            // rows 32 to 63: what their squares leave of the diagonal entry
@@ -197,14 +199,15 @@ constexpr int kBarSolved = 5, kBarNext = 6, kBarHandover = 7;
 constexpr int kWindowCount = 32 + 32 * kUpdateWarps, kPivotsCount = 32 + 32 * kUpdateWarps, kPivotsSolving = 32 + 64;
 
 // Limbs of four consecutive columns.
-__device__ __forceinline__ void load_limbs4(const Limbs* p, Limbs (&l)[4]) {
+template <typename T>
+__device__ __forceinline__ void load_limbs4(const T* p, T (&l)[4]) {
     const int4 a = reinterpret_cast<const int4*>(p)[0], b = reinterpret_cast<const int4*>(p)[1];
     l[0] = {a.x, a.y};
     l[1] = {a.z, a.w};
     l[2] = {b.x, b.y};
     l[3] = {b.z, b.w};
 }
-__device__ __forceinline__ void store_limbs4(Limbs* p, const Limbs (&l)[4]) {
+__device__ __forceinline__ void store_limbs4(Limbs29* p, const Limbs29 (&l)[4]) {
     reinterpret_cast<int4*>(p)[0] = make_int4(l[0].hi, l[0].lo, l[1].hi, l[1].lo);
     reinterpret_cast<int4*>(p)[1] = make_int4(l[2].hi, l[2].lo, l[3].hi, l[3].lo);
 }
@@ -221,7 +224,7 @@ __device__ __forceinline__ void pivot_warp(PanelSmem& sm, float diag) {
     const int lane = threadIdx.x;
     float rest = diag;
     int state = sm.diag_bad[lane];  // 1: the row has failed, 2: a pivot of weight infinity
-    Limbs prev[4];
+    Limbs29 prev[4];
 #pragma unroll 1
     for (int b = 0; b < 16; ++b) {
         const int k0 = 4 * b, row = (b >> 3) * kWin + lane, p0 = k0 & (kWin - 1);
@@ -232,13 +235,13 @@ __device__ __forceinline__ void pivot_warp(PanelSmem& sm, float diag) {
             rest = sm.rest[lane];
             state = sm.diag_bad[row];
         }
-        Acc t[4];
+        Acc29 t[4];
 #pragma unroll
         for (int c = 0; c < 4; ++c) t[c] = {sm.xw[b & 1][c][lane], 0};
         if (b > 0) {  // the previous round's update of these columns
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                Limbs l[4];
+                Limbs29 l[4];
                 load_limbs4(sm.L + (k0 + c) * kLS + k0 - 4, l);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) fx::fms(t[c], prev[k], l[k]);
@@ -256,16 +259,16 @@ __device__ __forceinline__ void pivot_warp(PanelSmem& sm, float diag) {
             fx::Rsqrt y = fx::rsqrt_fixed(d);  // (of a failed pivot: not used)
             bool ob = false;
             const long long ax = fx::scale_abs(v, y, &ob);
-            const Limbs al = fx::split(ax);
+            const Limbs29 al = fx::split29(ax);
             if (c < 3) {  // the next pivot, from its lane's own entry
-                Acc dn = t[c + 1];
+                Acc29 dn = t[c + 1];
                 if (st != 2) fx::fms(dn, al, al);
                 dv = fx::value(dn);
             }
             const bool zero = st == 2 || row < k0 + c;  // (or above the diagonal of the tile)
             if (ob && !zero && state == 0) state = 1;
             x[c] = zero ? 0 : v < 0 ? -ax : ax;
-            prev[c] = zero ? Limbs{0, 0} : v < 0 ? Limbs{-al.hi, -al.lo} : al;
+            prev[c] = zero ? Limbs29{0, 0} : v < 0 ? Limbs29{-al.hi, -al.lo} : al;
             if (lane == p0 + c) {
                 if (st == 2) y.y0 = 0;
                 sm.y[k0 + c] = y;
@@ -273,7 +276,7 @@ __device__ __forceinline__ void pivot_warp(PanelSmem& sm, float diag) {
             if (!zero) sq += square_of(ax);
 #pragma unroll
             for (int r = c + 1; r < 4; ++r) {
-                Limbs l;
+                Limbs29 l;
                 l.hi = __shfl_sync(0xffffffffu, prev[c].hi, p0 + r);
                 l.lo = __shfl_sync(0xffffffffu, prev[c].lo, p0 + r);
                 fx::fms(t[r], prev[c], l);
@@ -304,7 +307,7 @@ __device__ __forceinline__ void pivot_warp(PanelSmem& sm, float diag) {
 // A solving warp: row g of the tile's rows (row >= 64: below it), a round behind the pivots.
 __device__ __forceinline__ void solving_warp(PanelSmem& sm, int g, bool live, float rest, bool* rbad) {
     bar_sync(kBarNext, kWorkers);
-    Limbs* const mine = g < NB ? sm.L + g * kLS : sm.lx + 4 * (min(g, kRows - 1) - NB);
+    Limbs29* const mine = g < NB ? sm.L + g * kLS : sm.lx + 4 * (min(g, kRows - 1) - NB);
     const int gn = min(g, kRows - 1) - kWin;
 #pragma unroll 1
     for (int b = 0; b < 16; ++b) {
@@ -312,7 +315,7 @@ __device__ __forceinline__ void solving_warp(PanelSmem& sm, int g, bool live, fl
         bar_sync(bar_pivots_solving(b), kPivotsSolving);
         if (sm.fail_round == b + 1) return;
         if (g >= NB || b < 8) {  // rows 32 to 63 are the pivot warp's from round 8 on
-            Acc t[4];
+            Acc29 t[4];
 #pragma unroll
             for (int c = 0; c < 4; ++c) t[c] = {sm.xn[c][gn], 0};
 #pragma unroll
@@ -324,7 +327,7 @@ __device__ __forceinline__ void solving_warp(PanelSmem& sm, int g, bool live, fl
                 rest -= square_of(x);
                 if (ob || rest < -0.01f) *rbad = true;
                 if (*rbad) x = 0;
-                const Limbs xl = fx::split(x);
+                const Limbs29 xl = fx::split29(x);
                 if (live) {
                     (g < NB ? mine + k : mine + c)[0] = xl;
                     sm.lv[g * kLvS + k] = x;
@@ -350,12 +353,12 @@ __device__ __forceinline__ void solving_warp(PanelSmem& sm, int g, bool live, fl
 }
 
 // An updating warp: the thread's row g and columns 4 m + q.
-__device__ __forceinline__ void updating_warp(PanelSmem& sm, Acc (&a)[16], int g, int q) {
+__device__ __forceinline__ void updating_warp(PanelSmem& sm, Acc29 (&a)[16], int g, int q) {
     if (g < kWin) {
-        sm.xw[0][q][g] = a[0].c;
-        sm.xw[1][q][g] = a[1].c;
+        sm.xw[0][q][g] = fx::quarters(a[0]);
+        sm.xw[1][q][g] = fx::quarters(a[1]);
     } else {
-        sm.xn[q][g - kWin] = a[0].c;
+        sm.xn[q][g - kWin] = fx::quarters(a[0]);
     }
     bar_arrive(bar_window(0), kWindowCount);
     bar_arrive(bar_window(1), kWindowCount);
@@ -365,10 +368,10 @@ __device__ __forceinline__ void updating_warp(PanelSmem& sm, Acc (&a)[16], int g
     for (int b = 0; b < 16; ++b) {
         const int k0 = 4 * b, w0 = (b >> 3) * kWin, w1 = w0 + kWin;  // the window's rows
         const bool window = gw >= w0 && gw < w1, outside = gw >= w1;
-        const Limbs* const col = sm.L + (k0 + q) * kLS + k0;  // limbs of row k0 + q, columns k0 ..
+        const Limbs29* const col = sm.L + (k0 + q) * kLS + k0;  // limbs of row k0 + q, columns k0 ..
         bar_sync(bar_pivots(b), kPivotsCount);
         if (sm.fail_round == b + 1) return;
-        Limbs xr[4], l[4];
+        Limbs29 xr[4], l[4];
         // the window's columns two rounds ahead (those of the next round are the pivot warp's)
         if (window) {
             load_limbs4(sm.L + g * kLS + k0, xr);
@@ -376,7 +379,7 @@ __device__ __forceinline__ void updating_warp(PanelSmem& sm, Acc (&a)[16], int g
                 load_limbs4(col + 8 * kLS, l);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) fx::fms(a[2], xr[c], l[c]);
-                sm.xw[b & 1][q][g - w0] = fx::value(a[2]);
+                sm.xw[b & 1][q][g - w0] = fx::quarters(a[2]);
             }
         }
         if (b <= 13 && b != 6 && b != 7) bar_arrive(bar_window(b + 2), kWindowCount);
@@ -392,8 +395,8 @@ __device__ __forceinline__ void updating_warp(PanelSmem& sm, Acc (&a)[16], int g
 #pragma unroll
                 for (int c = 0; c < 4; ++c) fx::fms(a[m], xr[c], l[c]);
             }
-            sm.xn[q][g - kWin] = fx::value(a[1]);
-            if (g < NB && (b == 6 || b == 7)) sm.xw[b & 1][q][g - kWin] = fx::value(a[2]);
+            sm.xn[q][g - kWin] = fx::quarters(a[1]);
+            if (g < NB && (b == 6 || b == 7)) sm.xw[b & 1][q][g - kWin] = fx::quarters(a[2]);
         }
         if (b == 6 || b == 7) bar_arrive(bar_window(b + 2), kWindowCount);
         bar_arrive(kBarNext, kWorkers);
@@ -494,12 +497,11 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
     } else if (worker < kUpdateWarps) {
         const int g = 8 * worker + (lane >> 2), q = lane & 3;
         const bool live = g < NB || g - NB < nx;
-        Acc a[16];
+        Acc29 a[16];
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
             const int j = 4 * m + q;
-            a[m].c = live && (g >= NB || j <= g) ? F[matrix_row(g) + static_cast<long long>(j0 + j) * lda] : 0;
-            a[m].m = 0;
+            a[m] = fx::acc29(live && (g >= NB || j <= g) ? F[matrix_row(g) + static_cast<long long>(j0 + j) * lda] : 0);
         }
         updating_warp(sm, a, g, q);
     } else {
@@ -540,17 +542,14 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
         bool rb = lv ? bad[r] == 1 : true;
         float rs = lv ? static_cast<float>(F[r + static_cast<long long>(r) * lda]) * 0x1p-60f : 0.f;
         if (lv && bad[r] == 2) rs = 1.f;
-        Acc a[16];
+        Acc29 a[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) {
-            a[m].c = lv ? F[r + static_cast<long long>(j0 + 4 * m + q) * lda] : 0;
-            a[m].m = 0;
-        }
+        for (int m = 0; m < 16; ++m) a[m] = fx::acc29(lv ? F[r + static_cast<long long>(j0 + 4 * m + q) * lda] : 0);
         __syncthreads();  // sm.lv of the previous rows has been written out
         if (8 * warp < n) {
             for (int b = 0; b < 16; ++b) {
                 const int k0 = 4 * b;
-                Limbs xl[4], l[4];
+                Limbs29 xl[4], l[4];
                 load_limbs4(sm.L + (k0 + q) * kLS + k0, l);
 #pragma unroll
                 for (int c = 0; c < 4; ++c) {
@@ -561,11 +560,11 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
                         x = fx::scale(fx::value(a[0]), y, &ob);
                         if (ob || rb || y.y0 == 0) x = 0;
                     }
-                    const Limbs mine = fx::split(x);
+                    const Limbs29 mine = fx::split29(x);
                     xl[c].hi = __shfl_sync(0xffffffffu, mine.hi, c, 4);
                     xl[c].lo = __shfl_sync(0xffffffffu, mine.lo, c, 4);
                     rb = __shfl_sync(0xffffffffu, ob ? 1 : 0, c, 4) || rb;
-                    const float xf = static_cast<float>(xl[c].hi) * 0x1p-30f;
+                    const float xf = static_cast<float>(xl[c].hi) * 0x1p-31f;
                     rs = fmaf(-xf, xf, rs);
                     if (rs < -0.01f) rb = true;
                     if (q == c) sm.lv[g * kLvS + k0 + c] = x;

@@ -139,8 +139,7 @@ GBA_FX double to_double(long long v, int e) {
 // Products: v = hi 2^30 + lo, lo in [-2^29, 2^29). The product of two entries,
 // in units of 2^-60, is hi hi' + (hi lo' + lo hi' + lo lo' 2^-30) 2^-30: sums keep the
 // two parts in two 64-bit accumulators. lo lo' is below a quarter unit: fms leaves it
-// out (within a panel, whose rounds wait for one another: an entry takes at most 63
-// such products), fms_full takes it from the upper halves of the factors.
+// out, fms_full takes it from the upper halves of the factors.
 struct Limbs {
     int hi, lo;
 };
@@ -164,6 +163,35 @@ GBA_FX void fms_full(Acc& a, Limbs x, Limbs y) {
     a.m += static_cast<long long>(-x.lo >> 15) * (y.lo >> 15);
 }
 GBA_FX long long value(const Acc& a) { return a.c + ((a.m + (1ll << 29)) >> 30); }
+
+// The same within a panel, whose rounds wait for one another: split at 2^29, so that
+// lo lo', left out, is below a 16th of a unit (of the 63 squares subtracted from a
+// diagonal entry it is 1.3 units together; split at 2^30 5.3, and the solution's
+// error at condition 4e3 three times as large). 4,096 unknowns 4.76 -> 4.84 ms; 5.03
+// with fms_full.
+// The sums are kept, and passed on, in quarter units: entries below 2^61, their
+// products' sums as well; of m, at most 2^62.5 (Cauchy-Schwarz over 64 columns).
+struct Limbs29 {
+    int hi, lo;  // v = hi 2^29 + lo, lo in [-2^28, 2^28)
+};
+GBA_FX Limbs29 split29(long long v) {
+    Limbs29 l;
+    l.lo = static_cast<int>(static_cast<uint32_t>(static_cast<uint64_t>(v)) << 3) >> 3;
+    l.hi = static_cast<int>((v - l.lo) >> 29);
+    return l;
+}
+struct Acc29 {
+    long long c, m;  // (c + m 2^-29) / 4
+};
+GBA_FX Acc29 acc29(long long v) { return {v * 4, 0}; }
+GBA_FX void fms(Acc29& a, Limbs29 x, Limbs29 y) {  // a -= x y
+    const int nh = -x.hi, nl = -x.lo;
+    a.c += static_cast<long long>(nh) * y.hi;
+    a.m += static_cast<long long>(nh) * y.lo;
+    a.m += static_cast<long long>(nl) * y.hi;
+}
+GBA_FX long long quarters(const Acc29& a) { return a.c + ((a.m + (1ll << 28)) >> 29); }
+GBA_FX long long value(const Acc29& a) { return (a.c + ((a.m + (1ll << 30)) >> 29)) >> 2; }  // to nearest
 
 // 1 / sqrt(d 2^-60) = y0 2^-24 (1 - e)^(-1/2) 2^s for d in (0, 2^60): an FP32
 // reciprocal square root, the 24-bit y0 in [2^23, 2^24) and s in [1, 31], and
