@@ -441,22 +441,36 @@ __global__ void __launch_bounds__(256) syrk_update_quad_kernel(double* __restric
 // FP64 instructions each, and GB300 issues one per warp every 64 cycles: 27 us a
 // tile. So the diagonal tiles are inverted first, all at once (tile_inverse),
 // and the substitution through the tiles is then one kernel per tile: x_j =
-// L_jj^-1 b_j (in every block, for itself) and the update of the block's own rows
-// (forward) or columns (backward). What bounds a step: the launch, the 64 x 64
-// product at 1.7 FMA per cycle, and the update; the operands (constant during the
-// solve) are loaded before the previous step has ended. The first step is launched
-// to start when the inversion has ended: waiting inside the kernel would order only
-// the loads after the wait.
+// L_jj^-1 b_j, refined once with the residual b_j - L_jj x_j (in every block, for
+// itself), and the update of the block's own rows (forward) or columns (backward).
+// Without the refinement a tile's backward error is four times that of the
+// substitution (1.7 against 0.4 u |L||x|); with it, the same. What bounds a step: the
+// launch, the three 64 x 64 products at 1.7 FMA per cycle, and the update; the
+// operands (constant during the solve) are loaded before the previous step has ended.
+// The first step is launched to start when the inversion has ended: waiting inside the
+// kernel would order only the loads after the wait.
 
-// L_jj^-1 of every tile, column-major (inv) and transposed (invt): kInvCols columns
-// of X per block, X_k = (e_k - sum_m L_km X_m) / L_kk as rank-1 updates of the rows
-// below, one entry per thread. Bound by the 64 dependent steps (a product, a barrier
-// and the update, whose FP64 instructions the warps of a sub-partition take in
-// turn): one tile per block with its rows and columns in turn took 60 us, 12 us so.
+// A lower-triangular tile packed for its products with a vector: rows p and 63 - p have 65
+// entries together, held in order (row p's first) by lane p, one per 32 places.
+constexpr int kPacked = 65 * 32;
+__device__ __forceinline__ int packed_at(int i, int k) {  // i >= k
+    return i < 32 ? 32 * k + i : 32 * (k + 64 - i) + 63 - i;
+}
+// Per tile: its inverse and itself, and the same with rows and columns reversed and
+// transposed (the upper triangle of the transpose as a lower one).
+struct PackedTile {
+    double inv[kPacked], tile[kPacked], inv_t[kPacked], tile_t[kPacked];
+};
+
+// L_jj^-1 and L_jj of every tile, packed: kInvCols columns X of the inverse per block,
+// X_k = (e_k - sum_m L_km X_m) / L_kk as rank-1 updates of the rows below, one entry per
+// thread. Bound by the 64 dependent steps (a product, a barrier and the update, whose
+// FP64 instructions the warps of a sub-partition take in turn): one tile per block with
+// its rows and columns in turn took 60 us, 12 us so.
 constexpr int kInvCols = 8;
 constexpr int kInvT = NB * kInvCols;
-__global__ void __launch_bounds__(kInvT) tile_inverse(const double* __restrict__ L, int lda, double* __restrict__ inv,
-                                                     double* __restrict__ invt, const int* __restrict__ info) {
+__global__ void __launch_bounds__(kInvT) tile_inverse(const double* __restrict__ L, int lda,
+                                                     PackedTile* __restrict__ out, const int* __restrict__ info) {
     extern __shared__ double t[];         // t[column NB + row] of L
     __shared__ double x[NB][kInvCols], rinv[NB];
     pdl_wait();
@@ -472,40 +486,66 @@ __global__ void __launch_bounds__(kInvT) tile_inverse(const double* __restrict__
         __syncthreads();
         if ((r | 31) > k && r > k) v -= t[NB * k + r] * x[k][cl];
     }
-    if (r < first) v = 0.0;
-    inv[j0 * NB + NB * c + r] = v;
-    __syncthreads();
-    // transposed: row c of invt's tile is column c of the inverse
-    x[r][cl] = v;
-    __syncthreads();
-    const int cc = threadIdx.x & (kInvCols - 1), rr = threadIdx.x / kInvCols;
-    invt[j0 * NB + NB * rr + first + cc] = x[rr][cc];
+    if (r < c) return;
+    PackedTile& o = out[blockIdx.x];
+    double l = t[NB * c + r];
+    if (r == c && isinf(l)) l = 0.0;  // weight infinity: x is 0 there, and so is its part of a residual
+    const int at = packed_at(r, c), at_t = packed_at(63 - c, 63 - r);
+    o.inv[at] = v;
+    o.tile[at] = l;
+    o.inv_t[at_t] = v;
+    o.tile_t[at_t] = l;
 }
 
-// x = M b for a 64 x 64 tile M (column-major, 0 outside the triangle): 256
-// threads, thread (row, g) sums columns g, g + 4, ... with non-zeros (m, loaded
-// by load_tile_cols); b and x in shared memory, part: 4 x 64 doubles.
-__device__ __forceinline__ bool tile_col_used(bool lower, int r, int c) {
-    return lower ? c <= (r | 31) : c >= (r & 32);  // uniform over a warp
-}
-template <bool kLower>
-__device__ __forceinline__ void load_tile_cols(const double* __restrict__ M, double (&m)[16]) {
-    const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
+// Products of packed tiles with a vector in shared memory, by the first four warps: lane
+// p of warp q takes every fourth of its two rows' entries (17 FMAs; a thread per row
+// and group of columns, with the zeros that share a warp with entries, 32).
+constexpr int kPairT = 128, kPairN = 17;
+__device__ __forceinline__ void load_packed(const double* __restrict__ M, double (&m)[kPairN]) {
+    const int p = threadIdx.x & 31, q = threadIdx.x >> 5;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) m[i] = tile_col_used(kLower, r, g + 4 * i) ? M[r + NB * (g + 4 * i)] : 0.0;
+    for (int i = 0; i < kPairN; ++i) m[i] = q < 4 && q + 4 * i < 65 ? M[32 * (q + 4 * i) + p] : 0.0;
 }
-template <bool kLower>
-__device__ __forceinline__ void tile_product(const double (&m)[16], const double* b, double (*part)[NB], double* x) {
-    const int r = threadIdx.x & 63, g = threadIdx.x >> 6;
-    double s0 = 0.0, s1 = 0.0;
+__device__ __forceinline__ void pair_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+// Row r of M b, for threads r < 64 (all four warps call it).
+__device__ __forceinline__ double packed_row(const double (&m)[kPairN], const double* b, double (*part)[NB]) {
+    const int p = threadIdx.x & 31, q = threadIdx.x >> 5;
+    double s = 0.0, upper = 0.0;  // row 63 - p, row p
 #pragma unroll
-    for (int i = 0; i < 16; i += 2) {
-        if (tile_col_used(kLower, r, g + 4 * i)) s0 = fma(m[i], b[g + 4 * i], s0);
-        if (tile_col_used(kLower, r, g + 4 * i + 4)) s1 = fma(m[i + 1], b[g + 4 * i + 4], s1);
+    for (int i = 0; i < kPairN; ++i) {
+        const int e = q + 4 * i;
+        if (e >= 65) continue;
+        if (e > p && e - 4 <= p) {
+            upper = s;
+            s = 0.0;
+        }
+        s = fma(m[i], b[e > p ? e - p - 1 : e], s);
     }
-    part[g][r] = s0 + s1;
-    __syncthreads();
-    if (threadIdx.x < NB) x[r] = (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+    part[q][p] = upper;
+    part[q][63 - p] = s;
+    pair_sync();
+    const int r = threadIdx.x & 63;
+    return (part[0][r] + part[1][r]) + (part[2][r] + part[3][r]);
+}
+struct TileShared {
+    double part[4][NB], b[NB], x[NB];
+};
+// x = T^-1 b (sm.b, overwritten) with T's inverse m and T itself (t), refined once.
+// kReversed: b's rows and those of T are in reverse order, x's are not.
+template <bool kReversed>
+__device__ __forceinline__ void tile_solve(const double (&m)[kPairN], const double (&t)[kPairN], TileShared& sm,
+                                           double* x) {
+    if (threadIdx.x < kPairT) {
+        const int r = threadIdx.x;
+        const double x1 = packed_row(m, sm.b, sm.part);
+        if (r < NB) sm.x[r] = x1;
+        pair_sync();
+        const double ax = packed_row(t, sm.x, sm.part);
+        if (r < NB) sm.b[r] -= ax;
+        pair_sync();
+        const double v = x1 + packed_row(m, sm.b, sm.part);
+        if (r < NB) x[kReversed ? 63 - r : r] = isfinite(v) ? v : x1;  // (x1 out of range: no residual)
+    }
     __syncthreads();
 }
 
@@ -515,14 +555,16 @@ constexpr int kSolRows = 16;  // rows (columns) of L per pass of a block
 // Forward step j: y_j = L_jj^-1 b_j, b[j0 + 64 : r_end) -= L[.., j] y_j.
 // blockIdx.y = 1: the second chain's tile, dj rows further on.
 __global__ void __launch_bounds__(kSolT) forward_step(const double* __restrict__ L, int j0, int r_end, int dj, int lda,
-                                                     const double* __restrict__ inv, double* __restrict__ b,
+                                                     const PackedTile* __restrict__ tiles, double* __restrict__ b,
                                                      double* __restrict__ y, const int* __restrict__ info) {
-    __shared__ double part[4][NB], bs[NB], x[NB], red[kSolRows][kSolT / kSolRows + 1];
+    __shared__ TileShared sm;
+    __shared__ double x[NB], red[kSolRows][kSolT / kSolRows + 1];
     const int lr = threadIdx.x & (kSolRows - 1), kg = threadIdx.x / kSolRows;  // row, group of four columns
     j0 += blockIdx.y * dj;
     r_end += blockIdx.y * dj;
-    double m[16], l[4] = {0.0, 0.0, 0.0, 0.0};
-    load_tile_cols<true>(inv + static_cast<long long>(j0) * NB, m);
+    double m[kPairN], t[kPairN], l[4] = {0.0, 0.0, 0.0, 0.0};
+    load_packed(tiles[j0 / NB].inv, m);
+    load_packed(tiles[j0 / NB].tile, t);
     int r = j0 + NB + blockIdx.x * kSolRows + lr;
     if (r < r_end) {
 #pragma unroll
@@ -531,9 +573,9 @@ __global__ void __launch_bounds__(kSolT) forward_step(const double* __restrict__
     pdl_wait();
     pdl_trigger();
     if (*info) return;
-    if (threadIdx.x < NB) bs[threadIdx.x] = b[j0 + threadIdx.x];
+    if (threadIdx.x < NB) sm.b[threadIdx.x] = b[j0 + threadIdx.x];
     __syncthreads();
-    tile_product<true>(m, bs, part, x);
+    tile_solve<false>(m, t, sm, x);
     if (blockIdx.x == 0 && threadIdx.x < NB) y[j0 + threadIdx.x] = x[threadIdx.x];
     for (int base = j0 + NB + blockIdx.x * kSolRows; base < r_end; base += gridDim.x * kSolRows) {
         const int nr = base + gridDim.x * kSolRows + lr;
@@ -559,14 +601,19 @@ struct BackwardTile {
     int j0, i0, i1, known;
 };
 __global__ void __launch_bounds__(kSolT) backward_step(const double* __restrict__ L, BackwardTile t0, BackwardTile t1,
-                                                      int lda, const double* __restrict__ invt, double* __restrict__ y,
-                                                      double* __restrict__ b, const int* __restrict__ info) {
-    __shared__ double part[4][NB], bs[NB], x[NB];
+                                                      int lda, const PackedTile* __restrict__ tiles,
+                                                      double* __restrict__ y, double* __restrict__ b,
+                                                      const int* __restrict__ info) {
+    __shared__ TileShared sm;
+    __shared__ double x[NB];
     const int kg = threadIdx.x & 15, lc = threadIdx.x >> 4;  // group of four rows, column
     const BackwardTile t = blockIdx.y ? t1 : t0;
     const int j0 = t.j0;
-    double m[16], l[4] = {0.0, 0.0, 0.0, 0.0};
-    if (t.known < 0) load_tile_cols<false>(invt + static_cast<long long>(j0) * NB, m);
+    double m[kPairN], d[kPairN], l[4] = {0.0, 0.0, 0.0, 0.0};
+    if (t.known < 0) {
+        load_packed(tiles[j0 / NB].inv_t, m);
+        load_packed(tiles[j0 / NB].tile_t, d);
+    }
     int c = t.i0 + blockIdx.x * kSolRows + lc;
     if (c < t.i1) {
 #pragma unroll
@@ -579,9 +626,9 @@ __global__ void __launch_bounds__(kSolT) backward_step(const double* __restrict_
         if (threadIdx.x < NB) x[threadIdx.x] = b[t.known - threadIdx.x];
         __syncthreads();
     } else {
-        if (threadIdx.x < NB) bs[threadIdx.x] = y[j0 + threadIdx.x];
+        if (threadIdx.x < NB) sm.b[63 - threadIdx.x] = y[j0 + threadIdx.x];
         __syncthreads();
-        tile_product<false>(m, bs, part, x);
+        tile_solve<true>(m, d, sm, x);
         if (blockIdx.x == 0 && threadIdx.x < NB) b[j0 + threadIdx.x] = x[threadIdx.x];
     }
     for (; c - lc < t.i1; c += gridDim.x * kSolRows) {
@@ -653,20 +700,26 @@ static void dense_potrf_fp64(double* A, int n, int lda, int* info, cudaStream_t 
 }
 
 // first: the step after tile_inverse.
-static void launch_forward(bool first, dim3 grid, const double* L, int j0, int r_end, int dj, int lda, const double* inv,
-                           double* b, double* y, const int* info, cudaStream_t s) {
+static void launch_forward(bool first, dim3 grid, const double* L, int j0, int r_end, int dj, int lda,
+                           const PackedTile* tiles, double* b, double* y, const int* info, cudaStream_t s) {
     if (first) {
-        forward_step<<<grid, kSolT, 0, s>>>(L, j0, r_end, dj, lda, inv, b, y, info);
+        forward_step<<<grid, kSolT, 0, s>>>(L, j0, r_end, dj, lda, tiles, b, y, info);
         GBA_LAUNCH_CHECK();
     } else {
-        launch_pdl(forward_step, grid, kSolT, 0, s, L, j0, r_end, dj, lda, inv, b, y, info);
+        launch_pdl(forward_step, grid, kSolT, 0, s, L, j0, r_end, dj, lda, tiles, b, y, info);
     }
 }
 
-size_t dense_potrs_workspace(int n) { return (2ull * NB + 1) * n * sizeof(double); }
+// Of n rows: the packed tiles and a vector.
+struct SolveWork {
+    PackedTile* tiles;
+    double* y;
+    SolveWork(void* ws, int n) : tiles(static_cast<PackedTile*>(ws)), y(reinterpret_cast<double*>(tiles + n / NB)) {}
+};
+size_t dense_potrs_workspace(int n) { return n / NB * sizeof(PackedTile) + n * sizeof(double); }
 
-static void invert_tiles(const double* L, int nt, int lda, double* inv, double* invt, const int* info, cudaStream_t s) {
-    launch_pdl(tile_inverse, dim3(nt, NB / kInvCols), kInvT, NB * NB * sizeof(double), s, L, lda, inv, invt, info);
+static void invert_tiles(const double* L, int nt, int lda, const SolveWork& w, const int* info, cudaStream_t s) {
+    launch_pdl(tile_inverse, dim3(nt, NB / kInvCols), kInvT, NB * NB * sizeof(double), s, L, lda, w.tiles, info);
 }
 // Blocks of a step over `rows` rows (columns) of each chain. Two passes of a block at
 // most where the rows allow it: a further pass costs a block less than a further block
@@ -680,19 +733,17 @@ void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* 
     if (n % NB != 0 || bt < 0 || (bt < n / NB - 1 ? lda + 1 < (bt + 2) * NB : lda < n))
         throw std::invalid_argument("dense_potrs: n must be a multiple of 64 and lda hold the band");
     const int nt = n / NB;
-    double* inv = static_cast<double*>(workspace);
-    double* invt = inv + static_cast<size_t>(NB) * n;
-    double* y = invt + static_cast<size_t>(NB) * n;
-    invert_tiles(L, nt, lda, inv, invt, info, s);
+    const SolveWork w(workspace, n);
+    invert_tiles(L, nt, lda, w, info, s);
     for (int jb = 0; jb < nt; ++jb) {
         const int j0 = jb * NB;
         const int r_end = static_cast<int>(std::min<long long>(n, j0 + NB + (long long)bt * NB));
-        launch_forward(jb == 0, step_grid(r_end - j0 - NB, 1), L, j0, r_end, 0, lda, inv, b, y, info, s);
+        launch_forward(jb == 0, step_grid(r_end - j0 - NB, 1), L, j0, r_end, 0, lda, w.tiles, b, w.y, info, s);
     }
     for (int jb = nt - 1; jb >= 0; --jb) {
         const int j0 = jb * NB, i0 = std::max(0, j0 - bt * NB);
         const BackwardTile t{j0, i0, j0, -1};
-        launch_pdl(backward_step, step_grid(j0 - i0, 1), kSolT, 0, s, L, t, t, lda, invt, y, b, info);
+        launch_pdl(backward_step, step_grid(j0 - i0, 1), kSolT, 0, s, L, t, t, lda, w.tiles, w.y, b, info);
     }
 }
 
@@ -703,26 +754,24 @@ size_t band_twist_solve_workspace(int n, int bt) {
 void band_potrs_twisted(const double* F, int n, int lda, int bt, int ta, double* b, const int* info, void* workspace,
                         cudaStream_t s) {
     const int np = n + bt * NB, sep = bt * NB, a = ta * NB, base = a + sep, tb = n / NB - ta - bt;
-    double* inv = static_cast<double*>(workspace);
-    double* invt = inv + static_cast<size_t>(NB) * np;
-    double* y = invt + static_cast<size_t>(NB) * np;
-    double* x = y + np;
+    const SolveWork w(workspace, np);
+    double* x = w.y + np;
     launch_pdl(twist_rhs, ceil_div(np, 256), 256, 0, s, b, n, base, sep, x);
-    invert_tiles(F, n / NB, lda, inv, invt, info, s);  // not those of the copies
+    invert_tiles(F, n / NB, lda, w, info, s);  // not those of the copies
     for (int k = 0; k < std::max(ta, tb); ++k) {
         const int chains = k < ta && k < tb ? 2 : 1, j0 = k * NB + (k < ta ? 0 : base);
-        launch_forward(k == 0, step_grid(sep, chains), F, j0, j0 + NB + sep, base, lda, inv, x, y, info, s);
+        launch_forward(k == 0, step_grid(sep, chains), F, j0, j0 + NB + sep, base, lda, w.tiles, x, w.y, info, s);
     }
     launch_pdl(twist_merge_rhs, ceil_div(sep, 256), 256, 0, s, n, base, sep, x);
     for (int k = 0; k < bt; ++k) {
         const int j0 = a + k * NB;
-        launch_forward(false, step_grid(base - j0 - NB, 1), F, j0, base, 0, lda, inv, x, y, info, s);
+        launch_forward(false, step_grid(base - j0 - NB, 1), F, j0, base, 0, lda, w.tiles, x, w.y, info, s);
     }
     auto columns = [&](int j0, int first) { return std::max(first, j0 - sep); };
     for (int k = bt - 1; k >= 0; --k) {
         const int j0 = a + k * NB, i0 = columns(j0, 0);
         const BackwardTile t{j0, i0, j0, -1};
-        launch_pdl(backward_step, step_grid(j0 - i0, 1), kSolT, 0, s, F, t, t, lda, invt, y, x, info);
+        launch_pdl(backward_step, step_grid(j0 - i0, 1), kSolT, 0, s, F, t, t, lda, w.tiles, w.y, x, info);
     }
     // chain 0's tiles above, beside chain 1's: the rows between (known now), then its own
     for (int k = 0; k < std::max(ta, tb + bt); ++k) {
@@ -737,7 +786,8 @@ void band_potrs_twisted(const double* F, int n, int lda, int bt, int ta, double*
             // row j0 + i of chain 1 is row base + n - 1 - j0 - i of the band
             t[m++] = {j0, columns(j0, base), std::min(j0, n), k < bt ? base + n - 1 - j0 : -1};
         }
-        launch_pdl(backward_step, step_grid(sep, m), kSolT, 0, s, F, t[0], t[m - 1], lda, invt, y, x, info);
+        launch_pdl(backward_step, step_grid(sep, m), kSolT, 0, s, F, t[0], t[m - 1], lda, w.tiles, w.y, x,
+                   info);
     }
     launch_pdl(twist_solution, ceil_div(n, 256), 256, 0, s, x, n, base, info, b);
 }
