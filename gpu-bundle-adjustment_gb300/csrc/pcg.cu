@@ -40,6 +40,7 @@
 #include <cuda_bf16.h>
 
 #include "blocks.cuh"
+#include "cluster_sums.cuh"
 #include "common.cuh"
 #include "ff.cuh"
 #include "mlp.hpp"
@@ -1916,13 +1917,11 @@ __global__ void __launch_bounds__(kVT) pcg_direction(float* __restrict__ p32, co
 // 9-vectors per camera; between them stand only sums over all cameras. One
 // cluster of CTAs (16, or 8 where 16 do not fit a device) owns all cameras, `per`
 // consecutive ones per CTA, and takes those sums through distributed shared
-// memory: every CTA sends its partial to every other, one cluster barrier, and
-// all add the partials in the same order. FP64 instructions hold their warp's
-// scheduler for 64 cycles on this chip, so only single warps take the FP64
-// sums, and one thread the scalars.
+// memory (cluster_sums.cuh); one thread takes the scalars.
 constexpr int kTailMaxT = 1024;
-constexpr int kTailMinT = 128;   // four warps: the sums' roles below
-constexpr int kTailMaxCtas = 16;
+constexpr int kTailMinT = 128;   // four warps: the sums' roles
+constexpr int kTailMaxCtas = csum::kMaxCtas;
+static_assert(csum::kNine == kCoarse, "one sum per coarse basis column");
 // Two 9-vectors of a CTA's cameras in shared memory, also with 8 CTAs. Below, an
 // iteration (with its product) takes, separate kernels -> this one, block-Jacobi and
 // learned: 60 cameras 15.9 -> 12.5 and 10.6 -> 7.9 us; 500 18.3 -> 14.1, 19.4 -> 14.1;
@@ -1930,96 +1929,12 @@ constexpr int kTailMaxCtas = 16;
 constexpr int kTailMaxC = 24000;
 
 struct TailShared {
-    double slot[4][10][kTailMaxCtas];  // partials of each CTA, for the four sums
-    double tot[10];
-    float wp[10][33];                  // warp sums
+    csum::Shared sums;
     float cf[kCoarse];                 // coarse coefficients
     double c1[kCoarse];
     float scalar;                      // alpha, then beta
     int done;                          // the S_DONE value of this iteration
 };
-
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// Store v at `local`'s place in the shared memory of CTA `rank` of the cluster.
-__device__ __forceinline__ void cluster_store(double* local, int rank, double v) {
-    uint32_t a;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(local))), "r"(rank));
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-
-// Totals over the cluster of NS <= 2 scalars (v[0 .. NS)) and, with kNine, of nine
-// coarse sums (v[NS .. NS + 9), into sm.tot). fin(t0, t1) runs in thread 0 with
-// the scalars' totals; what it writes to sm is visible to every thread on return.
-// Warp sums in FP32; then FP64: a scalar's warps on one warp (warp j for scalar
-// j), the nine sums on four lanes each of warps 2 and 3 (runs of eight warps
-// added in FP32 first), then the CTAs' partials the same way.
-template <int NS, bool kNine, class Fin>
-__device__ __forceinline__ void cluster_totals(const float* v, TailShared& sm, int which, int rank, int nctas, Fin fin) {
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nw = blockDim.x >> 5;
-    double(&slot)[10][kTailMaxCtas] = sm.slot[which];
-#pragma unroll
-    for (int j = 0; j < NS; ++j) {
-        const float t = warp_sum(v[j]);
-        if (lane == 0) sm.wp[j][warp] = t;
-    }
-    if constexpr (kNine) {
-        // halve the values and the lanes that hold them: lane l ends with sum l / 2
-        float a[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) a[j] = j < kCoarse ? v[NS + j] : 0.f;
-#pragma unroll
-        for (int o = 16, h = 8; h >= 1; o >>= 1, h >>= 1) {
-            const bool up = lane & o;
-#pragma unroll
-            for (int j = 0; j < h; ++j) {
-                const float keep = up ? a[j + h] : a[j], send = up ? a[j] : a[j + h];
-                a[j] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-            }
-        }
-        a[0] += __shfl_xor_sync(0xffffffffu, a[0], 1);
-        if (!(lane & 1) && lane < 2 * kCoarse) sm.wp[NS + (lane >> 1)][warp] = a[0];
-    }
-    __syncthreads();
-    if (warp < NS) {
-        double d = lane < nw ? static_cast<double>(sm.wp[warp][lane]) : 0.0;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        if (lane < nctas) cluster_store(&slot[warp][rank], lane, d);
-    }
-    const int j9 = NS + ((tid - 64) >> 2), g = tid & 3;
-    const bool nine = kNine && (warp == 2 || warp == 3);
-    if (nine) {
-        float f = 0.f;
-        if (j9 < NS + kCoarse)
-            for (int w = 8 * g; w < min(8 * g + 8, nw); ++w) f += sm.wp[j9][w];
-        double d = static_cast<double>(f);
-        d += __shfl_xor_sync(0xffffffffu, d, 1);
-        d += __shfl_xor_sync(0xffffffffu, d, 2);
-        if (j9 < NS + kCoarse)
-            for (int c = g; c < nctas; c += 4) cluster_store(&slot[j9][rank], c, d);
-    }
-    __syncwarp();
-    cluster_arrive();
-    cluster_wait();
-    if (NS > 0 && warp == 0) {  // scalar 0 on the lower lanes, scalar 1 on the upper ones
-        const int c = lane & 15;
-        double d = c < nctas && (NS == 2 || lane < 16) ? slot[lane >> 4][c] : 0.0;
-#pragma unroll
-        for (int o = 8; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-        const double d1 = NS == 2 ? __shfl_sync(0xffffffffu, d, 16) : 0.0;
-        if (lane == 0) fin(d, d1);
-    }
-    if (nine) {
-        double d = 0.0;
-        if (j9 < NS + kCoarse)
-            for (int c = g; c < nctas; c += 4) d += slot[j9][c];
-        d += __shfl_xor_sync(0xffffffffu, d, 1);
-        d += __shfl_xor_sync(0xffffffffu, d, 2);
-        if (g == 0 && j9 < NS + kCoarse) sm.tot[j9 - NS] = d;
-    }
-    __syncthreads();
-}
 
 // E^-1 t by warps 2 and 3, four lanes per row; e: the lane's entries of its row
 // (columns g, g + 4, 8 of g = 0). Result in every lane of the row.
@@ -2045,13 +1960,14 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
     __shared__ TailShared sm;
     float* zs = tail_vec;            // w, then z (9 per camera of the CTA)
     float* rs = tail_vec + 9 * per;  // r, then r - SZ c1
-    cluster_arrive();
+    csum::cluster_arrive();
     const int tid = threadIdx.x, warp = tid >> 5;
     const int rank = blockIdx.x, nctas = gridDim.x;
     const int c0 = min(rank * per, C), m = min(per, C - c0);  // this CTA's cameras
     const long long n = 9ll * C, i0 = 9ll * c0;
     const int rows = 9 * m, step = kOne ? blockDim.x : 9 * (blockDim.x / 9);
     const int first = tid < step ? tid : rows;  // this thread's first row
+    const int rounds = kOne ? 1 : (rows + step - 1) / step;
     auto load9 = [&](float (&d)[9], const float* src, long long stride) {
 #pragma unroll
         for (int j = 0; j < 9; ++j) d[j] = src[j * stride];
@@ -2093,18 +2009,19 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
     }
     pdl_wait();
     pdl_trigger();
-    cluster_wait();  // every CTA of the cluster runs
+    csum::cluster_wait();  // every CTA of the cluster runs
     if (over) return;
 
-    float v[10];
-#pragma unroll
-    for (int j = 0; j < 10; ++j) v[j] = 0.f;
+    constexpr bool kPairs = !kOne;  // sums of several values per thread
+    const ff none = {0.f, 0.f};
+    ff sums[2] = {none, none}, nine = none;
+    float v[kCoarse];
     for (int i = first; i < rows; i += step) {
         if (!kOne) pv = *p_at(i);
         qv = q[i0 + i];
-        v[0] = fmaf(pv, qv, v[0]);
+        csum::add_term<kPairs>(sums[0], pv * qv);
     }
-    cluster_totals<1, false>(v, sm, 0, rank, nctas, [&](double pq, double) {
+    csum::totals<1, false, kPairs>(sums, nine, sm.sums, 0, rank, nctas, [&](double pq, double) {
         const bool ok = pq > 0.0 && isfinite(pq);
         alpha = ok ? rz_old / pq : 0.0;
         sm.scalar = static_cast<float>(alpha);
@@ -2117,24 +2034,31 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
     const float af = sm.scalar;
 
     // x, r; r.r and Z^T r, or z = M r and r.z
-    v[0] = 0.f;
-    for (int i = first; i < rows; i += step) {
-        if (!kOne) {
-            xv = x[i0 + i];
-            rv = r[i0 + i];
-            pv = *p_at(i);
-            qv = q[i0 + i];
-            if (kZ) load9(zc, Zc + i0 + i, n);
-        }
-        x[i0 + i] = fmaf(af, pv, xv);
-        rv = fmaf(-af, qv, rv);
-        r[i0 + i] = rv;
-        rs[i] = rv;
-        v[0] = fmaf(rv, rv, v[0]);
-        if (kZ) {
+    sums[0] = none;
+    for (int k0 = 0; k0 < rounds; k0 += csum::kFoldRows) {
 #pragma unroll
-            for (int j = 0; j < kCoarse; ++j) v[1 + j] = fmaf(zc[j], rv, v[1 + j]);
+        for (int j = 0; j < kCoarse; ++j) v[j] = 0.f;
+        for (int k = k0; k < min(k0 + csum::kFoldRows, rounds); ++k) {
+            const int i = first + k * step;
+            if (i >= rows) break;
+            if (!kOne) {
+                xv = x[i0 + i];
+                rv = r[i0 + i];
+                pv = *p_at(i);
+                qv = q[i0 + i];
+                if (kZ) load9(zc, Zc + i0 + i, n);
+            }
+            x[i0 + i] = fmaf(af, pv, xv);
+            rv = fmaf(-af, qv, rv);
+            r[i0 + i] = rv;
+            rs[i] = rv;
+            csum::add_term<kPairs>(sums[0], rv * rv);
+            if (kZ) {
+#pragma unroll
+                for (int j = 0; j < kCoarse; ++j) v[j] = fmaf(zc[j], rv, v[j]);
+            }
         }
+        if (kZ) csum::fold_nine<kPairs>(v, nine);
     }
     // the convergence test, and beta
     auto test = [&](double rr_t) { return rr_t <= tol2bb || iters >= max_iters ? 1 : 0; };
@@ -2163,15 +2087,15 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
 #pragma unroll
             for (int j = 0; j < 9; ++j) z = fmaf(mrow[j], r9[j], z);
             zs[i] = z;
-            v[1] = fmaf(rs[i], z, v[1]);
+            csum::add_term<kPairs>(sums[1], rs[i] * z);
         }
-        cluster_totals<2, false>(v, sm, 1, rank, nctas, [&](double rr_t, double rz_t) {
+        csum::totals<2, false, kPairs>(sums, nine, sm.sums, 1, rank, nctas, [&](double rr_t, double rz_t) {
             rr = rr_t;
             sm.done = test(rr_t);
             direction(rz_t);
         });
     } else {
-        cluster_totals<1, true>(v, sm, 1, rank, nctas, [&](double rr_t, double) {
+        csum::totals<1, true, kPairs>(sums, nine, sm.sums, 1, rank, nctas, [&](double rr_t, double) {
             rr = rr_t;
             sm.done = test(rr_t);
             if (sm.done) direction(1.0);
@@ -2181,7 +2105,7 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
         const int row = (tid - 64) >> 2;
         const bool coeff = (warp == 2 || warp == 3) && row < kCoarse && (tid & 3) == 0;
         if (warp == 2 || warp == 3) {
-            const double c = coarse_solve4(e, sm.tot);
+            const double c = coarse_solve4(e, sm.sums.tot);
             if (coeff) {
                 sm.c1[row] = c;
                 sm.cf[row] = static_cast<float>(c);
@@ -2196,29 +2120,35 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
             rs[i] = yi;
         }
         __syncthreads();
+        nine = none;
+        for (int k0 = 0; k0 < rounds; k0 += csum::kFoldRows) {
 #pragma unroll
-        for (int j = 0; j < kCoarse; ++j) v[j] = 0.f;
-        for (int i = first; i < rows; i += step) {
-            if (!kOne) {
-                load9(mrow, Minv + 9 * (i0 + i), 1);
-                load9(sz, SZ + i0 + i, n);
+            for (int j = 0; j < kCoarse; ++j) v[j] = 0.f;
+            for (int k = k0; k < min(k0 + csum::kFoldRows, rounds); ++k) {
+                const int i = first + k * step;
+                if (i >= rows) break;
+                if (!kOne) {
+                    load9(mrow, Minv + 9 * (i0 + i), 1);
+                    load9(sz, SZ + i0 + i, n);
+                }
+                const float* y9 = rs + i - i % 9;
+                float w = 0.f;
+#pragma unroll
+                for (int j = 0; j < 9; ++j) w = fmaf(mrow[j], y9[j], w);
+                zs[i] = w;
+#pragma unroll
+                for (int j = 0; j < kCoarse; ++j) v[j] = fmaf(sz[j], w, v[j]);
             }
-            const float* y9 = rs + i - i % 9;
-            float w = 0.f;
-#pragma unroll
-            for (int j = 0; j < 9; ++j) w = fmaf(mrow[j], y9[j], w);
-            zs[i] = w;
-#pragma unroll
-            for (int j = 0; j < kCoarse; ++j) v[j] = fmaf(sz[j], w, v[j]);
+            csum::fold_nine<kPairs>(v, nine);
         }
-        cluster_totals<0, true>(v, sm, 2, rank, nctas, [](double, double) {});
+        csum::totals<0, true, kPairs>(sums, nine, sm.sums, 2, rank, nctas, [](double, double) {});
         // z = w + Z (c1 - c2) and r.z
         if (warp == 2 || warp == 3) {
-            const double c = coarse_solve4(e, sm.tot);
+            const double c = coarse_solve4(e, sm.sums.tot);
             if (coeff) sm.cf[row] = static_cast<float>(sm.c1[row] - c);
         }
         __syncthreads();
-        v[0] = 0.f;
+        sums[0] = none;
         for (int i = first; i < rows; i += step) {
             if (!kOne) {
                 load9(zc, Zc + i0 + i, n);
@@ -2228,9 +2158,9 @@ __global__ void __launch_bounds__(kTailMaxT) pcg_tail(const float* __restrict__ 
 #pragma unroll
             for (int j = 0; j < kCoarse; ++j) z = fmaf(zc[j], sm.cf[j], z);
             zs[i] = z;
-            v[0] = fmaf(rv, z, v[0]);
+            csum::add_term<kPairs>(sums[0], rv * z);
         }
-        cluster_totals<1, false>(v, sm, 3, rank, nctas, [&](double rz_t, double) { direction(rz_t); });
+        csum::totals<1, false, kPairs>(sums, nine, sm.sums, 3, rank, nctas, [&](double rz_t, double) { direction(rz_t); });
     }
     if (sm.done) return;
     const float bf = sm.scalar;
