@@ -234,9 +234,10 @@ __global__ void rhs_finalize_kernel(const int* __restrict__ cam_chunk_off, const
 
 // ---------------------------------------------------------------- FP64 Cholesky
 //
-// The explicitly dense layout keeps the reference's arithmetic: an FP64
-// factorisation (the trailing update by mma.sync m8n8k4, the FP64 pipe's rate), to
-// check the fixed-point one (chol.cu), which serves every other call, against.
+// The explicitly chosen layouts, dense and band, keep the reference's arithmetic: an
+// FP64 factorisation (the trailing update by mma.sync m8n8k4, the FP64 pipe's rate), for
+// callers that want it and to check the fixed-point one (chol.cu) against, which serves
+// the automatic layout and the standalone calls.
 
 // Factor the NB x NB diagonal block at (j0, j0) in shared memory.
 // The pivot's square root and its reciprocal are taken once per column (by
@@ -391,8 +392,8 @@ __global__ void __launch_bounds__(256) syrk_update_kernel(double* __restrict__ A
 }
 
 // The trailing update by 32 x 32 quadrants (four CTAs per 64 x 64 tile, the
-// upper quadrant of a diagonal tile skipped): for steps with few tiles, so
-// that the update spreads over four times as many SMs.
+// upper quadrant of a diagonal tile skipped): for steps with few tiles (a
+// band's bt(bt+1)/2), so that the update spreads over four times as many SMs.
 // 8 warps per quadrant, each warp 8 x 16 = 1 x 2 DMMA tiles.
 constexpr int kSPq = 32 + 8;  // shared-memory stride (doubles) of the quadrant's K-major operands
 __global__ void __launch_bounds__(256) syrk_update_quad_kernel(double* __restrict__ A, int j0, int ntiles, int lda,
@@ -668,7 +669,8 @@ __global__ void twist_solution(const double* __restrict__ bt, int n, int base, c
 
 }  // namespace
 
-static void dense_potrf_fp64(double* A, int n, int lda, int* info, cudaStream_t s) {
+// bt, lda: as for dense_potrf (chol.cu).
+static void dense_potrf_fp64(double* A, int n, int lda, int bt, int* info, cudaStream_t s) {
     GBA_CUDA_CHECK(cudaMemsetAsync(info, 0, sizeof(int), s));
     static bool attr = false;
     const int smem = 2 * NB * kSP * sizeof(double);
@@ -683,9 +685,9 @@ static void dense_potrf_fp64(double* A, int n, int lda, int* info, cudaStream_t 
         const int j0 = jb * NB;
         potrf_diag_kernel<<<1, 256, 0, s>>>(A, j0, lda, info);
         GBA_LAUNCH_CHECK();
-        const int below = nt - jb - 1;
-        if (below == 0) break;
-        // few panel tiles (the last steps): split them over more CTAs
+        const int below = std::min(nt - jb - 1, bt);
+        if (below == 0) continue;
+        // few panel tiles (a band, or the last steps): split them over more CTAs
         const int sms = device_sm_count();
         const int rows = below * 4 <= sms ? 16 : NB;
         trsm_panel_kernel<<<below * (NB / rows), 256, tsmem, s>>>(A, j0, lda, rows, info);
@@ -872,8 +874,8 @@ int Solver::schur_dense(double lambda) {
         GBA_LAUNCH_CHECK();
     }
     cudaEvent_t ev = prof_start();
-    if (schur_layout_ == 1)
-        dense_potrf_fp64(S_.get(), n_pad_, lda, info_.get(), stream_);
+    if (schur_layout_ != 0)
+        dense_potrf_fp64(S_.get(), n_pad_, lda, bt, info_.get(), stream_);
     else if (twist_ta_)
         band_potrf_twisted(S_.get(), n_pad_, lda, bt, twist_ta_, twist_.get(), info_.get(), chol_ws_.get(), stream_);
     else

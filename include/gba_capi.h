@@ -65,10 +65,10 @@ typedef struct gba_lm_options {
  * of the cameras reordered by reverse Cuthill-McKee on the camera graph (block
  * rows of S within the band, the factor keeps the band). AUTO takes the band
  * when it holds at most a third of the dense matrix (sparse covisibility, e.g.
- * sequential captures); random covisibility stays dense. AUTO and BAND factor S
- * in scaled 64-bit fixed point (chol.cu: exact products, rounding 2^-60 of the
- * diagonal); DENSE, asked for explicitly, in FP64 as the reference does, to
- * check the others against (many times slower on large problems). */
+ * sequential captures); random covisibility stays dense. AUTO factors S in scaled
+ * 64-bit fixed point (chol.cu: exact products, rounding 2^-60 of the diagonal); DENSE
+ * and BAND, asked for explicitly, in FP64 as the reference does (many times slower
+ * on large problems). */
 enum { GBA_SCHUR_AUTO = 0, GBA_SCHUR_DENSE = 1, GBA_SCHUR_BAND = 2 };
 
 enum { GBA_LOSS_NONE = 0, GBA_LOSS_HUBER = 1 };
