@@ -515,7 +515,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
     }
     __syncthreads();
     if (sm.fail) {
-        if (blockIdx.x == 0 && tid == 0) *info = j0 + sm.fail;
+        if (blockIdx.x == 0 && tid == 0) atomicCAS(info, 0, j0 + sm.fail);  // (another chain's block may find one too)
         return;
     }
     if (srow >= NB && rbad) bad[matrix_row(srow)] = 1;
@@ -1070,7 +1070,5 @@ void band_potrf_twisted(const double* S, int n, int lda, int bt, int ta, double*
     launch_pdl(twist_merge, dim3(ceil_div(t.s, 64), t.s), 64, 0, s, Fi, t, lda, w.bad, dsep);
     for (int k = 0; k < bt; ++k) factor_panel(F, t.a + k * NB, 0, 1, bt - 1 - k, lda, w, info, s);
 }
-
-int band_twist_row(int i, int n, int bt, int ta) { return Twist(n, bt, ta).source(i); }
 
 }  // namespace gba

@@ -873,18 +873,26 @@ int Solver::schur_dense(double lambda) {
         extract_diag_blocks<<<ceil_div(81ll * C_, 256), 256, 0, stream_>>>(S_.get(), C_, lda, perm, Sdiag_.get());
         GBA_LAUNCH_CHECK();
     }
+    bool twisted = twist_ta_ > 0;  // the factor is in twist_, not in S
     cudaEvent_t ev = prof_start();
     if (schur_layout_ != 0)
         dense_potrf_fp64(S_.get(), n_pad_, lda, bt, info_.get(), stream_);
-    else if (twist_ta_)
+    else if (twisted)
         band_potrf_twisted(S_.get(), n_pad_, lda, bt, twist_ta_, twist_.get(), info_.get(), chol_ws_.get(), stream_);
     else
         dense_potrf(S_.get(), n_pad_, lda, bt, info_.get(), chol_ws_.get(), stream_);
     prof_stop("dense_potrf", ev);
     int info = 0;
     read_back({{&info, info_.get(), sizeof info}});
+    if (twisted && info > 0) {
+        // Which chain meets its bad pivot first, and where, is not what the rows in their
+        // order would say: ask them.
+        twisted = false;
+        dense_potrf(S_.get(), n_pad_, lda, bt, info_.get(), chol_ws_.get(), stream_);
+        read_back({{&info, info_.get(), sizeof info}});
+    }
     if (info < 0) throw std::runtime_error("dense_potrf: a wait of the trailing update ran out");
-    if (info != 0) return twist_ta_ ? band_twist_row(info - 1, n_pad_, bt, twist_ta_) + 1 : info;
+    if (info != 0) return info;
     // solve in a copy so rhs stays the assembled right-hand side (in the band
     // layout the copy is in the renumbered camera order; the padding stays 0)
     if (band_mode_) {
@@ -895,7 +903,7 @@ int Solver::schur_dense(double lambda) {
         GBA_CUDA_CHECK(cudaMemcpyAsync(pcg_x_.get(), rhs_.get(), n_pad_ * sizeof(double), cudaMemcpyDeviceToDevice,
                                        stream_));
     }
-    if (twist_ta_)
+    if (twisted)
         band_potrs_twisted(twist_.get(), n_pad_, lda, bt, twist_ta_, pcg_x_.get(), info_.get(), chol_ws_.get(), stream_);
     else
         dense_potrs(S_.get(), n_pad_, lda, bt, pcg_x_.get(), info_.get(), chol_ws_.get(), stream_);

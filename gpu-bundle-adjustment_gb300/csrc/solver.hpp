@@ -390,10 +390,9 @@ void dense_potrf(double* A, int n, int lda, int bt, int* info, void* workspace, 
 size_t dense_potrs_workspace(int n);
 // The same for a band S from both ends (chol.cu): ta tiles from the top, the bt tiles
 // after them last; S stays, F ((n + 64 bt) columns of lda + 1) holds the factor.
-// band_twist_row: the band row of a row of F (*info counts F's).
+// *info: whether it failed, not at which of the band's rows.
 size_t band_twist_workspace(int n, int bt);
 size_t band_twist_solve_workspace(int n, int bt);
-int band_twist_row(int i, int n, int bt, int ta);
 void band_potrf_twisted(const double* S, int n, int lda, int bt, int ta, double* F, int* info, void* workspace,
                         cudaStream_t s);
 void band_potrs_twisted(const double* F, int n, int lda, int bt, int ta, double* b, const int* info, void* workspace,
