@@ -586,6 +586,7 @@ int gba_solver_download(gba_solver* s, int buffer, void* dst, size_t bytes) {
         need(dst != nullptr, "null destination");
         need(buffer >= GBA_BUF_U && buffer <= GBA_BUF_JP32, "bad buffer id");
         size_t have = 0;
+        if (buffer == GBA_BUF_S) S(s).keep_factor();
         const void* src = S(s).buffer(static_cast<gba::Solver::Buf>(buffer), &have);
         need(src != nullptr, "buffer not held by this solver form");
         need(bytes <= have, "download larger than the buffer");
@@ -599,6 +600,7 @@ int gba_solver_device_ptr(gba_solver* s, int buffer, void** out) {
         need(out != nullptr, "null argument");
         need(buffer >= GBA_BUF_U && buffer <= GBA_BUF_JP32, "bad buffer id");
         size_t have = 0;
+        if (buffer == GBA_BUF_S) S(s).keep_factor();
         *out = const_cast<void*>(S(s).buffer(static_cast<gba::Solver::Buf>(buffer), &have));
     });
 }

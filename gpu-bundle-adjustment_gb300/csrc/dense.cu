@@ -825,6 +825,8 @@ void Solver::ensure_schur_storage() {
     schur_layout_planned_ = want;
 }
 
+static const char* const kWaitRanOut = "dense_potrf: a wait of the trailing update ran out";
+
 int Solver::schur_dense(double lambda) {
     ensure_schur_storage();
     const int lda = band_mode_ ? band_ldb_ - 1 : n_pad_;
@@ -874,6 +876,7 @@ int Solver::schur_dense(double lambda) {
         GBA_LAUNCH_CHECK();
     }
     bool twisted = twist_ta_ > 0;  // the factor is in twist_, not in S
+    s_assembled_ = false;
     cudaEvent_t ev = prof_start();
     if (schur_layout_ != 0)
         dense_potrf_fp64(S_.get(), n_pad_, lda, bt, info_.get(), stream_);
@@ -891,7 +894,7 @@ int Solver::schur_dense(double lambda) {
         dense_potrf(S_.get(), n_pad_, lda, bt, info_.get(), chol_ws_.get(), stream_);
         read_back({{&info, info_.get(), sizeof info}});
     }
-    if (info < 0) throw std::runtime_error("dense_potrf: a wait of the trailing update ran out");
+    if (info < 0) throw std::runtime_error(kWaitRanOut);
     if (info != 0) return info;
     // solve in a copy so rhs stays the assembled right-hand side (in the band
     // layout the copy is in the renumbered camera order; the padding stays 0)
@@ -903,6 +906,7 @@ int Solver::schur_dense(double lambda) {
         GBA_CUDA_CHECK(cudaMemcpyAsync(pcg_x_.get(), rhs_.get(), n_pad_ * sizeof(double), cudaMemcpyDeviceToDevice,
                                        stream_));
     }
+    s_assembled_ = twisted;
     if (twisted)
         band_potrs_twisted(twist_.get(), n_pad_, lda, bt, twist_ta_, pcg_x_.get(), info_.get(), chol_ws_.get(), stream_);
     else
@@ -914,8 +918,19 @@ int Solver::schur_dense(double lambda) {
         GBA_CUDA_CHECK(cudaMemcpyAsync(dc_.get(), pcg_x_.get(), 9ull * C_ * sizeof(double), cudaMemcpyDeviceToDevice,
                                        stream_));
     }
+    if (s_wanted_) keep_factor();
     sync();
     return 0;
+}
+
+void Solver::keep_factor() {
+    s_wanted_ = true;
+    if (!s_assembled_) return;
+    dense_potrf(S_.get(), n_pad_, band_ldb_ - 1, band_bt_, info_.get(), chol_ws_.get(), stream_);
+    s_assembled_ = false;
+    int info = 0;
+    read_back({{&info, info_.get(), sizeof info}});  // (S is there, on any stream)
+    if (info < 0) throw std::runtime_error(kWaitRanOut);
 }
 
 }  // namespace gba

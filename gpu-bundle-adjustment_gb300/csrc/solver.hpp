@@ -337,7 +337,12 @@ public:
     int band_ldb_ = 0, band_bt_ = 0;
     DevBuf<int> cam_perm_;
     int twist_ta_ = 0;         // > 0: the band is factored from both ends, this many tiles from the top
-    DevBuf<double> twist_;     // the two chains' factor (S_ keeps the assembled band then)
+    DevBuf<double> twist_;     // the two chains' factor (S_ keeps the assembled band then,
+                               // unless the caller looks at S: keep_factor)
+    bool s_wanted_ = false, s_assembled_ = false;
+    // S_ holds its factor, now and after every further schur_dense: for a caller that reads
+    // it. A band factored from both ends is factored in place as well.
+    void keep_factor();  // dense.cu
     void set_schur_layout(int layout) { schur_layout_ = layout; }
     void plan_schur_band();       // structure.cu: ordering and band size from the block list
     void ensure_schur_storage();  // dense.cu: allocates S for the chosen layout

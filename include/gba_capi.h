@@ -297,7 +297,9 @@ enum {
     GBA_BUF_W = 4,        /* double[27 E]  9x3 row-major per slot (plain form) */
     GBA_BUF_VINV = 5,     /* double[6 P]   packed */
     GBA_BUF_S = 6,        /* double[n_pad^2] column-major, or the band double[n_pad * ldb] (plain form;
-                             factor after schur_dense) */
+                             factor after schur_dense. A band that AUTO chose is solved from both ends;
+                             from the first gba_solver_download or _device_ptr of this buffer on it is
+                             also factored in place, for this buffer) */
     GBA_BUF_RHS = 7,      /* double[n_pad] (plain) or [9 C] (mixed) */
     GBA_BUF_DC = 8,       /* double[9 C] */
     GBA_BUF_DP = 9,       /* double[3 P] */
