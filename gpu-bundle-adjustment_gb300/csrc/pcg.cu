@@ -1915,14 +1915,14 @@ __global__ void __launch_bounds__(kVT) pcg_direction(float* __restrict__ p32, co
 // (pcg_update, coarse_w, coarse_z and pcg_direction do it in up to four launches).
 // Each of those is bound by its launch and two memory round trips, for a few
 // 9-vectors per camera; between them stand only sums over all cameras. One
-// cluster of CTAs (16, or 8 where 16 do not fit a device) owns all cameras, `per`
-// consecutive ones per CTA, and takes those sums through distributed shared
-// memory (cluster_sums.cuh); one thread takes the scalars.
+// cluster of 16 CTAs owns all cameras, `per` consecutive ones per CTA, and takes
+// those sums through distributed shared memory (cluster_sums.cuh); one thread takes
+// the scalars. Where a device refuses such a cluster, the separate kernels run.
 constexpr int kTailMaxT = 1024;
 constexpr int kTailMinT = 128;   // four warps: the sums' roles
-constexpr int kTailMaxCtas = csum::kMaxCtas;
+constexpr int kTailCtas = csum::kMaxCtas;
 static_assert(csum::kNine == kCoarse, "one sum per coarse basis column");
-// Two 9-vectors of a CTA's cameras in shared memory, also with 8 CTAs. Below, an
+// Two 9-vectors of a CTA's cameras in shared memory, 108 KB of them. Below, an
 // iteration (with its product) takes, separate kernels -> this one, block-Jacobi and
 // learned: 60 cameras 15.9 -> 12.5 and 10.6 -> 7.9 us; 500 18.3 -> 14.1, 19.4 -> 14.1;
 // 5,000 38 -> 29, 51 -> 37; 24,000 80 -> 69, 128 -> 99 us.
@@ -2496,7 +2496,7 @@ static cudaLaunchConfig_t tail_config(const TailPlan& t, cudaStream_t stream, cu
 }
 // What a cluster may need beyond the defaults (the same for every solver: solvers of
 // several threads share the kernels' attributes).
-constexpr int kTailMaxSmem = 2 * 9 * sizeof(float) * (kTailMaxC / (kTailMaxCtas / 2));
+constexpr int kTailMaxSmem = 2 * 9 * sizeof(float) * (kTailMaxC / kTailCtas);
 template <bool kZ, bool kOne>
 static void allow_tail() {
     GBA_CUDA_CHECK(cudaFuncSetAttribute(pcg_tail<kZ, kOne>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
@@ -2527,24 +2527,22 @@ static void launch_tail(Solver& s, const TailPlan& t, bool coarse, int max_iters
 static TailPlan plan_tail(Solver& s) {
     TailPlan t;
     if (s.C_ > kTailMaxC) return t;
-    auto with = [&](int ctas) {
-        t.ctas = ctas;
-        t.per = ceil_div(s.C_, ctas);
-        t.one_round = 9 * t.per <= kTailMaxT;
-        t.threads = t.one_round ? std::max(kTailMinT, 32 * ceil_div(9 * t.per, 32)) : kTailMaxT;
-        t.smem = 2 * 9 * sizeof(float) * t.per;
-    };
-    if (!s.tail_ctas_) {  // 16 CTAs per cluster are an opt-in the device may refuse
-        with(kTailMaxCtas);
+    t.ctas = kTailCtas;
+    t.per = ceil_div(s.C_, kTailCtas);
+    t.one_round = 9 * t.per <= kTailMaxT;
+    t.threads = t.one_round ? std::max(kTailMinT, 32 * ceil_div(9 * t.per, 32)) : kTailMaxT;
+    t.smem = 2 * 9 * sizeof(float) * t.per;
+    if (!s.tail_asked_) {  // 16 CTAs per cluster are an opt-in the device may refuse
         cudaLaunchAttribute at[2];
         const cudaLaunchConfig_t cfg = tail_config(t, s.stream_, at);
         int fit = 0;
         allow_tail<true, true>();
         const bool ok = cudaOccupancyMaxActiveClusters(&fit, pcg_tail<true, true>, &cfg) == cudaSuccess && fit > 0;
         if (!ok) cudaGetLastError();
-        s.tail_ctas_ = ok ? kTailMaxCtas : kTailMaxCtas / 2;
+        s.tail_fits_ = ok;
+        s.tail_asked_ = true;
     }
-    with(s.tail_ctas_);
+    if (!s.tail_fits_) t.ctas = 0;
     return t;
 }
 

@@ -244,7 +244,7 @@ public:
     static constexpr int kCamChunkSlots = 1024;  // most positions of a camera chunk
     bool one_pass_ = false;
     int n_acc_ = 0;
-    int tail_ctas_ = 0;  // cluster size of pcg_tail on this device (0: not asked yet)
+    bool tail_asked_ = false, tail_fits_ = false;  // does pcg_tail's cluster fit this device
     // the warp-level point passes' work: warp chunks (whole points, at most
     // 32 slots: int2 {first, end slot}); points with 33 to 256 observations in
     // lists of at most 256 slots per CTA (lchunk_: int2 {first entry of lpts_,
