@@ -8,7 +8,7 @@
 // chip, 64 cycles per warp FMA, whether by DFMA or DMMA. Here no FP64
 // arithmetic is left on the path:
 //   scale     row exponents e_i from the diagonal (A_ii 2^(-2 e_i) in [1/8, 1/2))
-//   convert   the lower triangle, in place, to 64-bit integers (2^-60 units)
+//   convert   the lower triangle, in place, to 64-bit integers (2^-62 units)
 //   per 64-column panel
 //     panel   the 64 x 64 diagonal tile and the rows below it (chol_panel): the
 //             factor's columns as FP64 in place, and the rows' base-512 digits
@@ -46,9 +46,7 @@
 namespace gba {
 namespace {
 
-using fx::Acc;
 using fx::Acc29;
-using fx::Limbs;
 using fx::Limbs29;
 
 constexpr int NB = 64;                        // panel width / tile size
@@ -93,7 +91,7 @@ __global__ void chol_scale(const double* __restrict__ A, int n, int lda, int* __
 // their diagonal entries are infinite.
 __device__ __forceinline__ long long convert_entry(double v, int ei, int ej, bool inf_row, bool inf_col, bool diagonal,
                                                    bool* bad) {
-    if (!inf_row && !inf_col) return fx::to_fixed(v, ei + ej, bad);
+    if (!inf_row && !inf_col) return fx::to_fixed<fx::kFracC>(v, ei + ej, bad);
     if (!diagonal && v != 0.0) {
         int x;
         uint64_t m;
@@ -199,8 +197,7 @@ constexpr int kBarSolved = 5, kBarNext = 6, kBarHandover = 7;
 constexpr int kWindowCount = 32 + 32 * kUpdateWarps, kPivotsCount = 32 + 32 * kUpdateWarps, kPivotsSolving = 32 + 64;
 
 // Limbs of four consecutive columns.
-template <typename T>
-__device__ __forceinline__ void load_limbs4(const T* p, T (&l)[4]) {
+__device__ __forceinline__ void load_limbs4(const Limbs29* p, Limbs29 (&l)[4]) {
     const int4 a = reinterpret_cast<const int4*>(p)[0], b = reinterpret_cast<const int4*>(p)[1];
     l[0] = {a.x, a.y};
     l[1] = {a.z, a.w};
@@ -480,7 +477,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
     auto matrix_row = [&](int g) { return g < NB ? j0 + g : j0 + NB + b0 + (g - NB); };
     auto diagonal = [&](int g) {
         const int r = matrix_row(g);
-        return bad[r] == 2 ? 1.f : static_cast<float>(F[r + static_cast<long long>(r) * lda]) * 0x1p-60f;
+        return bad[r] == 2 ? 1.f : static_cast<float>(F[r + static_cast<long long>(r) * lda]) * 0x1p-62f;
     };
     __syncthreads();
     // workers by sub-partition 1, 2, 3 (warp & 3) and slot (warp >> 2): updating
@@ -501,7 +498,7 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
 #pragma unroll
         for (int m = 0; m < 16; ++m) {
             const int j = 4 * m + q;
-            a[m] = fx::acc29(live && (g >= NB || j <= g) ? F[matrix_row(g) + static_cast<long long>(j0 + j) * lda] : 0);
+            a[m] = {live && (g >= NB || j <= g) ? F[matrix_row(g) + static_cast<long long>(j0 + j) * lda] : 0, 0};
         }
         updating_warp(sm, a, g, q);
     } else {
@@ -540,11 +537,11 @@ __global__ void __launch_bounds__(kPanelThreads, 1) chol_panel(double* __restric
         const int r = j0 + NB + c0 + g;
         const bool lv = g < n;
         bool rb = lv ? bad[r] == 1 : true;
-        float rs = lv ? static_cast<float>(F[r + static_cast<long long>(r) * lda]) * 0x1p-60f : 0.f;
+        float rs = lv ? static_cast<float>(F[r + static_cast<long long>(r) * lda]) * 0x1p-62f : 0.f;
         if (lv && bad[r] == 2) rs = 1.f;
         Acc29 a[16];
 #pragma unroll
-        for (int m = 0; m < 16; ++m) a[m] = fx::acc29(lv ? F[r + static_cast<long long>(j0 + 4 * m + q) * lda] : 0);
+        for (int m = 0; m < 16; ++m) a[m] = {lv ? F[r + static_cast<long long>(j0 + 4 * m + q) * lda] : 0, 0};
         __syncthreads();  // sm.lv of the previous rows has been written out
         if (8 * warp < n) {
             for (int b = 0; b < 16; ++b) {
@@ -601,20 +598,24 @@ __device__ __forceinline__ void place_diagonal(double* __restrict__ A, int j0, i
 //
 // C(I, J) -= L(I) L(J)^T for the lower tiles: 128 rows (two 64-row tiles) by 64
 // columns, K = 64 (the panel). With L = sum_s q_s 2^(52 - 9 s), the products of
-// digits s and t weigh 2^(44 - 9 (s + t)) units: group d = s + t is summed in one
-// FP32 accumulator of 64 TMEM columns (7 groups: 448 of 512 columns); 28 digit
-// products of 4 MMAs (K = 16). The sums of groups 0 to 4 stay below 2^24 and
-// are exact; a rounding in groups 5 and 6, whose bound is 2^24.4, would weigh
-// at most one of the entries' 2^-60 units. The products left out
-// (d > 6) weigh a third of a unit (root mean square).
+// digits s and t weigh 2^(46 - 9 (s + t)) of C's units of 2^-62: group d = s + t is
+// summed in one FP32 accumulator of 64 TMEM columns (8 groups: all 512 columns); 34
+// digit products of 4 MMAs (K = 16). The sums of groups 0 to 4 stay below 2^24 and
+// are exact; a rounding in group 5, whose bound is 2^24.4, would weigh two units, in
+// groups 6 and 7 less than one. The products left out (d > 7) weigh a hundredth of a
+// unit. With entries in units of 2^-60 and d = 7 left out, a third of such a unit, the
+// update was less precise than FP64 arithmetic from some 2,000 rows on: error of the
+// solution at 4,096 rows 3.0e-15, FP64 1.45e-15, so 6.4e-16 (and 23.5 ms for a trial
+// of 1,000 cameras, 22.7 without).
 //
 // One CTA per SM walks a contiguous run of tiles (row block by row block, so the
 // row block's digits are loaded once): warp 0 loads digit tiles (bulk copies,
 // columns double-buffered), warp 1 issues the MMAs, sixteen warps recombine. The
-// low groups (4, 5, 6) come first: the recombination of one part overlaps
-// the MMAs of the other. What bounds it: 28 x 4 MMAs of 128 x 64 x 16 a tile, which
+// low groups (4 to 7) come first: the recombination of one part overlaps
+// the MMAs of the other. What bounds it: 34 x 4 MMAs of 128 x 64 x 16 a tile, which
 // read their operands from shared memory at 6 KB per MMA, and the 16 bytes of
 // each entry per panel from and to HBM.
+constexpr int kGroups = 8;
 constexpr int kUpdWarps = 16;  // recombining warps: 32 rows x 16 columns each
 constexpr int kUpdThreads = 64 + 32 * kUpdWarps;
 constexpr int kABytes = kNS * 2 * kTileB, kBBytes = kNS * kTileB;
@@ -766,7 +767,7 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
             const uint32_t b = sB + st * kBBytes;
             auto group = [&](int d) {
                 bool acc = false;
-                for (int s = 0; s <= d; ++s) {
+                for (int s = max(0, d - kNS + 1); s <= min(d, kNS - 1); ++s) {
                     const uint64_t da = operand_desc(sA + s * 2 * kTileB), db = operand_desc(b + (d - s) * kTileB);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) {  // K = 16: 32 bytes along the swizzled row
@@ -777,7 +778,7 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
             };
             if (i > 0 && !mbar_wait(bar(B_LOEMPTY), (i - 1) & 1, &gave_up)) break;
             tc_fence_after();
-            for (int d = 4; d < kNS; ++d) group(d);
+            for (int d = 4; d < kGroups; ++d) group(d);
             mma_commit(bar(B_LOFULL));
             if (i > 0 && !mbar_wait(bar(B_HIEMPTY), (i - 1) & 1, &gave_up)) break;
             tc_fence_after();
@@ -806,15 +807,16 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
             tc_fence_after();
 #pragma unroll
             for (int k0 = 0; k0 < 16; k0 += 8) {
-                float g4[8], g5[8], g6[8];
+                float g4[8], g5[8], g6[8], g7[8];
                 tmem_load8(tm + 4 * 64 + k0, g4);
                 tmem_load8(tm + 5 * 64 + k0, g5);
                 tmem_load8(tm + 6 * 64 + k0, g6);
+                tmem_load8(tm + 7 * 64 + k0, g7);
                 tmem_wait_load();
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    c[k0 + k] = static_cast<long long>(__float2int_rn(g4[k])) * 256 +
-                                __float2int_rn(0.5f * fmaf(g6[k], 0x1p-9f, g5[k]));
+                    c[k0 + k] = static_cast<long long>(__float2int_rn(g4[k])) * 1024 +
+                                (2 * __float2int_rn(g5[k]) + __float2int_rn(0x1p-8f * fmaf(g7[k], 0x1p-9f, g6[k])));
             }
             tc_fence_before();
             __syncwarp();
@@ -831,10 +833,10 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
                 tmem_wait_load();
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
-                    const int top = small_int(g0[k]) * 512 + small_int(g1[k]);  // 2^35
-                    c[k0 + k] += (static_cast<long long>(top) << 35) +
-                                 static_cast<long long>(__float2int_rn(g2[k])) * (1 << 26) +
-                                 static_cast<long long>(__float2int_rn(g3[k])) * (1 << 17);
+                    const int top = small_int(g0[k]) * 512 + small_int(g1[k]);  // 2^37
+                    c[k0 + k] += (static_cast<long long>(top) << 37) +
+                                 static_cast<long long>(__float2int_rn(g2[k])) * (1 << 28) +
+                                 static_cast<long long>(__float2int_rn(g3[k])) * (1 << 19);
                 }
             }
             tc_fence_before();
@@ -868,7 +870,7 @@ __global__ void __launch_bounds__(kIntB * kIntB) chol_update_int(double* __restr
                                                                 const long long* __restrict__ rows,
                                                                 const double* __restrict__ diag,
                                                                 const int* __restrict__ info) {
-    __shared__ __align__(16) Limbs L[2][kIntB][NB + 2];
+    __shared__ __align__(16) Limbs29 L[2][kIntB][NB + 2];
     j1 += blockIdx.y * dj;
     if (blockIdx.x == gridDim.x - 1) {
         pdl_wait();
@@ -886,22 +888,22 @@ __global__ void __launch_bounds__(kIntB * kIntB) chol_update_int(double* __restr
     pdl_trigger();
     if (*info) return;
     long long* p = reinterpret_cast<long long*>(A) + row + static_cast<long long>(col) * lda;
-    Acc acc = {row >= col ? *p : 0, 0};
+    Acc29 acc = {row >= col ? *p : 0, 0};
 #pragma unroll
     for (int t = threadIdx.x; t < 2 * kIntB * NB; t += kIntB * kIntB) {
         const int h = t / (kIntB * NB), r = (t / NB) % kIntB, k = t % NB;
-        L[h][r][k] = fx::split(rows[static_cast<long long>(j1 + kIntB * (h ? cb : rb) + r) * NB + k]);
+        L[h][r][k] = fx::split29(rows[static_cast<long long>(j1 + kIntB * (h ? cb : rb) + r) * NB + k]);
     }
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < NB; k += 4) {
-        Limbs a[4], b[4];
+        Limbs29 a[4], b[4];
         load_limbs4(&L[0][i][k], a);
         load_limbs4(&L[1][j][k], b);
 #pragma unroll
         for (int q = 0; q < 4; ++q) fx::fms_full(acc, a[q], b[q]);
     }
-    if (row >= col) *p = fx::value(acc);
+    if (row >= col) *p = fx::quarters(acc);
 }
 // Most tiles below the diagonal tile that it serves: of a step (panel and update) of
 // 42 us, 5 us less at up to 8 tiles, 3 at 12, none at 16, 10 more at 24.

@@ -7,9 +7,11 @@
 // An SPD matrix is scaled symmetrically by powers of two, A_ij 2^-(e_i + e_j),
 // so that its diagonal lies in [1/8, 1/2). Every entry of every Schur complement
 // then stays below 1/2 and every entry of the scaled factor below 0.71: they are
-// held as 64-bit integers in units of 2^-60. The absolute rounding 2^-61
-// relative to sqrt(A_ii A_jj) is 128 times finer than that of an FP64 entry of
-// that size, and the sums are exact.
+// held as 64-bit integers, the factor's in units of 2^-60, the others, which are
+// rounded once per panel, of 2^-62. The absolute rounding relative to
+// sqrt(A_ii A_jj) is hundreds of times finer than that of an FP64 entry of that size.
+// An entry far below its diagonal keeps that absolute precision, not FP64's relative
+// one: of a coupling of 2^-k some 60 - k bits.
 //
 // Host and device: the same functions run on the CPU in tests/test_fix64.py.
 
@@ -81,8 +83,10 @@ GBA_FX int row_exponent(double d) {
     return (x + 3) >> 1;
 }
 
-// d 2^(-e) in fixed point, rounded to nearest; *bad is set where it is not
-// finite or too large for an entry of a scaled SPD matrix (0 is returned).
+// d 2^(-e) in fixed point with kF fraction bits (up to 62), rounded to nearest; *bad is
+// set where it is not finite or too large for an entry of a scaled SPD matrix (0 is
+// returned).
+template <int kF = kFrac>
 GBA_FX long long to_fixed(double d, int e, bool* bad) {
     const int64_t b = double_bits(d);
     if ((b & 0x7fffffffffffffffll) == 0) return 0;
@@ -93,9 +97,9 @@ GBA_FX long long to_fixed(double d, int e, bool* bad) {
     int x;
     uint64_t m;
     decompose(d, &x, &m);
-    const int s = x - 52 - e + kFrac;  // |d| 2^-e 2^60 = m 2^s
+    const int s = x - 52 - e + kF;  // |d| 2^-e 2^kF = m 2^s
     uint64_t v;
-    if (s >= 8) {
+    if (s >= kF - 52) {
         *bad = true;
         return 0;
     } else if (s >= 0) {
@@ -105,7 +109,7 @@ GBA_FX long long to_fixed(double d, int e, bool* bad) {
     } else {
         v = 0;
     }
-    if (v > static_cast<uint64_t>(kBig)) {
+    if (v > static_cast<uint64_t>(kBig) << (kF - kFrac)) {
         *bad = true;
         return 0;
     }
@@ -164,13 +168,13 @@ GBA_FX void fms_full(Acc& a, Limbs x, Limbs y) {
 }
 GBA_FX long long value(const Acc& a) { return a.c + ((a.m + (1ll << 29)) >> 30); }
 
-// The same within a panel, whose rounds wait for one another: split at 2^29, so that
-// lo lo', left out, is below a 16th of a unit (of the 63 squares subtracted from a
+// As the kernels take them: split at 2^29, so that within a panel, whose rounds wait for
+// one another, lo lo' can be left out (fms): it is below a 16th of a unit (of the 63 squares subtracted from a
 // diagonal entry it is 1.3 units together; split at 2^30 5.3, and the solution's
 // error at condition 4e3 three times as large). 4,096 unknowns 4.76 -> 4.84 ms; 5.03
-// with fms_full.
-// The sums are kept, and passed on, in quarter units: entries below 2^61, their
-// products' sums as well; of m, at most 2^62.5 (Cauchy-Schwarz over 64 columns).
+// with all products whole. The update of few tiles takes them whole (fms_full).
+// The sums are kept, and passed on, in quarter units, as the matrix is: entries below
+// 2^61, their products' sums as well; of m, at most 2^62.5 (Cauchy-Schwarz over 64 columns).
 struct Limbs29 {
     int hi, lo;  // v = hi 2^29 + lo, lo in [-2^28, 2^28)
 };
@@ -183,12 +187,16 @@ GBA_FX Limbs29 split29(long long v) {
 struct Acc29 {
     long long c, m;  // (c + m 2^-29) / 4
 };
-GBA_FX Acc29 acc29(long long v) { return {v * 4, 0}; }
+constexpr int kFracC = kFrac + 2;  // fraction bits of the matrix: quarter units
 GBA_FX void fms(Acc29& a, Limbs29 x, Limbs29 y) {  // a -= x y
     const int nh = -x.hi, nl = -x.lo;
     a.c += static_cast<long long>(nh) * y.hi;
     a.m += static_cast<long long>(nh) * y.lo;
     a.m += static_cast<long long>(nl) * y.hi;
+}
+GBA_FX void fms_full(Acc29& a, Limbs29 x, Limbs29 y) {
+    fms(a, x, y);
+    a.m += static_cast<long long>(-x.lo >> 14) * (y.lo >> 15);
 }
 GBA_FX long long quarters(const Acc29& a) { return a.c + ((a.m + (1ll << 28)) >> 29); }
 GBA_FX long long value(const Acc29& a) { return (a.c + ((a.m + (1ll << 30)) >> 29)) >> 2; }  // to nearest

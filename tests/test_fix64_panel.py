@@ -2,7 +2,8 @@
 against 128-bit integers.
 
 Bounds, in units of 2^-60: the low halves' product, left out, is below 2^56 2^-60, and
-a value is rounded to nearest (passed on, to a quarter unit). A panel's 63 squares together lose
+a value is rounded to nearest (passed on, to a quarter unit; with the low halves to
+2^-15 of that more). A panel's 63 squares together lose
 at most 63/16 and on average 63/48; the same sums split at 2^30 lose four times that.
 """
 import shutil
@@ -27,18 +28,29 @@ int main() {
         const long long w = ((static_cast<long long>(r() >> 3) - (1ll << 60)) >> (r() % 61)) / 4 * 3;
         const Limbs29 a = split29(v), b = split29(w);
         CHECK((static_cast<__int128>(a.hi) << 29) + a.lo == v && a.lo >= -(1 << 28) && a.lo < (1 << 28));
-        CHECK(value(acc29(v / 2)) == v / 2 && quarters(acc29(v / 2)) == v / 2 * 4);
-        Acc29 acc = acc29(0);
+        const Acc29 half{v / 2 * 4, 0};
+        CHECK(value(half) == v / 2 && quarters(half) == v / 2 * 4);
+        Acc29 acc{0, 0};
         fms(acc, a, b);
         const long double want = -ldexpl(static_cast<long double>(static_cast<__int128>(v) * w), -60);
         CHECK(fabsl(value(acc) - want) <= 0.5L + 0.125L + 0.0625L);
         CHECK(fabsl(quarters(acc) / 4.0L - want) <= 0.125L + 0.0625L);
+        Acc29 full{0, 0};
+        fms_full(full, a, b);
+        CHECK(fabsl(quarters(full) / 4.0L - want) <= 0.126L);
+        // the matrix itself, in quarter units
+        const int e = static_cast<int>(r() % 2000) - 1000;
+        bool bad = false;
+        const double d = ldexp(static_cast<double>(v), e - 60);
+        const long long f = to_fixed<kFracC>(d, e, &bad);
+        if (bad) CHECK(std::abs(v) > 3ll << 58);
+        else CHECK(f == ldexpl(static_cast<long double>(d), 62 - e) && std::abs(v) <= 3ll << 58);
     }
     // a diagonal entry: 63 squares, random and with the low halves at their largest
     long double sum = 0;
     for (int i = 0; i < 20000; ++i) {
         const long long d = (1ll << 59) - 1;
-        Acc29 acc = acc29(d);
+        Acc29 acc{4 * d, 0};
         __int128 exact = static_cast<__int128>(d) << 60;
         for (int k = 0; k < 63; ++k) {
             long long v = static_cast<long long>(r() >> 5) / 7;  // squares add up to less than 1/2
