@@ -169,12 +169,13 @@ GBA_FX void fms_full(Acc& a, Limbs x, Limbs y) {
 GBA_FX long long value(const Acc& a) { return a.c + ((a.m + (1ll << 29)) >> 30); }
 
 // As the kernels take them: split at 2^29, so that within a panel, whose rounds wait for
-// one another, lo lo' can be left out (fms): it is below a 16th of a unit (of the 63 squares subtracted from a
-// diagonal entry it is 1.3 units together; split at 2^30 5.3, and the solution's
-// error at condition 4e3 three times as large). 4,096 unknowns 4.76 -> 4.84 ms; 5.03
-// with all products whole. The update of few tiles takes them whole (fms_full).
-// The sums are kept, and passed on, in quarter units, as the matrix is: entries below
-// 2^61, their products' sums as well; of m, at most 2^62.5 (Cauchy-Schwarz over 64 columns).
+// one another, lo lo' can be left out (fms): it is below a 16th of a unit (of the 63
+// squares subtracted from a diagonal entry it is 1.3 units together; split at 2^30 5.3,
+// and the solution's error at condition 4e3 three times as large). 4,096 unknowns 4.76
+// -> 4.84 ms; 5.03 with all products whole. The update of few tiles takes them whole
+// (fms_full). The sums are kept, and passed on, in quarter units, as the matrix is:
+// entries below 2^61, their products' sums as well; of m, at most 2^62.5
+// (Cauchy-Schwarz over 64 columns).
 struct Limbs29 {
     int hi, lo;  // v = hi 2^29 + lo, lo in [-2^28, 2^28)
 };

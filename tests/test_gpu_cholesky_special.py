@@ -41,3 +41,33 @@ def test_entry_beside_an_infinite_diagonal(gba, torch_cuda, row, col, value):
     A[70, 70] = np.inf
     A[row, col] = A[col, row] = value
     assert _info(gba, torch_cuda, A) == _fp64_failed_column(A)
+
+
+def _cholesky_long_double(A):
+    A = A.astype(np.longdouble).copy()
+    L = np.zeros_like(A)
+    for k in range(len(A)):
+        L[k:, k] = A[k:, k] / np.sqrt(A[k, k])
+        A[k + 1:, k + 1:] -= np.outer(L[k + 1:, k], L[k + 1:, k])
+    return L
+
+
+@pytest.mark.parametrize("coupling", [2.0**-k for k in (3, 10, 20, 40, 60, 80)])
+def test_entries_far_below_the_diagonal(gba, torch_cuda, coupling):
+    """Blocks of nine coupled weakly: every entry of the factor within 16 units of 2^-60 of
+    its row's scale (at most sqrt(8 A_ii)) of the exact one, and an ulp of its own: what
+    the call promises of a coupling, however weak. Below 2^-62 the blocks are factored as
+    if there were none."""
+    torch = torch_cuda
+    n = 192
+    A = coupling * _spd(n, 7)
+    for k in range(0, n, 9):
+        m = min(9, n - k)
+        A[k:k + m, k:k + m] = _spd(m, k)
+    d, info = torch.from_numpy(A).cuda(), torch.zeros(1, dtype=torch.int32, device="cuda")
+    gba.dense_potrf(d.data_ptr(), n, n, info.data_ptr())
+    torch.cuda.synchronize()
+    assert int(info.item()) == 0
+    want = _cholesky_long_double(A)
+    err = np.abs(np.tril(d.cpu().numpy().T) - want)
+    assert (err <= 16 * 2.0**-60 * np.sqrt(8 * np.diag(A))[:, None] + 2.0**-53 * np.abs(want)).all()
