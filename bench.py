@@ -245,8 +245,7 @@ UNITS = {"matvec": ("schur_matvec_f32", "schur_point_pass_f32", "schur_camera_pa
 
 # DRAM bytes (read + write) per launch from one ncu capture (dram__bytes_read.sum +
 # dram__bytes_write.sum, --clock-control none) of each kernel at workload 5; copied
-# here, not measured in this run (profiles/schur_matvec_onepass.md,
-# profiles/mixed_kernels_workload5_ncu.md).
+# here, not measured in this run.
 NCU_TRAFFIC_W5 = {"point_pass_f32": 221.5e6 + 1596.8e6, "camera_pass_f32": None,
                   "schur_matvec_f32": 861.7e6 + 11.5e6 + 368.1e6 + 9.2e6,  # schur_matvec_warp + schur_matvec_long
                   "schur_point_pass_f32": 992.6e6 + 66.4e6, "schur_camera_pass_f32": 774.4e6 + 3.8e6,
@@ -348,7 +347,7 @@ def fp64_tensor_peak_tflops():
 
 
 def roofline_potrf(solver, C):
-    """The factorisation of S: FP16 digit products of its trailing updates (28 per
+    """The factorisation of S: FP16 digit products of its trailing updates (34 per
     entry product, csrc/chol.cu) against the measured 16-bit tensor peak, and its
     FP64-equivalent rate beside cuBLAS DGEMM."""
     n_launch, k_ms = solver.kernel_stats("dense_potrf")
@@ -358,12 +357,12 @@ def roofline_potrf(solver, C):
     n = 9 * C
     fp64_rate = n ** 3 / 3.0 / per_launch_s / 1e12
     peaks, src = _peaks()
-    achieved, peak = 28 * fp64_rate, peaks["bf16_tflops"]
+    achieved, peak = 34 * fp64_rate, peaks["bf16_tflops"]
     return {"bound": "tensor", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
             "frac": achieved / peak, "traffic": None, "kernel": "dense_potrf",
             "launches": n_launch, "avg_launch_s": per_launch_s,
             "fp64_equivalent_tflops": fp64_rate, "dgemm_tflops": fp64_tensor_peak_tflops(),
-            "peak_source": f"{src} 16-bit tensor peak (MEASURED_PEAKS.json bf16_tflops); 28 FP16 digit products per "
+            "peak_source": f"{src} 16-bit tensor peak (MEASURED_PEAKS.json bf16_tflops); 34 FP16 digit products per "
                            "FP64 product; dgemm_tflops: cuBLAS DGEMM 8192^3 in this run"}
 
 

@@ -18,10 +18,11 @@
 //             TMEM, exact: small integers), recombined into the 64-bit entries;
 //             or, where few tiles are left, by integer multiply-adds (chol_update_int)
 // A band is eliminated from both of its ends at once (band_potrf_twisted).
-// Every entry is a sum of products rounded at 2^-60 of sqrt(A_ii A_jj): against
-// long double the factor is closer to the exact one than FP64's up to condition
-// 1e5 or so (192 rows: 5.9e-17 against 2.4e-16 at 20, 6.1e-16 against 13.2e-16 at
-// 4e3, 4.4e-15 both at 4e5), beyond it within a factor of two.
+// Every entry is a sum of products rounded at 2^-62 of sqrt(A_ii A_jj) once a panel (a
+// factor's at 2^-60). Against long double the factor is closer to the exact one than
+// that of the FP64 kernels (dense.cu): 192 rows 5.0e-17 against 2.4e-16 at condition 20,
+// 9.2e-17 against 13.2e-16 at 4e3, 3.1e-16 against 4.4e-15 at 4e5, 1.1e-15 against
+// 9.4e-15 at 4e7; so is the solution (4,096 rows 6.4e-16 against 1.45e-15).
 //
 // A row that cannot belong to an SPD matrix (a diagonal entry that is not
 // positive, an entry that is not finite or larger than the diagonal allows, a
@@ -861,8 +862,8 @@ __global__ void __launch_bounds__(kUpdThreads, 1) chol_update(double* __restrict
 }
 
 // The update of a few tiles with integer multiply-adds, 16 x 16 entries per block, one
-// per thread: a tile of chol_update occupies one SM for the 112 MMAs of its 28 digit
-// products (77 cycles each) and its operands' way to shared memory, 10.4 us with the
+// per thread: a tile of chol_update occupies one SM for the 136 MMAs of its 34 digit
+// products (77 cycles each) and its operands' way to shared memory, 11.7 us with the
 // launch, however few tiles there are; here they spread over all SMs. 576 rows
 // (9 panels) 380 -> 338 us. One more block places the panel's diagonal tile.
 constexpr int kIntB = 16;

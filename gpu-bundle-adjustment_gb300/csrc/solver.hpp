@@ -393,8 +393,11 @@ void dense_potrf(double* A, int n, int lda, int bt, int* info, void* workspace, 
 // (nothing is done where *info != 0). workspace: dense_potrs_workspace(n) bytes of
 // device memory, the call's own until the stream has passed it.
 size_t dense_potrs_workspace(int n);
-// The same for a band S from both ends (chol.cu): ta tiles from the top, the bt tiles
-// after them last; S stays, F ((n + 64 bt) columns of lda + 1) holds the factor.
+void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* info, void* workspace,
+                 cudaStream_t s);
+
+// Both for a band S, factored from both ends (chol.cu): ta tiles from the top, the bt
+// tiles after them last; S stays, F ((n + 64 bt) columns of lda + 1) holds the factor.
 // *info: whether it failed, not at which of the band's rows.
 size_t band_twist_workspace(int n, int bt);
 size_t band_twist_solve_workspace(int n, int bt);
@@ -402,8 +405,7 @@ void band_potrf_twisted(const double* S, int n, int lda, int bt, int ta, double*
                         cudaStream_t s);
 void band_potrs_twisted(const double* F, int n, int lda, int bt, int ta, double* b, const int* info, void* workspace,
                         cudaStream_t s);
-void dense_potrs(const double* L, int n, int lda, int bt, double* b, const int* info, void* workspace,
-                 cudaStream_t s);
+
 // Residual + Jacobian for E independent observations (device pointers, original
 // layout). Jc, Jp may be null. FP64 or FP32 arithmetic.
 void launch_eval_edges_f64(const double* cams, const double* pts, const int* oc, const int* op,
